@@ -79,7 +79,7 @@ struct ispmv_plan_s {
   double *mm_sum = nullptr;
   size_t mm_cap = 0;                 // doubles in mm_sum
   size_t mm_rows_cap = 0;            // entries of mm_row
-  UIN k1_long = 0;                   // K1: leading chunks run a warp each
+  UIN k1_cta = 0, k1_long = 0;       // K1: chunks [0, k1_cta) a CTA each, [k1_cta, k1_long) a warp each
   std::vector<void *> owned;
   ispmv_plan_info info{};
   std::vector<cudaEvent_t> tev;      // kernel timing: event pairs around the main kernel (a ring)
@@ -93,7 +93,6 @@ namespace {
 
 constexpr size_t SS = sss::SS;      // slots per staged stage; streams pad to it
 constexpr size_t SEG_SLOTS = 2048;  // default slots per warp segment
-constexpr UIN K1_LONG = 64;         // K1 chunks of at least this many columns run a warp each
 
 #define TRY(expr)        \
   do {                   \
@@ -1065,14 +1064,32 @@ ISPMV_API int ispmv_plan_k1(const str_matCSR *csr, const str_matK1 *k1, int reor
   p->nnz = csr->nnz;
   p->slots = k1->lenVC;
   p->chunkNum = k1->chunkNum;
-  // the long chunks (a warp each): the prefix of chunks with at least
-  // K1_LONG columns (nmc never increases: rows are sorted by length)
-  p->k1_long = 0;
-  while (p->k1_long < k1->chunkNum && k1->nmc[p->k1_long] >= K1_LONG) p->k1_long++;
-  std::vector<double> v(k1->val, k1->val + k1->lenVC);
+  // the long chunks (a CTA or a warp each): prefixes of the chunks, whose
+  // column counts never increase (rows are sorted by length)
+  while (p->k1_long < k1->chunkNum && k1->nmc[p->k1_long] >= pk::K1_LONG) p->k1_long++;
+  while (p->k1_cta < p->k1_long && k1->nmc[p->k1_cta] >= pk::K1_CTA) p->k1_cta++;
+  std::vector<double> v;
+  const UIN *kc = k1->col, *chp = k1->chp;
+  size_t lenVC = k1->lenVC;
+  std::vector<UIN> c2, o2;
+  // the kernel reads pairs of slots: if a chunk is at an odd offset (the
+  // builders make none), the chunks are moved to even ones
+  if (std::any_of(chp, chp + k1->chunkNum, [](UIN o) { return o & 1u; })) {
+    for (UIN c = 0; c < k1->chunkNum; c++) {
+      const size_t a = chp[c], e = a + (size_t)8 * k1->nmc[c];
+      o2.push_back((UIN)v.size());
+      v.insert(v.end(), k1->val + a, k1->val + e);
+      c2.insert(c2.end(), kc + a, kc + e);
+    }
+    kc = c2.data();
+    chp = o2.data();
+    lenVC = v.size();
+  } else {
+    v.assign(k1->val, k1->val + lenVC);
+  }
   int st = upload_values(p, v);
-  if (!st) st = dev_upload(p, k1->col, k1->lenVC, &p->col);
-  if (!st) st = dev_upload(p, k1->chp, k1->chunkNum, &p->chp);
+  if (!st) st = dev_upload(p, kc, lenVC, &p->col);
+  if (!st) st = dev_upload(p, chp, k1->chunkNum, &p->chp);
   if (!st) st = dev_upload(p, k1->nmc, k1->chunkNum, &p->nmc);
   if (!st) st = dev_upload(p, k1->permi, (size_t)k1->chunkNum * 8, &p->permi);
   if (!st && !reorder) st = dev_alloc(p, (size_t)k1->chunkNum * 8, &p->res);
@@ -1549,13 +1566,13 @@ int run_main(ispmv_plan_s *p, const FPT *x, FPT *y, int beta, cudaStream_t s) {
       return check_launch("csr_vec");
     }
     case P_K1: {
-      const unsigned g = (unsigned)((pk::k1_warps(p->chunkNum, p->k1_long) * 32 + pk::TPB - 1) / pk::TPB);
+      const unsigned g = (unsigned)pk::k1_ctas(p->chunkNum, p->k1_cta, p->k1_long);
       if (p->fmt == F_K1P) {
-        pk::k1_chunks<VT, true><<<g, pk::TPB, 0, s>>>(p->n, p->chunkNum, p->k1_long, p->chp, p->nmc, p->permi,
+        pk::k1_chunks<VT, true><<<g, pk::TPB, 0, s>>>(p->n, p->chunkNum, p->k1_cta, p->k1_long, p->chp, p->nmc, p->permi,
                                                       p->col, val, x, y, beta);
         return check_launch("k1_chunks<scatter>");
       }
-      pk::k1_chunks<VT, false><<<g, pk::TPB, 0, s>>>(p->n, p->chunkNum, p->k1_long, p->chp, p->nmc, p->permi,
+      pk::k1_chunks<VT, false><<<g, pk::TPB, 0, s>>>(p->n, p->chunkNum, p->k1_cta, p->k1_long, p->chp, p->nmc, p->permi,
                                                      p->col, val, x, p->res, beta);
       return check_launch("k1_chunks");
     }

@@ -72,83 +72,164 @@ __global__ void __launch_bounds__(TPB) axc_rows(UIN n, const UIN *__restrict__ b
 // ----------------------------------------------------------------- K1 --
 // K1 orders rows by length (descending), so a chunk's rows are unrelated
 // rows of the matrix and nearly every gather misses the lines its
-// neighbours touched; the chunks' column counts nmc never increase.  The
-// first `nlong` chunks (the long ones) get a warp each: 4 groups of 8 lanes
-// (lane = row of the chunk) take every 4th column, 8 columns at a time, and
-// combine their sums with two shuffles.  The rest go 4 chunks to a warp,
-// 8 lanes each, also 8 columns at a time.  A lane keeps its 8 value/column
-// loads and then its 8 gathers in flight together, with independent sums.
-// SCATTER writes y[permi] (K1 with integrated reordering), else res in
-// chunk order (then k1_order).  Every chunk column is one coalesced 64-byte
-// load of values.
+// neighbours touched: the gathers (one L1 tag lookup each) bound the kernel,
+// as long as no chunk is one thread group's serial chain.  The chunks' column
+// counts nmc never increase, so three prefixes of the chunks get as many
+// lanes as their length pays for:
+//   chunks [0, ncta), at least K1_CTA columns: a CTA each, its 32 groups of 8
+//     lanes take every 32nd column pair, sums joined in shared memory;
+//   chunks [ncta, nlong), at least K1_LONG columns: a warp each, 4 groups;
+//   the rest: 4 chunks to a warp, one group each.
+// A group reads two columns of its chunk at once: lane l holds rows 2(l%4)
+// and 2(l%4)+1 of column parity l/4, so a value load is 128 contiguous bytes
+// per group (16 B per lane) and touches half the lines one column per load
+// would.  Each lane keeps K1_U pairs of loads, then their 2*K1_U gathers, in
+// flight, in the remainder of a chunk too (predicated, not one after the
+// other).  SCATTER writes y[permi] (K1 with integrated reordering), else res
+// in chunk order (then k1_order).  Measured on power-law rows (n = 1M, 14.9M
+// nonzeros, longest row 1,100-3,000, FP64, K1p): 147.7 us with the long
+// chunks on one warp each and the remainders serial, 67.3 us so; the L1's one
+// tag lookup per gather and cycle alone takes 52 us.
+constexpr UIN K1_LONG = 64;   // columns from which a chunk gets a warp
+constexpr UIN K1_CTA = 256;   // columns from which a chunk gets a CTA
+constexpr int K1_U = 4;       // column pairs in flight per lane
+
+__device__ __forceinline__ double2 ld_pair(const double *p) { return ld_stream(reinterpret_cast<const double2 *>(p)); }
+__device__ __forceinline__ float2 ld_pair(const float *p) { return ld_stream(reinterpret_cast<const float2 *>(p)); }
+
+// Sums of this lane's two rows over the column pairs kp0, kp0 + stride, ...
+// of a chunk of m columns at slot `off`.
 template <typename VT, int STRIDE>
-__device__ __forceinline__ double k1_sum(const VT *__restrict__ val, const UIN *__restrict__ col,
-                                         const FPT *__restrict__ x, size_t off, UIN k0, UIN m, unsigned lane8) {
-  constexpr int U = 8;
-  double acc[U];
+__device__ __forceinline__ double2 k1_sum(const VT *__restrict__ val, const UIN *__restrict__ col,
+                                          const FPT *__restrict__ x, size_t off, UIN kp0, UIN m, unsigned lane8) {
+  using V2 = decltype(ld_pair((const VT *)nullptr));
+  double a0[K1_U], a1[K1_U];
 #pragma unroll
-  for (int u = 0; u < U; u++) acc[u] = 0.0;
-  UIN k = k0;
-  for (; k + (U - 1) * STRIDE < m; k += U * STRIDE) {
-    const size_t p = off + (size_t)k * 8 + lane8;
-    VT v[U];
-    UIN cc[U];
+  for (int u = 0; u < K1_U; u++) a0[u] = a1[u] = 0.0;
+  const UIN np = m / 2 + (m & ((lane8 >> 2) ^ 1u));  // pairs whose column of my parity exists
+  const size_t base = off + 2u * lane8;
+  UIN k = kp0;
+  for (; (uint64_t)k + (K1_U - 1) * STRIDE < np; k += K1_U * STRIDE) {
+    V2 v[K1_U];
+    uint2 c[K1_U];
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      v[u] = ld_stream(val + p + (size_t)8 * STRIDE * u);
-      cc[u] = ld_stream(col + p + (size_t)8 * STRIDE * u);
+    for (int u = 0; u < K1_U; u++) {
+      const size_t p = base + (size_t)16 * (k + (UIN)(u * STRIDE));
+      v[u] = ld_pair(val + p);
+      c[u] = ld_stream(reinterpret_cast<const uint2 *>(col + p));
     }
-    double xv[U];
+    double x0[K1_U], x1[K1_U];
 #pragma unroll
-    for (int u = 0; u < U; u++) xv[u] = ldg(x + cc[u]);
+    for (int u = 0; u < K1_U; u++) {
+      x0[u] = ldg(x + c[u].x);
+      x1[u] = ldg(x + c[u].y);
+    }
 #pragma unroll
-    for (int u = 0; u < U; u++) acc[u] = fmac<VT>(v[u], xv[u], acc[u]);
-  }
-#pragma unroll
-  for (int u = 0; u < U; u++) {  // the last columns of this lane's share
-    const UIN kk = k + (UIN)(u * STRIDE);
-    if (kk < m) {
-      const size_t p = off + (size_t)kk * 8 + lane8;
-      acc[u] = fmac<VT>(ld_stream(val + p), ldg(x + ld_stream(col + p)), acc[u]);
+    for (int u = 0; u < K1_U; u++) {
+      a0[u] = fmac<VT>(v[u].x, x0[u], a0[u]);
+      a1[u] = fmac<VT>(v[u].y, x1[u], a1[u]);
     }
   }
-  return ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+  if (k < np) {  // the remainder: at most K1_U - 1 pairs, in flight together
+    V2 v[K1_U - 1];
+    uint2 c[K1_U - 1];
+    double x0[K1_U - 1], x1[K1_U - 1];
+#pragma unroll
+    for (int u = 0; u < K1_U - 1; u++) {
+      const UIN kk = k + (UIN)(u * STRIDE);
+      if (kk < np) {
+        const size_t p = base + (size_t)16 * kk;
+        v[u] = ld_pair(val + p);
+        c[u] = ld_stream(reinterpret_cast<const uint2 *>(col + p));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < K1_U - 1; u++) {
+      if (k + (UIN)(u * STRIDE) < np) {
+        x0[u] = ldg(x + c[u].x);
+        x1[u] = ldg(x + c[u].y);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < K1_U - 1; u++) {
+      if (k + (UIN)(u * STRIDE) < np) {
+        a0[u] = fmac<VT>(v[u].x, x0[u], a0[u]);
+        a1[u] = fmac<VT>(v[u].y, x1[u], a1[u]);
+      }
+    }
+  }
+  return make_double2((a0[0] + a0[1]) + (a0[2] + a0[3]), (a1[0] + a1[1]) + (a1[2] + a1[3]));
 }
 
 template <typename VT, bool SCATTER>
-__global__ void __launch_bounds__(TPB) k1_chunks(UIN n, UIN chunkNum, UIN nlong, const UIN *__restrict__ chp,
-                                                 const UIN *__restrict__ nmc, const UIN *__restrict__ permi,
-                                                 const UIN *__restrict__ col, const VT *__restrict__ val,
-                                                 const FPT *__restrict__ x, FPT *__restrict__ out, int beta) {
+__global__ void __launch_bounds__(TPB) k1_chunks(UIN n, UIN chunkNum, UIN ncta, UIN nlong,
+                                                 const UIN *__restrict__ chp, const UIN *__restrict__ nmc,
+                                                 const UIN *__restrict__ permi, const UIN *__restrict__ col,
+                                                 const VT *__restrict__ val, const FPT *__restrict__ x,
+                                                 FPT *__restrict__ out, int beta) {
   pdl_trigger();
-  const unsigned lane = threadIdx.x & 31u, lane8 = lane & 7u;
-  const size_t w = ((size_t)blockIdx.x * TPB + threadIdx.x) >> 5;
+  __shared__ double2 part[TPB / 32][4];
+  const unsigned lane = threadIdx.x & 31u, lane8 = lane & 7u, wib = threadIdx.x >> 5;
   size_t c;
-  double s;
-  if (w < nlong) {  // one warp per long chunk: group g takes columns g, g + 4, ...
-    c = w;
-    s = k1_sum<VT, 4>(val, col, x, chp[c], lane >> 3, nmc[c], lane8);
-    s += __shfl_xor_sync(FULL, s, 8);
-    s += __shfl_xor_sync(FULL, s, 16);
-    if (lane >= 8) return;
+  double2 s;
+  if (blockIdx.x < ncta) {  // one CTA per chunk (the whole CTA takes this branch)
+    c = blockIdx.x;
+    s = k1_sum<VT, TPB / 8>(val, col, x, chp[c], threadIdx.x >> 3, nmc[c], lane8);
+#pragma unroll
+    for (int d = 4; d < 32; d <<= 1) {  // column parities and groups: lanes of the same rows
+      s.x += __shfl_xor_sync(FULL, s.x, d);
+      s.y += __shfl_xor_sync(FULL, s.y, d);
+    }
+    if (lane < 4) part[wib][lane] = s;
+    __syncthreads();
+    if (threadIdx.x >= 4) return;
+    s = part[0][lane];
+#pragma unroll
+    for (int w = 1; w < TPB / 32; w++) {
+      s.x += part[w][lane].x;
+      s.y += part[w][lane].y;
+    }
   } else {
-    c = nlong + (w - nlong) * 4 + (lane >> 3);
-    if (c >= chunkNum) return;
-    s = k1_sum<VT, 1>(val, col, x, chp[c], 0, nmc[c], lane8);
+    const size_t w = (size_t)(blockIdx.x - ncta) * (TPB / 32) + wib;
+    if (w < nlong - ncta) {  // one warp per chunk: group g takes pairs g, g + 4, ...
+      c = ncta + w;
+      s = k1_sum<VT, 4>(val, col, x, chp[c], lane >> 3, nmc[c], lane8);
+#pragma unroll
+      for (int d = 4; d < 32; d <<= 1) {
+        s.x += __shfl_xor_sync(FULL, s.x, d);
+        s.y += __shfl_xor_sync(FULL, s.y, d);
+      }
+      if (lane >= 4) return;
+    } else {
+      c = nlong + (w - (nlong - ncta)) * 4 + (lane >> 3);
+      const bool live = c < chunkNum;
+      s = live ? k1_sum<VT, 1>(val, col, x, chp[c], 0, nmc[c], lane8) : make_double2(0.0, 0.0);
+      s.x += __shfl_xor_sync(FULL, s.x, 4);
+      s.y += __shfl_xor_sync(FULL, s.y, 4);
+      if (!live || lane8 >= 4) return;
+    }
   }
-  const size_t i = c * 8 + lane8;
+  const size_t i = c * 8 + 2u * (lane8 & 3u);  // my rows: i, i + 1
   if (SCATTER) {
     if (i < n) {
       const UIN r = permi[i];
-      out[r] = beta ? s + out[r] : s;
+      out[r] = beta ? s.x + out[r] : s.x;
+    }
+    if (i + 1 < n) {
+      const UIN r = permi[i + 1];
+      out[r] = beta ? s.y + out[r] : s.y;
     }
   } else {
-    out[i] = s;
+    *reinterpret_cast<double2 *>(out + i) = s;  // chunk-order scratch of chunkNum * 8 entries
   }
 }
 
-// Warps of a K1 launch: one per long chunk, one per 4 other chunks.
-inline size_t k1_warps(UIN chunkNum, UIN nlong) { return (size_t)nlong + ((size_t)(chunkNum - nlong) + 3) / 4; }
+// CTAs of a K1 launch: one per CTA chunk, then warps: one per long chunk,
+// one per 4 other chunks.
+inline size_t k1_ctas(UIN chunkNum, UIN ncta, UIN nlong) {
+  const size_t warps = (size_t)(nlong - ncta) + ((size_t)(chunkNum - nlong) + 3) / 4;
+  return ncta + (warps + TPB / 32 - 1) / (TPB / 32);
+}
 
 // K1's reorder (orderArrayK1): y in original row order from the chunk-order
 // result; a programmatic dependent launch of k1_chunks where the stream
