@@ -40,6 +40,16 @@ int sm_count();
 // anything.  Both are no-ops for ordinary launches.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A pointer (or texture handle) to what the awaited grid wrote, for use after
+// pdl_wait.  The compiler may move loads through a const __restrict__
+// parameter (read-only for the kernel's lifetime, as far as it is told) above
+// the wait; loads through the value returned here depend on this point.
+template <typename T>
+__device__ __forceinline__ T after_wait(T p) {
+  static_assert(sizeof(T) == 8, "a pointer or a texture handle");
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
 
 // Inclusive segmented sum over the 32 lanes of a warp.  `head` marks the
 // first lane of each run; lanes of one run end up holding the running sum

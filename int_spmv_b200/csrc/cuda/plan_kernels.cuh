@@ -234,9 +234,10 @@ inline size_t k1_ctas(UIN chunkNum, UIN ncta, UIN nlong) {
 // K1's reorder (orderArrayK1): y in original row order from the chunk-order
 // result; a programmatic dependent launch of k1_chunks where the stream
 // allows it, so it first waits for that grid and its writes.
-__global__ void k1_order(UIN n, const UIN *__restrict__ permi, const FPT *__restrict__ res, FPT *__restrict__ y,
-                         int beta) {
+__global__ void k1_order(UIN n, const UIN *__restrict__ permi, const FPT *res_, FPT *y_, int beta) {
   pdl_wait();
+  const FPT *res = after_wait(res_);
+  FPT *y = after_wait(y_);
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
     const UIN r = permi[i];

@@ -98,10 +98,12 @@ __device__ __forceinline__ void finish(const State &st, const Out &o, size_t seg
 // overlaps the main kernel's last CTAs: griddepcontrol.wait then blocks until
 // the main kernel has completed and its records and rows are visible (it
 // returns at once for an ordinary launch).
-__global__ void fixup(size_t nrec, const UIN *__restrict__ rec_row, const double *__restrict__ rec_sum,
-                      const UIN *__restrict__ rowmap, const UIN *__restrict__ empty, size_t nempty,
-                      FPT *__restrict__ y, int beta) {
+__global__ void fixup(size_t nrec, const UIN *rec_row_, const double *rec_sum_, const UIN *__restrict__ rowmap,
+                      const UIN *__restrict__ empty, size_t nempty, FPT *y_, int beta) {
   pdl_wait();
+  const UIN *rec_row = after_wait(rec_row_);
+  const double *rec_sum = after_wait(rec_sum_);
+  FPT *y = after_wait(y_);
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < nempty && !beta) y[empty[i]] = 0.0;
   if (i >= nrec) return;

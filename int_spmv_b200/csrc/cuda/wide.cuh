@@ -372,11 +372,15 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
       for (int k = 0; k < SPL; k++) c[k] = e[k];
     }
     const unsigned bits = (__ldg(heads + (b >> 5) + ((SPL * lane) >> 5)) >> ((SPL * lane) & 31u)) & MASK;
+    const XT *xg = x;
+    cudaTextureObject_t tg = xtex;
     if constexpr (sizeof(XT) == 4) {
       // FP32 x is written by x_to_f32, of which this kernel is a programmatic
       // dependent: its first batch's values and columns are loaded, now wait
       // for that grid and its writes before the first gather
       if (j == 0) pdl_wait();
+      xg = after_wait(xg);
+      if constexpr (TEX) tg = after_wait(tg);
     }
     if constexpr (STG) {
       if (wlen) {  // first batch: the window must have landed (bounded wait)
@@ -397,11 +401,13 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
         xv[k] = gather<NW>(w, sxa, x, c[k]);
       } else if constexpr (TEX) {
         if constexpr (sizeof(XT) == 8) {
-          const int2 t = tex1Dfetch<int2>(xtex, (int)c[k]);
+          const int2 t = tex1Dfetch<int2>(tg, (int)c[k]);
           xv[k] = __hiloint2double(t.y, t.x);
         } else {
-          xv[k] = tex1Dfetch<float>(xtex, (int)c[k]);
+          xv[k] = tex1Dfetch<float>(tg, (int)c[k]);
         }
+      } else if constexpr (sizeof(XT) == 4) {
+        xv[k] = xg[c[k]];  // written while this kernel may already run: no read-only load
       } else {
         xv[k] = __ldg(x + c[k]);
       }
