@@ -43,6 +43,8 @@ struct ispmv_plan_s {
   ispmv_plan_opts opts{};
   UIN n = 0, nnz = 0, th = 1, bs = 0, lanes = 8;
   size_t slots = 0, slots_pad = 0, nunits = 0;
+  bool no_win = false;  // staged variants: empty x windows
+  size_t fslots = 0;  // the format's slots, padding included (stream path: slots holds none)
   size_t seg_slots = 0, nseg = 0;
   UIN useg = 0;
   void *val = nullptr;  // double or float
@@ -149,7 +151,7 @@ void finish_info(ispmv_plan_s *p, const char *name) {
   ispmv_plan_info &i = p->info;
   i.nrows = p->n;
   i.nnz = p->nnz;
-  i.slots = p->slots;
+  i.slots = p->path == P_STREAM ? p->fslots : p->slots;
   i.format = p->fmt;
   i.val_kind = p->opts.val_kind;
   i.col_kind = p->opts.col_kind;
@@ -227,7 +229,8 @@ size_t seg_slots_of(const ispmv_plan_s *p, size_t upu) {
 // stream_wide variants, numbered as measured (numbers not listed here were
 // measured and retired: x bands in shared memory, per-warp row buffers,
 // other segment sizes, stage counts and window sizes):
-// slots per lane, per-CTA x window (cap doubles), segment slots, CTAs per SM
+// slots per lane, per-CTA x window (cap doubles), segment slots (at most:
+// wide_seg), CTAs per SM
 // the registers are sized for (plain loads), and for the staged form (tma)
 // the stages per warp and warps per CTA.
 struct WideCfg {
@@ -261,6 +264,31 @@ WideCfg wide_variant(int v) {
   }
 }
 
+// Slots per warp segment of a lane-interleaved plan of `slots` slots: the
+// variant's segment at most, and short enough that every warp the GPU holds
+// at once has one.  A warp works its batches of 32*spl slots one after the
+// other, about 1.5 us each when little else runs, so a matrix below one full
+// load of warps takes the time of its longest warp.  Near one load and above
+// it, the segments are cut so that the last load is nearly full (3% slack):
+// 1.24 loads of 3072 slots take 30.9 us where 0.93 of 4096 take 25.6
+// (27-point stencil, 80^3, FP32 values).  The bulk-copy staged kernel's
+// persistent warps take segments in turn: 2.3 each leave a quarter of the
+// warps idle in the last turn.  Measured against the variants' fixed segments:
+// 5-point 512^2 15.6 -> 10.6 us (from 2048 slots, padding dropped), power-law n =
+// 30,000 17.8 -> 8.4 us, 32 FEM blocks of 22M nonzeros in one graph 57.2 ->
+// 54.8 us (staged, from 4096).
+size_t wide_seg(const WideCfg &w, size_t slots) {
+  if (w.tmem) return w.seg;
+  if (w.tma) {  // persistent warps, segments dealt in turn: at least 8 per warp
+    const size_t s = slots / ((size_t)sm_count() * 4 * w.warps * 8);
+    return std::min(w.seg, std::max(SS, (s + SS - 1) / SS * SS));
+  }
+  const size_t held = (size_t)sm_count() * w.minb * WIDE_WARPS * 97 / 100;
+  const size_t loads = std::max<size_t>(1, (slots + held * w.seg - 1) / (held * w.seg));
+  const size_t s = (slots + loads * held - 1) / (loads * held);
+  return std::min(w.seg, std::max(SS, (s + SS - 1) / SS * SS));
+}
+
 // Fraction of a deterministic sample of the nonzeros whose column lies
 // far from the diagonal (|c - r| > 1536, outside a 3072-column window) with
 // no column of the next row within 16 of c + 1: gathers with no locality
@@ -287,6 +315,12 @@ double random_far_fraction(const str_matCSR *csr) {
   return (double)far / (double)S;
 }
 
+// AUTO's staged plans of fewer nonzeros than this leave the windows empty: a
+// window is copied before a CTA's first gather, and where a warp has a batch
+// or two that wait shows (n = 30,000: 10.3 us with windows, 8.4 without; n =
+// 100,000, 1.5M nonzeros: equal).
+constexpr UIN WIN_MIN_NNZ = 1u << 20;
+
 // AUTO on a slot-stream plan: the lane-interleaved kernel (stream_wide) and
 // its variant.  8 slots per lane for rows of fewer than 16 nonzeros on
 // average, with per-CTA x windows where the columns are scattered (FP64
@@ -307,6 +341,7 @@ void auto_wide(ispmv_plan_s *p, const str_matCSR *csr) {
   p->opts.kernel = ISPMV_KERNEL_WIDE;
   if (p->opts.variant != 0) return;
   p->opts.variant = auto_variant(p, (double)csr->nnz >= 16.0 * (double)p->n, random_far_fraction(csr) >= 0.05);
+  p->no_win = csr->nnz < WIN_MIN_NNZ;
 }
 
 // The per-CTA x windows of the staged stream_wide variants: CTA t walks
@@ -320,6 +355,7 @@ int stage_windows(ispmv_plan_s *p, const std::vector<double> &v, const std::vect
   const UIN W = wide_variant(p->opts.variant).cap & ~1u, ne = p->n & ~1u;
   const size_t T = (size_t)WIDE_WARPS * p->seg_slots, nt = std::max<size_t>(1, (p->nseg + WIDE_WARPS - 1) / WIDE_WARPS);
   std::vector<UIN> lo(nt, 0), len(nt, 0);
+  if (!p->no_win) {
 #pragma omp parallel for schedule(dynamic, 16)
   for (long long t = 0; t < (long long)nt; t++) {
     if (ne <= W) {  // all of x (but an odd last element) fits
@@ -347,22 +383,47 @@ int stage_windows(ispmv_plan_s *p, const std::vector<double> &v, const std::vect
     lo[t] = (UIN)l & ~1u;
     len[t] = W;
   }
+  }
   UIN *dlo, *dlen;
   TRY(dev_upload(p, lo.data(), lo.size(), &dlo));
   TRY(dev_upload(p, len.data(), len.size(), &dlen));
   p->xw.tlo = dlo;
   p->xw.tlen = dlen;
-  p->xw.cap = W;
+  p->xw.cap = p->no_win ? 0 : W;
   p->xw.nwin = 1;
   p->xw.n = p->n;
   return ISPMV_OK;
 }
 
+// Drops the formats' row padding (AXC bricks, AXT tiles: rows padded to 8
+// slots, or to tileH) from the slot streams: the kernels find rows by their
+// start bits and need none, and every slot costs its 12 bytes and a gather of
+// x[0].  On power-law rows (14.9 nonzeros) tileH = 8 pads 24%: 61.1 -> 54.8
+// us at n = 1M (beta = 1); on 5-point rows 8 slots hold 5.
+void pack_rows(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v, std::vector<UIN> &c,
+               std::vector<size_t> &start) {
+  std::vector<double> pv(csr->nnz);
+  std::vector<UIN> pc(csr->nnz);
+#pragma omp parallel for schedule(static)
+  for (long long r = 0; r < (long long)csr->nrows; r++) {
+    const UIN a = csr->row[r], l = csr->row[r + 1] - a;
+    if (!l) continue;  // a row without slots: start[r] names no slot of its own
+    std::copy_n(v.begin() + start[r], l, pv.begin() + a);
+    std::copy_n(c.begin() + start[r], l, pc.begin() + a);
+    start[r] = a;
+  }
+  v.swap(pv);
+  c.swap(pc);
+  p->slots = csr->nnz;
+}
+
 // The stream path: `v`/`c` the slot streams (length p->slots), `start[r]`
 // the first slot of row r (rows with no slot are skipped).
 int setup_stream(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v, std::vector<UIN> &c,
-                 const std::vector<size_t> &start) {
+                 std::vector<size_t> &start) {
   p->path = P_STREAM;
+  p->fslots = p->slots;
+  if (p->slots != csr->nnz) pack_rows(p, csr, v, c, start);
   p->slots_pad = std::max(SS, (p->slots + SS - 1) / SS * SS);
   if (p->opts.kernel == ISPMV_KERNEL_WIDE && wide_variant(p->opts.variant).tmem) {
     // whole CTAs: every consumer warp of stream_tmem walks a full segment
@@ -383,7 +444,6 @@ int setup_stream(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v,
     rowmap.push_back(r);
   }
   const bool wide = p->opts.kernel == ISPMV_KERNEL_WIDE;
-  size_t wide_seg = 0;
   if (wide) {
     const WideCfg wc = wide_variant(p->opts.variant);
     const bool lo16 = p->opts.val_kind == ISPMV_VAL_F32_LO16;
@@ -392,11 +452,10 @@ int setup_stream(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v,
       return fail(ISPMV_ERR_UNSUPPORTED,
                   "stream_wide: 16-bit column deltas and BF16 lo-words on the plain-load variants "
                   "(lo-words: not the texture-gather variants)");
-    wide_seg = wc.seg;
   }
   p->seg_slots = seg_slots_of(p, 1);
-  if (wide && (p->opts.units_per_warp <= 0 || wide_variant(p->opts.variant).tmem)) p->seg_slots = wide_seg;
-  if (wide && p->seg_slots % SS) p->seg_slots = (p->seg_slots + SS - 1) / SS * SS;
+  if (wide && (p->opts.units_per_warp <= 0 || wide_variant(p->opts.variant).tmem))
+    p->seg_slots = wide_seg(wide_variant(p->opts.variant), p->slots_pad);
   p->nseg = (p->slots_pad + p->seg_slots - 1) / p->seg_slots;
   std::vector<UIN> segh(std::max<size_t>(1, p->nseg), 0);
   UIN acc = 0;
@@ -823,6 +882,8 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
   if (p->opts.val_kind == ISPMV_VAL_F32_LO16 || p->opts.col_kind != ISPMV_COL_U32)
     return fail(ISPMV_ERR_UNSUPPORTED, "plan from a device CSR: FP64/FP32 values, u32 columns");
   // the matrix is checked before any pass indexes through it
+  p->n = n;
+  p->nnz = nnz;
   DevTmp tmp;
   int *bad;
   UIN *flag, *pos;
@@ -865,6 +926,7 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
         scattered = (double)hfar / (double)S >= 0.05;
       }
       p->opts.variant = auto_variant(p, long_rows, scattered);
+      p->no_win = nnz < WIN_MIN_NNZ;
     }
   }
   const WideCfg wc = wide_variant(p->opts.variant);
@@ -874,12 +936,9 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
     return fail(ISPMV_ERR_UNSUPPORTED, "plan from a device CSR: per-CTA x windows up to 2^31 - 1 nonzeros");
   p->fmt = F_CSR;
   p->path = P_STREAM;
-  p->n = n;
-  p->nnz = nnz;
-  p->slots = nnz;
+  p->slots = p->fslots = nnz;
   p->slots_pad = std::max(SS, (p->slots + SS - 1) / SS * SS);
-  p->seg_slots = p->opts.units_per_warp <= 0 ? wc.seg : seg_slots_of(p, 1);
-  if (p->seg_slots % SS) p->seg_slots = (p->seg_slots + SS - 1) / SS * SS;
+  p->seg_slots = p->opts.units_per_warp <= 0 ? wide_seg(wc, p->slots_pad) : seg_slots_of(p, 1);
   p->nseg = (p->slots_pad + p->seg_slots - 1) / p->seg_slots;
   const unsigned spl = (unsigned)wc.spl;
   void *vi;
@@ -917,6 +976,10 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
     TRY(dev_alloc(p, nt, &tlo));
     TRY(dev_alloc(p, nt, &tlen));
     TRY(tmp.alloc(nt + 1, &off));
+    if (p->no_win) {
+      ISPMV_TRY(cudaMemsetAsync(tlo, 0, nt * sizeof(UIN), s));
+      ISPMV_TRY(cudaMemsetAsync(tlen, 0, nt * sizeof(UIN), s));
+    } else {
     dcsr_win_offsets<<<(unsigned)((nt + 1 + 255) / 256), 256, 0, s>>>(nt, T, nnz, off);
     TRY(check_launch("dcsr_win_offsets"));
     if (ne > W && nnz) {
@@ -934,9 +997,10 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
     }
     dcsr_windows<<<(unsigned)nt, 256, 0, s>>>(nt, off, sorted, W, ne, tlo, tlen);
     TRY(check_launch("dcsr_windows"));
+    }
     p->xw.tlo = tlo;
     p->xw.tlen = tlen;
-    p->xw.cap = W;
+    p->xw.cap = p->no_win ? 0 : W;
     p->xw.nwin = 1;
     p->xw.n = p->n;
   }

@@ -33,9 +33,14 @@ struct Out {
 
 __device__ __forceinline__ UIN real_row(const Out &o, UIN r) { return o.rowmap ? o.rowmap[r] : r; }
 
+// The row's value to y.  beta = 1 adds with a reduction at L2 (red.add: y + v
+// in FP64, rounded once, as a load and an add give it; every row is written
+// once, so the result does not depend on any order): a load of y in the
+// middle of a batch stalls its warp.
 __device__ __forceinline__ void write_row(const Out &o, UIN r, double v) {
-  const UIN rr = real_row(o, r);
-  o.y[rr] = o.beta ? v + o.y[rr] : v;
+  FPT *q = o.y + real_row(o, r);
+  if (o.beta) asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(q), "d"(v) : "memory");
+  else *q = v;
 }
 
 // One batch of 32 units, one per lane: `p` the unit's partial sum, `r` its

@@ -57,3 +57,44 @@ def test_k1_chunk_classes(env, reorder, val_kind, top):
     csr = F.CSR(row, col, val)
     plan = D.Plan(csr, F.getFormatDataK1(8, csr, np.zeros(n))[1], reorder=reorder, val=val_kind)
     check(env, row, col, val, plan, val_kind)
+
+
+@pytest.mark.parametrize("fmt", ["CSR", "AXC", "NOC1", "NOC8", "NOC16"])
+@pytest.mark.parametrize("nnz", [1, 511, 512, 513, 4097, 70_001, 2_300_001])
+def test_segment_sizes(env, fmt, nnz):
+    """The lengths of a warp's segment (512 slots up to the variant's), the
+    stream's last partial segment, and formats whose row padding the plan drops."""
+    _, D, F, _ = env
+    n = max(40, nnz // 7)
+    lengths = np.full(n, nnz // n)
+    lengths[: nnz - int(lengths.sum())] += 1
+    lengths[n // 2] += lengths[n // 3]  # an empty row and a longer one
+    lengths[n // 3] = 0
+    rng = np.random.default_rng(nnz)
+    row = np.zeros(n + 1, np.uint32)
+    row[1:] = np.cumsum(lengths)
+    col = np.concatenate([(r + 3 * np.arange(k)) % n for r, k in enumerate(lengths)]).astype(np.uint32)
+    val = rng.standard_normal(nnz)
+    csr = F.CSR(row, col, val)
+    z = np.zeros(n)
+    f = None if fmt == "CSR" else F.getFormatDataAXC(0, csr, z)[1] if fmt == "AXC" else \
+        F.getFormatDataAXT(0, 128, 8, int(fmt[3:]), "NOC", csr, z)[1]
+    for val_kind in ("f64", "f32"):
+        plan = D.Plan(csr, f, val=val_kind)
+        check(env, row, col, val, plan, val_kind)
+        if fmt != "CSR":
+            assert plan.info["slots"] >= nnz  # the format's own slots, its padding included
+
+
+def test_padding_reads_no_x(env):
+    """A format's row padding contributes nothing, whatever x[0] is."""
+    torch, D, F, orc = env
+    row, col, val = rows_of(np.array([2, 3, 5, 1, 0, 4]), 6, 3)
+    col = np.maximum(col, 1).astype(np.uint32)  # no element in column 0
+    csr = F.CSR(row, col, val)
+    x = np.random.default_rng(1).uniform(-1, 1, 6)
+    ref, absax = orc.cf_csr(row, col, val, x), orc.abs_csr(row, col, val, x)
+    x[0] = np.inf
+    for f in (F.getFormatDataAXC(0, csr, x)[1], F.getFormatDataAXT(0, 128, 8, 1, "NOC", csr, x)[1],
+              F.getFormatDataAXT(0, 128, 8, 4, "NOC", csr, x)[1]):
+        assert_parity(D.Plan(csr, f).spmv(torch.from_numpy(x).cuda()).cpu().numpy(), ref, absax, TOL_F64)
