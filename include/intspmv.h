@@ -536,6 +536,12 @@ const char *ispmv_last_error(void);
 /* Kernel launches issued by the library since load (all ispmv_* calls). */
 unsigned long long ispmv_launch_count(void);
 
+/* Device memory that plans and GPU-built formats gave up is kept for later
+ * ones (at most 2 GiB, all devices together).  Gives kept blocks back to the
+ * device until at most keep_bytes remain; *kept (may be NULL) = the bytes
+ * still kept. */
+int ispmv_pool_trim(uint64_t keep_bytes, uint64_t *kept);
+
 /* Self-test of the bounded device wait the staged kernels use on their
  * mbarriers (no reference counterpart): waits on a barrier nothing completes,
  * and returns ISPMV_ERR_TIMEOUT when the wait gave up after its limit (about

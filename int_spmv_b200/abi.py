@@ -165,6 +165,7 @@ PROTOTYPES: dict[str, tuple] = {
     "ispmv_status_string": (C.c_char_p, [C.c_int]),
     "ispmv_last_error": (C.c_char_p, []),
     "ispmv_launch_count": (C.c_ulonglong, []),
+    "ispmv_pool_trim": (C.c_int, [C.c_uint64, C.POINTER(C.c_uint64)]),
 }
 
 # status codes (include/intspmv.h)

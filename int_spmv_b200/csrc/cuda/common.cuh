@@ -24,6 +24,15 @@ const char *last_launch();
 // Records a library error text for ispmv_last_error() and returns `status`.
 int fail(int status, const char *text);
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
+// Device memory from the library's pool (mempool.cu): alloc as cudaMalloc; free
+// keeps the blocks for later requests once no work can use them: `idle` says
+// that the caller has synchronised the stream they were used on, else the
+// device is synchronised.
+int pool_alloc(void **out, size_t bytes);
+void pool_free(void *const *ptrs, size_t count, bool idle);
+// Id of the calling thread's current context; 0 when there is none yet or
+// the driver entry points are unavailable.
+unsigned long long current_ctx_id();
 // Number of SMs of the current device (cached per device).
 int sm_count();
 

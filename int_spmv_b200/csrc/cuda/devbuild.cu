@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 
 #include <cub/device/device_radix_sort.cuh>
 
@@ -200,6 +201,13 @@ __global__ void fill_k1(UIN n, const UIN *__restrict__ row, const UIN *__restric
   }
 }
 
+// Gives builder scratch back once the work on `s` that uses it is done.
+void free_scratch(std::initializer_list<void *> a, cudaStream_t s) {
+  const bool idle = cudaStreamSynchronize(s) == cudaSuccess;
+  if (!idle) (void)cudaGetLastError();
+  pool_free(a.begin(), a.size(), idle);
+}
+
 UIN floor_log2_lt1024(UIN v) {  // M:1286-1287 / M:1341-1348: the largest i < 10 with (v >> i) == 1
   UIN r = 0;
   for (UIN i = 0; i < 10; i++)
@@ -223,9 +231,8 @@ ISPMV_API int ispmv_dev_axt_export(const str_matAXT *m, UIN *con, FPT *ax, UIN *
 
 ISPMV_API int ispmv_dev_axt_free(str_matAXT *m) {
   if (!m) return ISPMV_ERR_ARG;
-  cudaFree(m->con);
-  cudaFree(m->ax);
-  cudaFree(m->sec);
+  void *a[] = {m->con, m->ax, m->sec};
+  pool_free(a, 3, false);
   std::memset(m, 0, sizeof *m);
   return ISPMV_OK;
 }
@@ -264,11 +271,15 @@ ISPMV_API int ispmv_dev_build_axt(UIN bs, UIN thw, UIN th, const char *mode, UIN
       goto done;                                  \
     }                                             \
   } while (0)
+#define DB_ALLOC(ptr, bytes)                                          \
+  do {                                                                \
+    if ((st = pool_alloc((void **)&(ptr), (bytes)))) goto done;       \
+  } while (0)
   DB_TRY(cudaEventCreate(&e0));
   DB_TRY(cudaEventCreate(&e1));
-  DB_TRY(cudaMalloc(&cnt, len * sizeof(uint64_t)));
-  DB_TRY(cudaMalloc(&off, len * sizeof(uint64_t)));
-  DB_TRY(cudaMalloc(&bsum, nb * sizeof(uint64_t)));
+  DB_ALLOC(cnt, len * sizeof(uint64_t));
+  DB_ALLOC(off, len * sizeof(uint64_t));
+  DB_ALLOC(bsum, nb * sizeof(uint64_t));
   DB_TRY(cudaEventRecord(e0, s));
   row_slots<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(n, d_row, grp, noc, cnt);
   if ((st = check_launch("row_slots"))) goto done;
@@ -300,9 +311,9 @@ ISPMV_API int ispmv_dev_build_axt(UIN bs, UIN thw, UIN th, const char *mode, UIN
     m->tileN = (UIN)tiles;
     m->lenAX = (UIN)lenAX;
     m->lenSEC = (UIN)lenSEC;
-    DB_TRY(cudaMalloc(&m->con, std::max<size_t>(1, n) * sizeof(UIN)));
-    DB_TRY(cudaMalloc(&m->ax, std::max<uint64_t>(1, lenAX) * sizeof(FPT)));
-    DB_TRY(cudaMalloc(&m->sec, std::max<uint64_t>(1, lenSEC) * sizeof(UIN)));
+    DB_ALLOC(m->con, std::max<size_t>(1, n) * sizeof(UIN));
+    DB_ALLOC(m->ax, std::max<uint64_t>(1, lenAX) * sizeof(FPT));
+    DB_ALLOC(m->sec, std::max<uint64_t>(1, lenSEC) * sizeof(UIN));
     DB_TRY(cudaMemsetAsync(m->ax, 0, lenAX * sizeof(FPT), s));
     DB_TRY(cudaMemsetAsync(m->sec, 0, lenSEC * sizeof(UIN), s));
     fill_axt<<<(unsigned)(((size_t)n * 32 + 255) / 256), 256, 0, s>>>(n, d_row, d_col, d_val, d_x, off, thw, th,
@@ -323,10 +334,9 @@ ISPMV_API int ispmv_dev_build_axt(UIN bs, UIN thw, UIN th, const char *mode, UIN
     }
   }
 #undef DB_TRY
+#undef DB_ALLOC
 done:
-  cudaFree(cnt);
-  cudaFree(off);
-  cudaFree(bsum);
+  free_scratch({cnt, off, bsum}, s);
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   if (st != ISPMV_OK) ispmv_dev_axt_free(m);
@@ -336,11 +346,8 @@ done:
 // ---------------------------------------------------------------- K1 --
 ISPMV_API int ispmv_dev_k1_free(str_matK1 *m) {
   if (!m) return ISPMV_ERR_ARG;
-  cudaFree(m->permi);
-  cudaFree(m->nmc);
-  cudaFree(m->chp);
-  cudaFree(m->val);
-  cudaFree(m->col);
+  void *a[] = {m->permi, m->nmc, m->chp, m->val, m->col};
+  pool_free(a, 5, false);
   std::memset(m, 0, sizeof *m);
   return ISPMV_OK;
 }
@@ -386,20 +393,24 @@ ISPMV_API int ispmv_dev_build_k1(UIN n, UIN nnz, const UIN *d_row, const UIN *d_
       goto done;                    \
     }                               \
   } while (0)
+#define DB_ALLOC(ptr, bytes)                                          \
+  do {                                                                \
+    if ((st = pool_alloc((void **)&(ptr), (bytes)))) goto done;       \
+  } while (0)
   DB_TRY(cudaEventCreate(&e0));
   DB_TRY(cudaEventCreate(&e1));
-  DB_TRY(cudaMalloc(&rl, (size_t)n * sizeof(UIN)));
-  DB_TRY(cudaMalloc(&rls, ((size_t)cn * 8) * sizeof(UIN)));
-  DB_TRY(cudaMalloc(&ids, (size_t)n * sizeof(UIN)));
-  DB_TRY(cudaMalloc(&m->permi, ((size_t)cn + 1) * 8 * sizeof(UIN)));
-  DB_TRY(cudaMalloc(&m->nmc, std::max<size_t>(1, cn) * sizeof(UIN)));
-  DB_TRY(cudaMalloc(&m->chp, std::max<size_t>(1, cn) * sizeof(UIN)));
-  DB_TRY(cudaMalloc(&cnt, len * sizeof(uint64_t)));
-  DB_TRY(cudaMalloc(&off, len * sizeof(uint64_t)));
-  DB_TRY(cudaMalloc(&bsum, nb * sizeof(uint64_t)));
+  DB_ALLOC(rl, (size_t)n * sizeof(UIN));
+  DB_ALLOC(rls, ((size_t)cn * 8) * sizeof(UIN));
+  DB_ALLOC(ids, (size_t)n * sizeof(UIN));
+  DB_ALLOC(m->permi, ((size_t)cn + 1) * 8 * sizeof(UIN));
+  DB_ALLOC(m->nmc, std::max<size_t>(1, cn) * sizeof(UIN));
+  DB_ALLOC(m->chp, std::max<size_t>(1, cn) * sizeof(UIN));
+  DB_ALLOC(cnt, len * sizeof(uint64_t));
+  DB_ALLOC(off, len * sizeof(uint64_t));
+  DB_ALLOC(bsum, nb * sizeof(uint64_t));
   DB_TRY(cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp_bytes, rl, rls, ids, m->permi, (int)n, 0,
                                                    32, s));
-  DB_TRY(cudaMalloc(&tmp, std::max<size_t>(1, tmp_bytes)));
+  DB_ALLOC(tmp, std::max<size_t>(1, tmp_bytes));
   DB_TRY(cudaEventRecord(e0, s));
   DB_TRY(cudaMemsetAsync(m->permi, 0, ((size_t)cn + 1) * 8 * sizeof(UIN), s));  // zero beyond n (M:851-852)
   DB_TRY(cudaMemsetAsync(rls, 0, (size_t)cn * 8 * sizeof(UIN), s));
@@ -425,8 +436,8 @@ ISPMV_API int ispmv_dev_build_k1(UIN n, UIN nnz, const UIN *d_row, const UIN *d_
   m->nnz = nnz;
   m->chunkNum = cn;
   m->lenVC = (UIN)lenVC;
-  DB_TRY(cudaMalloc(&m->val, std::max<uint64_t>(1, lenVC) * sizeof(FPT)));
-  DB_TRY(cudaMalloc(&m->col, std::max<uint64_t>(1, lenVC) * sizeof(UIN)));
+  DB_ALLOC(m->val, std::max<uint64_t>(1, lenVC) * sizeof(FPT));
+  DB_ALLOC(m->col, std::max<uint64_t>(1, lenVC) * sizeof(UIN));
   DB_TRY(cudaMemsetAsync(m->val, 0, lenVC * sizeof(FPT), s));
   DB_TRY(cudaMemsetAsync(m->col, 0, lenVC * sizeof(UIN), s));
   fill_k1<<<(unsigned)(((size_t)n + 255) / 256), 256, 0, s>>>(n, d_row, d_col, d_val, m->permi, off, m->chp, m->val,
@@ -445,14 +456,9 @@ ISPMV_API int ispmv_dev_build_k1(UIN n, UIN nnz, const UIN *d_row, const UIN *d_
     fd->ct = ms * 1e-3;
   }
 #undef DB_TRY
+#undef DB_ALLOC
 done:
-  cudaFree(rl);
-  cudaFree(rls);
-  cudaFree(ids);
-  cudaFree(cnt);
-  cudaFree(off);
-  cudaFree(bsum);
-  cudaFree(tmp);
+  free_scratch({rl, rls, ids, cnt, off, bsum, tmp}, s);
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   if (st != ISPMV_OK) ispmv_dev_k1_free(m);

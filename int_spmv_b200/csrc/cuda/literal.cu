@@ -29,8 +29,6 @@
 // the `_f32` suffix through intspmv.h).  Products and sums are FP64 in both;
 // an FP32 result is rounded once when it is stored (or, for the AXT kernels,
 // when each row run is added to y).
-#include <cuda.h>
-
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
@@ -309,39 +307,6 @@ struct K1RowsAddr {
 };
 std::mutex g_k1_rows_mu;
 K1RowsAddr g_k1_rows_addr[64] = {};
-
-// cuCtxGetCurrent / cuCtxGetId through the runtime's driver entry points, so
-// the library links no driver library.  Null when unavailable.
-typedef CUresult(CUDAAPI *CtxGetCurrentFn)(CUcontext *);
-typedef CUresult(CUDAAPI *CtxGetIdFn)(CUcontext, unsigned long long *);
-CtxGetCurrentFn g_ctx_current = nullptr;
-CtxGetIdFn g_ctx_id = nullptr;
-std::once_flag g_ctx_fns_once;
-
-void find_ctx_fns() {
-  void *f = nullptr;
-  cudaDriverEntryPointQueryResult q;
-  if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
-      q == cudaDriverEntryPointSuccess)
-    g_ctx_current = reinterpret_cast<CtxGetCurrentFn>(f);
-  f = nullptr;
-  if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
-      q == cudaDriverEntryPointSuccess)
-    g_ctx_id = reinterpret_cast<CtxGetIdFn>(f);
-  (void)cudaGetLastError();
-}
-
-// Id of the calling thread's current context; 0 when there is none yet or
-// the driver entry points are unavailable.
-unsigned long long current_ctx_id() {
-  std::call_once(g_ctx_fns_once, find_ctx_fns);
-  if (!g_ctx_current || !g_ctx_id) return 0;
-  CUcontext c = nullptr;
-  unsigned long long id = 0;
-  if (g_ctx_current(&c) != CUDA_SUCCESS || !c) return 0;
-  if (g_ctx_id(c, &id) != CUDA_SUCCESS) return 0;
-  return id;
-}
 
 // The array's address in the current context (the host-side symbol is not a
 // device address).  Looked up with cudaGetSymbolAddress the first time a

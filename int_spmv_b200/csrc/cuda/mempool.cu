@@ -1,0 +1,194 @@
+// mempool.cu - device memory of plans, GPU-built formats and builder scratch.
+//
+// cudaMalloc and cudaFree map and unmap memory: a plan built from a device
+// CSR and dropped again after one product (a matrix assembled anew in every
+// step) spent 5-11 ms of its 6-12 on them at n = 1M, 14.9M nonzeros, where
+// its kernels take 0.9.  Freed blocks are kept here, by device, and given
+// to later requests of nearly their size.
+//   - Bounded: at most POOL_MAX bytes are kept; the block kept longest goes
+//     first.  ispmv_pool_trim gives them back on demand, and a failing
+//     cudaMalloc empties the pool and tries again.
+//   - A block is kept only once no work can use it any more: the caller has
+//     synchronised the stream it was used on (idle = true), or the device is
+//     synchronised here, as cudaFree did.  Whatever that returns an error
+//     for (a capture under way, a context that is gone) is left to cudaFree.
+//   - Blocks belong to the context they were allocated in: ones of a context
+//     that was destroyed (cudaDeviceReset) are forgotten.
+//   - One lock; the pool lives until the process ends.
+#include <cuda.h>
+
+#include <algorithm>
+#include <mutex>
+#include <unordered_map>
+#include <vector>
+
+#include "common.cuh"
+
+namespace ispmv {
+namespace {
+
+constexpr size_t POOL_MAX = (size_t)2 << 30;
+
+// cuCtxGetCurrent / cuCtxGetId through the runtime's driver entry points, so
+// the library links no driver library.  Null when unavailable.
+typedef CUresult(CUDAAPI *CtxGetCurrentFn)(CUcontext *);
+typedef CUresult(CUDAAPI *CtxGetIdFn)(CUcontext, unsigned long long *);
+CtxGetCurrentFn g_ctx_current = nullptr;
+CtxGetIdFn g_ctx_id = nullptr;
+std::once_flag g_ctx_fns_once;
+
+void find_ctx_fns() {
+  void *f = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
+      q == cudaDriverEntryPointSuccess)
+    g_ctx_current = reinterpret_cast<CtxGetCurrentFn>(f);
+  f = nullptr;
+  if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
+      q == cudaDriverEntryPointSuccess)
+    g_ctx_id = reinterpret_cast<CtxGetIdFn>(f);
+  (void)cudaGetLastError();
+}
+
+struct Block {
+  void *ptr;
+  size_t bytes;
+  int dev;
+  unsigned long long ctx;
+};
+struct Pool {
+  std::mutex mu;
+  std::vector<Block> kept;                  // oldest first
+  size_t kept_bytes = 0;
+  std::unordered_map<void *, Block> live;   // blocks handed out
+};
+Pool &pool() {
+  static Pool *p = new Pool();  // never destroyed: plans may outlive static objects
+  return *p;
+}
+
+// Requests are rounded up to steps of 1/8 of their power of two (512 bytes
+// at least), so that a matrix of nearly the same size finds the same blocks.
+size_t rounded(size_t n) {
+  size_t step = 512;
+  while (step * 16 <= n) step *= 2;
+  return std::max<size_t>(1, (n + step - 1) / step) * step;
+}
+
+// Frees kept blocks, oldest first, until at most `keep` bytes are kept.
+void trim_locked(Pool &p, size_t keep) {
+  size_t k = 0;
+  const unsigned long long ctx = p.kept_bytes > keep ? current_ctx_id() : 0;
+  for (; k < p.kept.size() && p.kept_bytes > keep; k++) {
+    const Block &b = p.kept[k];
+    p.kept_bytes -= b.bytes;
+    int dev = 0;
+    // a block of this device but another context: that context is gone
+    if (cudaGetDevice(&dev) == cudaSuccess && dev == b.dev && ctx != b.ctx) continue;
+    if (cudaFree(b.ptr) != cudaSuccess) (void)cudaGetLastError();
+  }
+  p.kept.erase(p.kept.begin(), p.kept.begin() + k);
+}
+
+}  // namespace
+
+unsigned long long current_ctx_id() {
+  std::call_once(g_ctx_fns_once, find_ctx_fns);
+  if (!g_ctx_current || !g_ctx_id) return 0;
+  CUcontext c = nullptr;
+  unsigned long long id = 0;
+  if (g_ctx_current(&c) != CUDA_SUCCESS || !c) return 0;
+  if (g_ctx_id(c, &id) != CUDA_SUCCESS) return 0;
+  return id;
+}
+
+int pool_alloc(void **out, size_t bytes) {
+  *out = nullptr;
+  int dev = 0;
+  ISPMV_TRY(cudaGetDevice(&dev));
+  Pool &p = pool();
+  const size_t want = rounded(bytes);
+  {
+    const unsigned long long ctx = current_ctx_id();
+    std::lock_guard<std::mutex> g(p.mu);
+    size_t best = p.kept.size();
+    for (size_t i = 0; ctx && i < p.kept.size(); i++) {
+      const Block &b = p.kept[i];
+      if (b.dev == dev && b.ctx == ctx && b.bytes >= want && b.bytes <= want + want / 4 &&
+          (best == p.kept.size() || b.bytes < p.kept[best].bytes))
+        best = i;
+    }
+    if (best < p.kept.size()) {
+      const Block b = p.kept[best];
+      p.kept.erase(p.kept.begin() + best);
+      p.kept_bytes -= b.bytes;
+      p.live[b.ptr] = b;
+      *out = b.ptr;
+      return ISPMV_OK;
+    }
+  }
+  void *ptr = nullptr;
+  cudaError_t e = cudaMalloc(&ptr, want);
+  if (e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    {
+      std::lock_guard<std::mutex> g(p.mu);
+      trim_locked(p, 0);
+    }
+    e = cudaMalloc(&ptr, want);
+  }
+  if (e != cudaSuccess) return cuda_status(e, "cudaMalloc");
+  const unsigned long long ctx = current_ctx_id();
+  std::lock_guard<std::mutex> g(p.mu);
+  p.live[ptr] = Block{ptr, want, dev, ctx};
+  *out = ptr;
+  return ISPMV_OK;
+}
+
+void pool_free(void *const *ptrs, size_t count, bool idle) {
+  Pool &p = pool();
+  int cur = -1;
+  if (cudaGetDevice(&cur) != cudaSuccess) cur = -1;
+  unsigned long long ctx = 0;
+  int synced = -1;  // the device whose work is known to be done
+  for (size_t i = 0; i < count; i++) {
+    if (!ptrs[i]) continue;
+    Block b{nullptr, 0, -1, 0};
+    {
+      std::lock_guard<std::mutex> g(p.mu);
+      auto it = p.live.find(ptrs[i]);
+      if (it != p.live.end()) {
+        b = it->second;
+        p.live.erase(it);
+      }
+    }
+    bool keep = b.ptr && b.ctx && b.bytes <= POOL_MAX && cur >= 0;
+    if (keep && synced != b.dev) {
+      keep = (cur == b.dev || cudaSetDevice(b.dev) == cudaSuccess) &&
+             (idle || cudaDeviceSynchronize() == cudaSuccess);
+      ctx = keep ? current_ctx_id() : 0;
+      if (keep) synced = b.dev;
+      else (void)cudaGetLastError();
+      if (cur != b.dev) (void)cudaSetDevice(cur);
+    }
+    if (keep && ctx == b.ctx) {
+      std::lock_guard<std::mutex> g(p.mu);
+      p.kept.push_back(b);
+      p.kept_bytes += b.bytes;
+      trim_locked(p, POOL_MAX);
+    } else if (cudaFree(ptrs[i]) != cudaSuccess) {
+      (void)cudaGetLastError();
+    }
+  }
+}
+
+}  // namespace ispmv
+
+ISPMV_API int ispmv_pool_trim(uint64_t keep_bytes, uint64_t *kept) {
+  using namespace ispmv;
+  Pool &p = pool();
+  std::lock_guard<std::mutex> g(p.mu);
+  trim_locked(p, (size_t)keep_bytes);
+  if (kept) *kept = p.kept_bytes;
+  return ISPMV_OK;
+}

@@ -105,7 +105,7 @@ constexpr size_t SEG_SLOTS = 2048;  // default slots per warp segment
 template <typename T>
 int dev_upload(ispmv_plan_s *p, const T *h, size_t n, T **d) {
   void *ptr = nullptr;
-  ISPMV_TRY(cudaMalloc(&ptr, (n ? n : 1) * sizeof(T)));
+  TRY(pool_alloc(&ptr, (n ? n : 1) * sizeof(T)));
   p->owned.push_back(ptr);
   if (n && h) ISPMV_TRY(cudaMemcpy(ptr, h, n * sizeof(T), cudaMemcpyHostToDevice));
   *d = static_cast<T *>(ptr);
@@ -638,7 +638,7 @@ ISPMV_API int ispmv_plan_destroy(ispmv_plan p) {
   if (p->graph_exec) cudaGraphExecDestroy(p->graph_exec);
   if (p->graph) cudaGraphDestroy(p->graph);
   if (p->cap_stream) cudaStreamDestroy(p->cap_stream);
-  for (void *q : p->owned) cudaFree(q);
+  pool_free(p->owned.data(), p->owned.size(), false);
   delete p;
   return ISPMV_OK;
 }
@@ -748,15 +748,22 @@ __global__ void dcsr_interleave(size_t nnz, size_t spad, unsigned spl, const UIN
   }
 }
 
-struct DevTmp {  // builder scratch, freed on every exit
+// Builder scratch, given back on every exit; the stream it was used on is
+// synchronised first.
+struct DevTmp {
+  cudaStream_t s;
   std::vector<void *> v;
+  explicit DevTmp(cudaStream_t st) : s(st) {}
   ~DevTmp() {
-    for (void *q : v) cudaFree(q);
+    if (v.empty()) return;
+    const bool idle = cudaStreamSynchronize(s) == cudaSuccess;
+    if (!idle) (void)cudaGetLastError();
+    pool_free(v.data(), v.size(), idle);
   }
   template <typename T>
   int alloc(size_t n, T **d) {
     void *q = nullptr;
-    ISPMV_TRY(cudaMalloc(&q, (n ? n : 1) * sizeof(T)));
+    TRY(pool_alloc(&q, (n ? n : 1) * sizeof(T)));
     v.push_back(q);
     *d = static_cast<T *>(q);
     return ISPMV_OK;
@@ -884,7 +891,7 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
   // the matrix is checked before any pass indexes through it
   p->n = n;
   p->nnz = nnz;
-  DevTmp tmp;
+  DevTmp tmp(s);
   int *bad;
   UIN *flag, *pos;
   TRY(tmp.alloc(1, &bad));

@@ -43,6 +43,15 @@ def to_device(a: np.ndarray, device="cuda") -> torch.Tensor:
     return torch.from_numpy(np.ascontiguousarray(a)).to(device)
 
 
+def trim_pool(keep_bytes: int = 0) -> int:
+    """Give the device memory that dropped plans and GPU-built formats left
+    in the library's pool (at most 2 GiB) back to the device, all but
+    `keep_bytes`; returns the bytes still kept."""
+    kept = C.c_uint64()
+    check(load().ispmv_pool_trim(keep_bytes, C.byref(kept)), "ispmv_pool_trim")
+    return kept.value
+
+
 # --- the reference's kernels on device tensors (intSpmv_main.c line cited) ---
 
 def cf_CSR(row, col, val, x, y, stream=None):  # :382

@@ -1,0 +1,92 @@
+"""The library's memory pool: plans and GPU-built formats on recycled
+blocks, dropped with work in flight, from several threads, and given back."""
+from __future__ import annotations
+
+import threading
+
+import numpy as np
+import pytest
+
+from paritylib import assert_parity
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def env():
+    import torch
+    from int_spmv_b200 import device as D
+    from int_spmv_b200 import matrices as M
+    from oracle import Oracle
+    return torch, D, M, Oracle()
+
+
+def make(env, n, seed):
+    torch, D, M, orc = env
+    row, col, val = M.random_csr(n, seed, rl_max=30, empty_frac=0.1)
+    x = M.uniform_x(n, seed)
+    dev = [D.to_device(a) for a in (row, col, val, x)]
+    return dev, orc.cf_csr(row, col, val, x), orc.abs_csr(row, col, val, x)
+
+
+def test_recycled_blocks(env):
+    """Plans and formats of nearly the same sizes, one after the other: each
+    starts on memory that holds another's arrays."""
+    torch, D, _, _ = env
+    for i in range(6):
+        (row, col, val, x), ref, absax = make(env, 20_000 + 37 * i, i)
+        for kind in ("f64", "f32"):
+            y = D.Plan.from_device_csr(row, col, val, val_kind=kind).spmv(x)
+            assert_parity(y.cpu().numpy(), ref, absax, 1e-12 if kind == "f64" else 1e-6)
+        for mode, th in (("COM", 1), ("NOC", 1), ("NOC", 4)):
+            y = D.DeviceAXT(row, col, val, x, th=th, mode=mode).spmv(torch.zeros_like(x))
+            assert_parity(y.cpu().numpy(), ref, absax)
+        assert_parity(D.DeviceK1(row, col, val).spmv(x, torch.empty_like(x)).cpu().numpy(), ref, absax)
+    assert 0 < D.trim_pool(1 << 40) <= 2 << 30
+    assert D.trim_pool(0) == 0
+
+
+def test_dropped_in_flight(env):
+    """A plan dropped right after its product is launched on another stream:
+    its blocks are not reused before the product is done."""
+    torch, D, _, _ = env
+    (row, col, val, x), ref, absax = make(env, 60_000, 3)
+    (row2, col2, val2, x2), ref2, absax2 = make(env, 60_100, 4)
+    side = torch.cuda.Stream()
+    a = torch.randn(4096, 4096, device="cuda")
+    for _ in range(5):
+        plan, y = D.Plan.from_device_csr(row, col, val), torch.empty_like(x)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            a @ a  # keeps the product waiting
+            plan.spmv(x, y)
+        del plan
+        y2 = D.Plan.from_device_csr(row2, col2, val2).spmv(x2)
+        torch.cuda.synchronize()
+        assert_parity(y.cpu().numpy(), ref, absax)
+        assert_parity(y2.cpu().numpy(), ref2, absax2)
+
+
+def test_threads(env):
+    """Four threads build, multiply and drop at once, each on its stream."""
+    torch, D, _, _ = env
+    mats = [make(env, 8_000 + 11 * t, t) for t in range(4)]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(t):
+        (row, col, val, x), ref, absax = mats[t]
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            for _ in range(20):
+                y = D.Plan.from_device_csr(row, col, val).spmv(x)
+                s.synchronize()
+                if np.any(np.abs(y.cpu().numpy() - ref) > 1e-12 * absax):
+                    wrong.append(t)
+
+    ts = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not wrong
