@@ -21,10 +21,10 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include <cub/device/device_scan.cuh>
-#include <cub/device/device_segmented_radix_sort.cuh>
 
 #include "plan_tma.cuh"
 #include "spmm.cuh"
@@ -345,51 +345,80 @@ void auto_wide(ispmv_plan_s *p, const str_matCSR *csr) {
 }
 
 // The per-CTA x windows of the staged stream_wide variants: CTA t walks
-// slots [t*T, (t+1)*T), T = WIDE_WARPS*seg_slots; its window is the
-// cap-long interval of x holding the most of those slots' columns (padding
-// slots excluded), centred on them, clamped to x and started at an even
-// column, so the bulk copy starts on a 16-byte boundary and moves a
-// multiple of 16 bytes, all inside x[0, n rounded down to even).  Columns
-// outside a CTA's window are gathered from x.
-int stage_windows(ispmv_plan_s *p, const std::vector<double> &v, const std::vector<UIN> &c) {
-  const UIN W = wide_variant(p->opts.variant).cap & ~1u, ne = p->n & ~1u;
-  const size_t T = (size_t)WIDE_WARPS * p->seg_slots, nt = std::max<size_t>(1, (p->nseg + WIDE_WARPS - 1) / WIDE_WARPS);
-  std::vector<UIN> lo(nt, 0), len(nt, 0);
-  if (!p->no_win) {
-#pragma omp parallel for schedule(dynamic, 16)
-  for (long long t = 0; t < (long long)nt; t++) {
-    if (ne <= W) {  // all of x (but an odd last element) fits
-      len[t] = ne;
-      continue;
+// slots [t*T, (t+1)*T), T = WIDE_WARPS*seg_slots; its window is W = cap
+// columns of x that hold many of those slots' columns, started at an even
+// column inside x[0, n rounded down to even), so the bulk copy starts on a
+// 16-byte boundary and moves a multiple of 16 bytes.  Columns outside a CTA's
+// window are gathered from x, so the choice costs time only; it is made from
+// every fourth group of 8 slots, by counting twice:
+//   1. columns per bin of 2^s1 (at most 8192 bins): the l1 neighbouring bins
+//      with the most columns, l1 bins being wide enough for any W columns;
+//   2. columns per bin of 2^s2 inside those (at most 2048 bins): the W >> s2
+//      bins with the most; the first of equals in both.
+// The device builder makes the same choice (dcsr_windows).
+struct WinGeom {
+  UIN W, ne, s1, nb1, l1, s2, nb2, w2;
+};
+WinGeom win_geom(UIN n, UIN cap) {
+  WinGeom g{};
+  g.W = cap & ~1u;
+  g.ne = n & ~1u;
+  for (g.s1 = 10; ((n - 1) >> g.s1) >= 8192u;) g.s1++;
+  g.nb1 = ((n - 1) >> g.s1) + 1;
+  g.l1 = ((g.W + (1u << g.s1) - 1) >> g.s1) + 1;
+  for (g.s2 = 0; (((uint64_t)g.l1 << g.s1) >> g.s2) > 2048u;) g.s2++;
+  g.nb2 = (UIN)(((uint64_t)g.l1 << g.s1) >> g.s2);
+  g.w2 = std::max<UIN>(1, g.W >> g.s2);
+  return g;
+}
+__host__ __device__ inline bool win_sampled(size_t slot) { return ((slot >> 3) & 3u) == 0; }
+
+// The first start of the `w` neighbouring bins with the most counts.
+UIN best_run(const UIN *h, UIN nb, UIN w) {
+  uint64_t sum = 0, best = 0;
+  UIN at = 0;
+  for (UIN i = 0; i < std::min(w, nb); i++) sum += h[i];
+  best = sum;
+  for (UIN i = 1; i < nb; i++) {
+    sum -= h[i - 1];
+    if ((uint64_t)i + w - 1 < nb) sum += h[i + w - 1];
+    if (sum > best) {
+      best = sum;
+      at = i;
     }
-    const size_t a = (size_t)t * T, e = std::min(p->slots, a + T);
-    std::vector<UIN> cs;
-    cs.reserve(T);
-    for (size_t q = a; q < e; q++)
-      if (v[q] != 0.0) cs.push_back(c[q]);
-    long long l = 0;
-    if (!cs.empty()) {
-      std::sort(cs.begin(), cs.end());
-      size_t best = 0, ba = 0, bb = 1;
-      for (size_t i = 0, j = 0; i < cs.size(); i++) {  // [cs[i], cs[i] + W - 1)
-        if (j < i) j = i;
-        while (j < cs.size() && cs[j] - cs[i] < W - 1) j++;
-        if (j - i > best) { best = j - i; ba = i; bb = j; }
-      }
-      const long long span = (long long)cs[bb - 1] - (long long)cs[ba] + 1;
-      l = (long long)cs[ba] - ((long long)W - span) / 2;
-    }
-    l = std::max(0LL, std::min(l, (long long)(ne - W)));
-    lo[t] = (UIN)l & ~1u;
-    len[t] = W;
   }
+  return at;
+}
+
+int stage_windows(ispmv_plan_s *p, const std::vector<UIN> &c) {
+  const WinGeom g = win_geom(p->n, wide_variant(p->opts.variant).cap);
+  const size_t T = (size_t)WIDE_WARPS * p->seg_slots, nt = std::max<size_t>(1, (p->nseg + WIDE_WARPS - 1) / WIDE_WARPS);
+  std::vector<UIN> lo(nt, 0), len(nt, p->no_win ? 0 : std::min(g.ne, g.W));
+  if (!p->no_win && g.ne > g.W) {
+#pragma omp parallel
+    {
+      std::vector<UIN> h1(g.nb1), h2(g.nb2);
+#pragma omp for schedule(dynamic, 16)
+      for (long long t = 0; t < (long long)nt; t++) {
+        const size_t a = (size_t)t * T, e = std::min(p->slots, a + T);
+        std::fill(h1.begin(), h1.end(), 0u);
+        std::fill(h2.begin(), h2.end(), 0u);
+        for (size_t q = a; q < e; q++)
+          if (win_sampled(q) && (c[q] >> g.s1) < g.nb1) h1[c[q] >> g.s1]++;
+        const UIN r = best_run(h1.data(), g.nb1, g.l1) << g.s1;
+        for (size_t q = a; q < e; q++)
+          if (win_sampled(q) && c[q] >= r && ((c[q] - r) >> g.s2) < g.nb2) h2[(c[q] - r) >> g.s2]++;
+        const uint64_t l = (uint64_t)r + ((uint64_t)best_run(h2.data(), g.nb2, g.w2) << g.s2);
+        lo[t] = (UIN)std::min<uint64_t>(l, g.ne - g.W) & ~1u;
+      }
+    }
   }
   UIN *dlo, *dlen;
   TRY(dev_upload(p, lo.data(), lo.size(), &dlo));
   TRY(dev_upload(p, len.data(), len.size(), &dlen));
   p->xw.tlo = dlo;
   p->xw.tlen = dlen;
-  p->xw.cap = p->no_win ? 0 : W;
+  p->xw.cap = p->no_win ? 0 : g.W;
   p->xw.nwin = 1;
   p->xw.n = p->n;
   return ISPMV_OK;
@@ -608,7 +637,7 @@ int setup_stream(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v,
   if (any_empty) TRY(dev_upload(p, rowmap.data(), rowmap.size(), &p->rowmap));
   p->nrowmap = any_empty ? rowmap.size() : 0;
   const bool stg = wide && wide_variant(p->opts.variant).stg;
-  if (stg) TRY(stage_windows(p, v, c));
+  if (stg) TRY(stage_windows(p, c));
   TRY(empty_rows(p, csr));
   TRY(alloc_records(p));
   if (stg) p->xw.status = p->status;
@@ -686,65 +715,57 @@ ISPMV_API int ispmv_plan_csr(const str_matCSR *csr, const ispmv_plan_opts *o, is
 // atomicOr, so the bitmap does not depend on the order of the writes.
 namespace {
 
-// *bad = 1 if the row pointer decreases, row[0] != 0, row[n] != nnz, or a
-// column is >= n.  Only reads row[0..n] and col[0..nnz).
-__global__ void dcsr_check(UIN n, UIN nnz, const UIN *__restrict__ row, const UIN *__restrict__ col,
-                           int *__restrict__ bad) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t r = i; r < n; r += stride)
-    if (row[r + 1] < row[r]) *bad = 1;
-  for (size_t j = i; j < nnz; j += stride)
-    if (col[j] >= n) *bad = 1;
-  if (i == 0 && (row[0] != 0 || row[n] != nnz)) *bad = 1;
-}
-
-// flag[r] = 1 for a row with elements; flag[n] = 0, so the exclusive prefix
+// *bad = 1 if the row pointer decreases, row[0] != 0 or row[n] != nnz;
+// flag[r] = 1 for a row with elements, flag[n] = 0, so the exclusive prefix
 // at n is the count of non-empty rows.
-__global__ void dcsr_flags(UIN n, const UIN *__restrict__ row, UIN *__restrict__ flag) {
+__global__ void dcsr_check_rows(UIN n, UIN nnz, const UIN *__restrict__ row, UIN *__restrict__ flag,
+                                int *__restrict__ bad) {
   const size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r <= n) flag[r] = r < n && row[r + 1] > row[r] ? 1u : 0u;
+  if (r > n) return;
+  if (r == n) {
+    flag[n] = 0;
+    if (row[0] != 0 || row[n] != nnz) *bad = 1;
+    return;
+  }
+  const UIN a = row[r], e = row[r + 1];
+  flag[r] = e > a;
+  if (e < a) *bad = 1;
 }
 
 // Row-start bits, the compressed -> real map and the empty-row list from the
-// prefix `pos` of the non-empty flags.
+// prefix `pos` of the non-empty flags; and segh[g] = row starts at slots
+// below g*seg = pos[first r with row[r] >= g*seg], written by that r's thread
+// (n's, past the last row).
 __global__ void dcsr_rows(UIN n, const UIN *__restrict__ row, const UIN *__restrict__ pos, UIN *__restrict__ heads,
-                          UIN *__restrict__ rowmap, UIN *__restrict__ empty) {
+                          UIN *__restrict__ rowmap, UIN *__restrict__ empty, size_t nseg, UIN seg,
+                          UIN *__restrict__ segh) {
   const size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  const UIN a = row[r];
+  if (r > n) return;
+  const UIN a = row[r], q = pos[r];
+  const size_t g1 = r == n ? nseg : min((size_t)(a / seg) + 1, nseg);
+  for (size_t g = r == 0 ? 0 : (size_t)(row[r - 1] / seg) + 1; g < g1; g++) segh[g] = q;
+  if (r == n) return;
   if (row[r + 1] > a) {
     atomicOr(&heads[a >> 5], 1u << (a & 31u));
-    if (rowmap) rowmap[pos[r]] = (UIN)r;
+    if (rowmap) rowmap[q] = (UIN)r;
   } else if (empty) {
-    empty[r - pos[r]] = (UIN)r;
+    empty[r - q] = (UIN)r;
   }
 }
 
-// segh[g] = row starts at slots below g*seg: the non-empty rows r with
-// row[r] < g*seg, i.e. pos[first r with row[r] >= g*seg].
-__global__ void dcsr_segh(size_t nseg, size_t seg, UIN n, const UIN *__restrict__ row, const UIN *__restrict__ pos,
-                          UIN *__restrict__ segh) {
-  const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= nseg) return;
-  const uint64_t S = (uint64_t)g * seg;
-  UIN lo = 0, hi = n;  // first r in [0, n) with row[r] >= S, else n
-  while (lo < hi) {
-    const UIN mid = lo + (hi - lo) / 2;
-    if ((uint64_t)row[mid] < S) lo = mid + 1;
-    else hi = mid;
-  }
-  segh[g] = pos[lo];
-}
-
-// The lane-interleaved value and column copies, zero beyond nnz.
-template <typename VT>
-__global__ void dcsr_interleave(size_t nnz, size_t spad, unsigned spl, const UIN *__restrict__ col,
-                                const FPT *__restrict__ val, VT *__restrict__ vi, UIN *__restrict__ ci) {
+// The lane-interleaved value and column copies, zero beyond nnz; *bad = 1 for
+// a column >= n (no pass before this one indexes by a column).
+template <typename VT, int SPL>
+__global__ void dcsr_interleave(UIN n, size_t nnz, size_t spad, const UIN *__restrict__ col,
+                                const FPT *__restrict__ val, VT *__restrict__ vi, UIN *__restrict__ ci,
+                                int *__restrict__ bad) {
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < spad; q += stride) {
     const bool in = q < nnz;
-    vi[wide::il_pos(q, spl, 16u / (unsigned)sizeof(VT))] = (VT)(in ? val[q] : 0.0);
-    ci[wide::il_pos(q, spl, 4u)] = in ? col[q] : 0u;
+    vi[wide::il_pos_c<SPL, 16u / sizeof(VT)>(q)] = (VT)(in ? val[q] : 0.0);
+    const UIN c = in ? col[q] : 0u;
+    if (c >= n) *bad = 1;
+    ci[wide::il_pos_c<SPL, 4u>(q)] = c;
   }
 }
 
@@ -771,116 +792,122 @@ struct DevTmp {
 };
 
 // random_far_fraction on a device CSR: the same sample (nonzero
-// j = (size_t)(i * stride)), its row by binary search (the r with
-// row[r] <= j < row[r+1]), the same test; *far counts the hits.
-__global__ void dcsr_far(size_t S, double stride, UIN n, const UIN *__restrict__ row, const UIN *__restrict__ col,
-                         unsigned long long *__restrict__ far) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+// j = (size_t)(i * stride)), its row the r with row[r] <= j < row[r+1], the
+// same test; *far counts the hits.  8 lanes per sample: a 9-way search for
+// the row (7 steps at a million rows, where a thread's binary search takes 20
+// dependent loads), then the next row's columns 8 at a time.  Does nothing
+// when the row pointer is malformed (*bad).
+__global__ void __launch_bounds__(256) dcsr_far(size_t S, double stride, UIN n, const UIN *__restrict__ row,
+                                                const UIN *__restrict__ col, const int *__restrict__ bad,
+                                                unsigned long long *__restrict__ far) {
+  if (*bad) return;
+  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const unsigned g = threadIdx.x & 7u, sh = threadIdx.x & 24u, gm = 0xFFu << sh;
   if (i >= S) return;
   const size_t j = (size_t)(i * stride);
-  UIN a = 1, b = n;  // first k in [1, n] with row[k] > j (row[n] = nnz > j)
-  while (a < b) {
-    const UIN m = a + (b - a) / 2;
-    if (row[m] > j) b = m;
-    else a = m + 1;
+  UIN a = 1, b = n;  // first k in [a, b] with row[k] > j (row[n] = nnz > j)
+  while (b - a >= 8u) {
+    const UIN step = (b - a) / 9u + 1u, k = a + min((g + 1u) * step, b - a);
+    const unsigned m = (__ballot_sync(gm, row[k] > j) & gm) >> sh;  // a suffix of the lanes, or none
+    const unsigned f = m ? __ffs(m) - 1u : 8u;
+    const UIN na = f ? a + min(f * step, b - a) + 1u : a;
+    if (f < 8u) b = a + min((f + 1u) * step, b - a);
+    a = min(na, b);
+  }
+  {
+    const UIN k = a + min(g, b - a);
+    const unsigned m = (__ballot_sync(gm, row[k] > j) & gm) >> sh;
+    a = m ? a + min((UIN)__ffs(m) - 1u, b - a) : b;
   }
   const size_t r = a - 1;
   const long long c = col[j];
   if (llabs(c - (long long)r) <= 1536) return;
   bool near_next = false;
   if (r + 1 < n)
-    for (UIN k = row[r + 1]; k < row[r + 2] && !near_next; k++) near_next = llabs((long long)col[k] - c - 1) <= 16;
-  if (!near_next) atomicAdd(far, 1ull);
+    for (UIN k = row[r + 1] + g; k < row[r + 2]; k += 8u) near_next |= llabs((long long)col[k] - c - 1) <= 16;
+  if (!(__ballot_sync(gm, near_next) & gm) && g == 0) atomicAdd(far, 1ull);
 }
 
-// Window keys: the column of every nonzero value, ~0 for a zero value
-// (sorted last, left out of the window choice as on the host).
-__global__ void dcsr_win_keys(size_t nnz, const UIN *__restrict__ col, const FPT *__restrict__ val,
-                              UIN *__restrict__ keys) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < nnz; q += stride)
-    keys[q] = val[q] != 0.0 ? col[q] : 0xFFFFFFFFu;
-}
-
-__global__ void dcsr_win_offsets(size_t nt, size_t T, size_t nnz, int *__restrict__ off) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t <= nt) off[t] = (int)std::min(t * T, nnz);
-}
-
-// One CTA per plan CTA tile: stage_windows' choice from the tile's sorted
-// keys - the first i with the most keys in [cs[i], cs[i] + W - 1), the
-// interval centred on them, clamped to [0, ne - W], started at an even column.
-__global__ void __launch_bounds__(256) dcsr_windows(size_t nt, const int *__restrict__ off,
-                                                    const UIN *__restrict__ keys, UIN W, UIN ne,
-                                                    UIN *__restrict__ tlo, UIN *__restrict__ tlen) {
-  __shared__ UIN sb[8], si[8], sj[8];
-  const size_t t = blockIdx.x;
-  if (t >= nt) return;
-  if (ne <= W) {
-    if (threadIdx.x == 0) {
-      tlo[t] = 0;
-      tlen[t] = ne;
-    }
-    return;
+// best_run by one CTA of 256 threads: h holds the counts of nb bins (bin i
+// at WH(i): a word of padding per 32 keeps the threads' runs of bins in
+// different banks) and becomes their exclusive prefix.
+__device__ __forceinline__ UIN WH(UIN i) { return i + (i >> 5); }
+__device__ UIN cta_best_run(UIN *h, UIN nb, UIN w, unsigned long long *red) {
+  const unsigned t = threadIdx.x, lane = t & 31u, wid = t >> 5;
+  const UIN per = (nb + 255u) / 256u, i0 = min(nb, t * per), i1 = min(nb, i0 + per);
+  UIN sum = 0;
+  for (UIN i = i0; i < i1; i++) sum += h[WH(i)];
+  UIN incl = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const UIN u = __shfl_up_sync(FULL, incl, d);
+    if ((int)lane >= d) incl += u;
   }
-  const UIN *cs = keys + off[t];
-  const UIN all = (UIN)(off[t + 1] - off[t]);
-  UIN a = 0, b = all;  // m: keys below the sentinel
-  while (a < b) {
-    const UIN mid = a + (b - a) / 2;
-    if (cs[mid] == 0xFFFFFFFFu) b = mid;
-    else a = mid + 1;
-  }
-  const UIN m = a;
-  UIN best = 0, bi = 0xFFFFFFFFu, bj = 0;
-  for (UIN i = threadIdx.x; i < m; i += blockDim.x) {
-    const uint64_t lim = (uint64_t)cs[i] + (W - 1);
-    UIN lo = i, hi = m;  // first j in [i, m) with cs[j] >= lim
-    while (lo < hi) {
-      const UIN mid = lo + (hi - lo) / 2;
-      if ((uint64_t)cs[mid] < lim) lo = mid + 1;
-      else hi = mid;
-    }
-    if (lo - i > best) {
-      best = lo - i;
-      bi = i;
-      bj = lo;
-    }
-  }
-  // the largest count, the smallest i among equal counts
-  for (int d = 16; d > 0; d >>= 1) {
-    const UIN ob = __shfl_down_sync(FULL, best, d), oi = __shfl_down_sync(FULL, bi, d),
-              oj = __shfl_down_sync(FULL, bj, d);
-    if (ob > best || (ob == best && oi < bi)) {
-      best = ob;
-      bi = oi;
-      bj = oj;
-    }
-  }
-  const unsigned w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31u) == 0) {
-    sb[w] = best;
-    si[w] = bi;
-    sj[w] = bj;
-  }
+  if (lane == 31) red[wid] = incl;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (unsigned k = 1; k < blockDim.x / 32; k++)
-      if (sb[k] > best || (sb[k] == best && si[k] < bi)) {
-        best = sb[k];
-        bi = si[k];
-        bj = sj[k];
-      }
-    long long l = 0;
-    if (m > 0) {
-      const long long span = (long long)cs[bj - 1] - (long long)cs[bi] + 1;
-      l = (long long)cs[bi] - ((long long)W - span) / 2;
-    }
-    l = l < 0 ? 0 : l;
-    l = l > (long long)(ne - W) ? (long long)(ne - W) : l;
-    tlo[t] = (UIN)l & ~1u;
-    tlen[t] = W;
+  UIN run = incl - sum;
+  for (unsigned k = 0; k < wid; k++) run += (UIN)red[k];
+  for (UIN i = i0; i < i1; i++) {
+    const UIN c = h[WH(i)];
+    h[WH(i)] = run;
+    run += c;
   }
+  if (t == 255) h[WH(nb)] = run;  // the total
+  __syncthreads();
+  unsigned long long best = 0;  // count, then the smallest start
+  for (UIN i = i0; i < i1; i++) {
+    const UIN cnt = h[WH(w < nb - i ? i + w : nb)] - h[WH(i)];
+    const unsigned long long k = ((unsigned long long)cnt << 32) | (0xFFFFFFFFu - i);
+    best = k > best ? k : best;
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    const unsigned long long o = __shfl_xor_sync(FULL, best, d);
+    best = o > best ? o : best;
+  }
+  if (lane == 0) red[wid] = best;
+  __syncthreads();
+  best = red[0];
+#pragma unroll
+  for (unsigned k = 1; k < 8; k++) best = red[k] > best ? red[k] : best;
+  __syncthreads();  // red and h are free again
+  return 0xFFFFFFFFu - (UIN)best;
+}
+
+// One CTA per plan CTA tile: stage_windows' choice.  Reads a quarter of the
+// columns (twice, the second time from L2); a sort of every tile's columns
+// and a search for the densest interval took 690 us of the 860 a plan's
+// kernels did at n = 1M, 14.9M nonzeros.
+__global__ void __launch_bounds__(256) dcsr_windows(WinGeom g, size_t T, size_t nnz, const UIN *__restrict__ col,
+                                                    UIN *__restrict__ tlo, UIN *__restrict__ tlen) {
+  __shared__ UIN h[8192 + 256 + 1];
+  __shared__ unsigned long long red[8];
+  const size_t a = blockIdx.x * T, e = min(nnz, a + T);
+  auto count = [&](UIN nb, UIN lo, UIN s) {
+    for (UIN i = threadIdx.x; i < WH(nb) + 1; i += 256) h[i] = 0;
+    __syncthreads();
+    // groups of 8 slots 0, 4, 8, ... of the tile (T is a multiple of 32)
+    for (size_t k = threadIdx.x;; k += 256) {
+      const size_t q = a + (k >> 3) * 32 + (k & 7u);
+      if (q >= e) break;
+      const UIN c = col[q];
+      if (c >= lo && ((c - lo) >> s) < nb) atomicAdd(&h[WH((c - lo) >> s)], 1u);
+    }
+    __syncthreads();
+  };
+  count(g.nb1, 0u, g.s1);
+  const UIN r = cta_best_run(h, g.nb1, g.l1, red) << g.s1;
+  count(g.nb2, r, g.s2);
+  const unsigned long long l = r + ((unsigned long long)cta_best_run(h, g.nb2, g.w2, red) << g.s2);
+  if (threadIdx.x == 0) {
+    tlo[blockIdx.x] = (UIN)min(l, (unsigned long long)(g.ne - g.W)) & ~1u;
+    tlen[blockIdx.x] = g.W;
+  }
+}
+
+__global__ void fill_u32(size_t n, UIN v, UIN *__restrict__ a) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) a[i] = v;
 }
 
 int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *col, const FPT *val, cudaStream_t s) {
@@ -888,66 +915,60 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
     return fail(ISPMV_ERR_UNSUPPORTED, "plan from a device CSR: the lane-interleaved kernel");
   if (p->opts.val_kind == ISPMV_VAL_F32_LO16 || p->opts.col_kind != ISPMV_COL_U32)
     return fail(ISPMV_ERR_UNSUPPORTED, "plan from a device CSR: FP64/FP32 values, u32 columns");
-  // the matrix is checked before any pass indexes through it
+  // the row pointer is checked before any pass indexes through it, the
+  // columns by the pass that copies them
+  struct Found {
+    unsigned long long far;
+    UIN nonempty;
+    int bad;
+  } *found, hf{};
+  DevTmp tmp(s);
   p->n = n;
   p->nnz = nnz;
-  DevTmp tmp(s);
-  int *bad;
   UIN *flag, *pos;
-  TRY(tmp.alloc(1, &bad));
+  TRY(tmp.alloc(1, &found));
   TRY(tmp.alloc((size_t)n + 1, &flag));
   TRY(tmp.alloc((size_t)n + 1, &pos));
-  ISPMV_TRY(cudaMemsetAsync(bad, 0, sizeof(int), s));
-  const unsigned gchk = (unsigned)std::min<size_t>(((size_t)std::max(n, nnz) + 255) / 256, (size_t)sm_count() * 16);
-  dcsr_check<<<std::max(1u, gchk), 256, 0, s>>>(n, nnz, row, col, bad);
-  TRY(check_launch("dcsr_check"));
-  dcsr_flags<<<(unsigned)(((size_t)n + 1 + 255) / 256), 256, 0, s>>>(n, row, flag);
-  TRY(check_launch("dcsr_flags"));
+  int *const bad = &found->bad;
+  ISPMV_TRY(cudaMemsetAsync(found, 0, sizeof *found, s));
+  dcsr_check_rows<<<(unsigned)(((size_t)n + 1 + 255) / 256), 256, 0, s>>>(n, nnz, row, flag, bad);
+  TRY(check_launch("dcsr_check_rows"));
   size_t tb = 0;
   ISPMV_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, flag, pos, (int)n + 1, s));
   void *tst;
   TRY(tmp.alloc(tb, reinterpret_cast<unsigned char **>(&tst)));
   ISPMV_TRY(cub::DeviceScan::ExclusiveSum(tst, tb, flag, pos, (int)n + 1, s));
-  int hbad = 0;
-  UIN nonempty = 0;
-  ISPMV_TRY(cudaMemcpyAsync(&hbad, bad, sizeof hbad, cudaMemcpyDeviceToHost, s));
-  ISPMV_TRY(cudaMemcpyAsync(&nonempty, pos + n, sizeof nonempty, cudaMemcpyDeviceToHost, s));
+  const size_t S = std::min<size_t>(nnz, 1u << 16);
+  const bool choose = p->opts.kernel == ISPMV_KERNEL_AUTO && p->opts.variant == 0;
+  if (choose && S) {
+    dcsr_far<<<(unsigned)((S * 8 + 255) / 256), 256, 0, s>>>(S, (double)nnz / (double)S, n, row, col, bad,
+                                                               &found->far);
+    TRY(check_launch("dcsr_far"));
+  }
+  ISPMV_TRY(cudaMemcpyAsync(&found->nonempty, pos + n, sizeof(UIN), cudaMemcpyDeviceToDevice, s));
+  ISPMV_TRY(cudaMemcpyAsync(&hf, found, sizeof hf, cudaMemcpyDeviceToHost, s));
   ISPMV_TRY(cudaStreamSynchronize(s));
-  if (hbad) return fail(ISPMV_ERR_ARG, "plan from a device CSR: malformed row pointer or a column >= n");
+  const char *malformed = "plan from a device CSR: malformed row pointer or a column >= n";
+  if (hf.bad) return fail(ISPMV_ERR_ARG, malformed);
+  const UIN nonempty = hf.nonempty;
   if (p->opts.kernel == ISPMV_KERNEL_AUTO) {
     // the compacted AXT's default (ispmv_plan_axt), with the scatter test
     // run on the device sample
     p->opts.kernel = ISPMV_KERNEL_WIDE;
-    if (p->opts.variant == 0) {
-      const bool long_rows = (double)nnz >= 16.0 * (double)n;
-      bool scattered = false;
-      const size_t S = std::min<size_t>(nnz, 1u << 16);
-      if (S) {
-        unsigned long long *dfar, hfar = 0;
-        TRY(tmp.alloc(1, &dfar));
-        ISPMV_TRY(cudaMemsetAsync(dfar, 0, sizeof *dfar, s));
-        dcsr_far<<<(unsigned)((S + 255) / 256), 256, 0, s>>>(S, (double)nnz / (double)S, n, row, col, dfar);
-        TRY(check_launch("dcsr_far"));
-        ISPMV_TRY(cudaMemcpyAsync(&hfar, dfar, sizeof hfar, cudaMemcpyDeviceToHost, s));
-        ISPMV_TRY(cudaStreamSynchronize(s));
-        scattered = (double)hfar / (double)S >= 0.05;
-      }
-      p->opts.variant = auto_variant(p, long_rows, scattered);
+    if (choose) {
+      p->opts.variant = auto_variant(p, (double)nnz >= 16.0 * (double)n, S && (double)hf.far / (double)S >= 0.05);
       p->no_win = nnz < WIN_MIN_NNZ;
     }
   }
   const WideCfg wc = wide_variant(p->opts.variant);
   if (!wc.ok || wc.tmem)
     return fail(ISPMV_ERR_UNSUPPORTED, "plan from a device CSR: the lane-interleaved kernel without TMEM staging");
-  if (wc.stg && nnz > 0x7FFFFFFFu)
-    return fail(ISPMV_ERR_UNSUPPORTED, "plan from a device CSR: per-CTA x windows up to 2^31 - 1 nonzeros");
   p->fmt = F_CSR;
   p->path = P_STREAM;
   p->slots = p->fslots = nnz;
   p->slots_pad = std::max(SS, (p->slots + SS - 1) / SS * SS);
   p->seg_slots = p->opts.units_per_warp <= 0 ? wide_seg(wc, p->slots_pad) : seg_slots_of(p, 1);
   p->nseg = (p->slots_pad + p->seg_slots - 1) / p->seg_slots;
-  const unsigned spl = (unsigned)wc.spl;
   void *vi;
   if (p->opts.val_kind == ISPMV_VAL_F64) TRY(dev_alloc(p, p->slots_pad, reinterpret_cast<double **>(&vi)));
   else TRY(dev_alloc(p, p->slots_pad, reinterpret_cast<float **>(&vi)));
@@ -963,57 +984,50 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
   }
   ISPMV_TRY(cudaMemsetAsync(p->heads, 0, p->slots_pad / 32 * sizeof(UIN), s));
   const unsigned gi = (unsigned)std::min<size_t>((p->slots_pad + 255) / 256, (size_t)sm_count() * 32);
-  if (p->opts.val_kind == ISPMV_VAL_F64)
-    dcsr_interleave<double><<<gi, 256, 0, s>>>(nnz, p->slots_pad, spl, col, val, static_cast<double *>(vi), p->col);
-  else
-    dcsr_interleave<float><<<gi, 256, 0, s>>>(nnz, p->slots_pad, spl, col, val, static_cast<float *>(vi), p->col);
+  auto interleave = [&](auto *v, auto spl_c) {
+    dcsr_interleave<std::remove_pointer_t<decltype(v)>, decltype(spl_c)::value>
+        <<<gi, 256, 0, s>>>(n, nnz, p->slots_pad, col, val, v, p->col, bad);
+  };
+  using S8 = std::integral_constant<int, 8>;
+  using S16 = std::integral_constant<int, 16>;
+  if (p->opts.val_kind == ISPMV_VAL_F64) {
+    if (wc.spl == 8) interleave(static_cast<double *>(vi), S8{});
+    else interleave(static_cast<double *>(vi), S16{});
+  } else {
+    if (wc.spl == 8) interleave(static_cast<float *>(vi), S8{});
+    else interleave(static_cast<float *>(vi), S16{});
+  }
   TRY(check_launch("dcsr_interleave"));
-  dcsr_rows<<<(unsigned)(((size_t)n + 255) / 256), 256, 0, s>>>(n, row, pos, p->heads, p->rowmap, p->empty);
+  dcsr_rows<<<(unsigned)(((size_t)n + 1 + 255) / 256), 256, 0, s>>>(n, row, pos, p->heads, p->rowmap, p->empty,
+                                                                      p->nseg, (UIN)p->seg_slots, p->segh);
   TRY(check_launch("dcsr_rows"));
-  dcsr_segh<<<(unsigned)((p->nseg + 255) / 256), 256, 0, s>>>(p->nseg, p->seg_slots, n, row, pos, p->segh);
-  TRY(check_launch("dcsr_segh"));
   size_t nt = 0;
   if (wc.stg) {
     // per-CTA x windows, as stage_windows picks them on the host
-    const UIN W = wc.cap & ~1u, ne = n & ~1u;
-    const size_t T = (size_t)WIDE_WARPS * p->seg_slots;
+    const WinGeom g = win_geom(n, wc.cap);
     nt = std::max<size_t>(1, (p->nseg + WIDE_WARPS - 1) / WIDE_WARPS);
-    UIN *tlo, *tlen, *keys = nullptr, *sorted = nullptr;
-    int *off;
+    UIN *tlo, *tlen;
     TRY(dev_alloc(p, nt, &tlo));
     TRY(dev_alloc(p, nt, &tlen));
-    TRY(tmp.alloc(nt + 1, &off));
-    if (p->no_win) {
+    if (!p->no_win && g.ne > g.W) {
+      dcsr_windows<<<(unsigned)nt, 256, 0, s>>>(g, (size_t)WIDE_WARPS * p->seg_slots, nnz, col, tlo, tlen);
+      TRY(check_launch("dcsr_windows"));
+    } else {  // no window, or all of x (but an odd last element)
       ISPMV_TRY(cudaMemsetAsync(tlo, 0, nt * sizeof(UIN), s));
-      ISPMV_TRY(cudaMemsetAsync(tlen, 0, nt * sizeof(UIN), s));
-    } else {
-    dcsr_win_offsets<<<(unsigned)((nt + 1 + 255) / 256), 256, 0, s>>>(nt, T, nnz, off);
-    TRY(check_launch("dcsr_win_offsets"));
-    if (ne > W && nnz) {
-      TRY(tmp.alloc(nnz, &keys));
-      TRY(tmp.alloc(nnz, &sorted));
-      dcsr_win_keys<<<gi, 256, 0, s>>>(nnz, col, val, keys);
-      TRY(check_launch("dcsr_win_keys"));
-      size_t sb = 0;
-      ISPMV_TRY(cub::DeviceSegmentedRadixSort::SortKeys(nullptr, sb, keys, sorted, (int)nnz, (int)nt, off, off + 1,
-                                                         0, 32, s));
-      void *sst;
-      TRY(tmp.alloc(sb, reinterpret_cast<unsigned char **>(&sst)));
-      ISPMV_TRY(cub::DeviceSegmentedRadixSort::SortKeys(sst, sb, keys, sorted, (int)nnz, (int)nt, off, off + 1, 0, 32,
-                                                         s));
-    }
-    dcsr_windows<<<(unsigned)nt, 256, 0, s>>>(nt, off, sorted, W, ne, tlo, tlen);
-    TRY(check_launch("dcsr_windows"));
+      fill_u32<<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(nt, p->no_win ? 0u : g.ne, tlen);
+      TRY(check_launch("fill_u32"));
     }
     p->xw.tlo = tlo;
     p->xw.tlen = tlen;
-    p->xw.cap = p->no_win ? 0 : W;
+    p->xw.cap = p->no_win ? 0 : g.W;
     p->xw.nwin = 1;
     p->xw.n = p->n;
   }
   TRY(alloc_records(p));
   if (wc.stg) p->xw.status = p->status;
+  ISPMV_TRY(cudaMemcpyAsync(&hf.bad, bad, sizeof hf.bad, cudaMemcpyDeviceToHost, s));
   ISPMV_TRY(cudaStreamSynchronize(s));
+  if (hf.bad) return fail(ISPMV_ERR_ARG, malformed);
   p->info.device_bytes = (uint64_t)(8 * nt) + (uint64_t)p->slots_pad * (vbytes(p) + 4) + p->slots_pad / 8;
   return ISPMV_OK;
 }

@@ -98,3 +98,25 @@ def test_padding_reads_no_x(env):
     for f in (F.getFormatDataAXC(0, csr, x)[1], F.getFormatDataAXT(0, 128, 8, 1, "NOC", csr, x)[1],
               F.getFormatDataAXT(0, 128, 8, 4, "NOC", csr, x)[1]):
         assert_parity(D.Plan(csr, f).spmv(torch.from_numpy(x).cuda()).cpu().numpy(), ref, absax, TOL_F64)
+
+
+@pytest.mark.parametrize("n", [3583, 3584, 3585, 3586, 8191, 9000, 70_001])
+def test_windows_host_device(env, n):
+    """Per-CTA x windows at sizes around the window's (3584): the device's
+    choice is the host's, inside x, and the product is right; far columns at
+    both ends of x, tiles past the last slot."""
+    torch, D, F, _ = env
+    rng = np.random.default_rng(n)
+    lengths = rng.integers(1, 9, n)
+    row, col, val = rows_of(np.zeros(n, int), n, n)
+    row[1:] = np.cumsum(lengths)
+    near = (np.repeat(np.arange(n), lengths) + rng.integers(-40, 41, int(row[-1]))) % n
+    col = np.where(rng.random(len(near)) < 0.6, near, rng.integers(0, n, len(near))).astype(np.uint32)
+    val = rng.standard_normal(len(col))
+    host = D.Plan(F.CSR(row, col, val), None, kernel="wide", variant=26)
+    dev = D.Plan.from_device_csr(D.to_device(row), D.to_device(col), D.to_device(val), kernel="wide", variant=26)
+    a, b = host.export_stream(), dev.export_stream()
+    for k in ("val", "col", "heads", "segh", "win_lo", "win_len"):
+        assert np.array_equal(a[k], b[k]), k
+    assert np.all(a["win_lo"] % 2 == 0) and np.all(a["win_lo"].astype(int) + a["win_len"] <= n)
+    check(env, row, col, val, dev, "f64")
