@@ -12,13 +12,13 @@
 //   int_axc         8 lanes per row, lane k takes element k of every brick.
 //   int_k1 / k1p    8 lanes per chunk (lane = row of the chunk): each column
 //                   of a chunk is one coalesced 64-byte load of values.
-//   int_axt_noc_h1  8 lanes per tile, 4 tiles per warp step; tile sums are
-//                   combined per row with a segmented warp scan, so a row
-//                   costs one atomic per warp instead of one per tile.
+//   int_axt_noc_h1  4 slots per lane (two lanes per tile) and a segmented
+//                   warp scan per 128 slots, so a row costs one atomic per
+//                   warp instead of one per tile.
 //   int_axt_noc     one warp per tile: lane = (sub-row group, column),
 //                   columns reduced over sub-rows, then per-row runs of the
 //                   8 columns combined before the atomics.
-//   int_axt_com_h1  32 slots per warp step with a segmented scan; every slot
+//   int_axt_com_h1  the same kernel; every slot
 //                   carrying a descriptor, and every block start, opens a
 //                   segment, so row-0 segments whose descriptor is 0 are
 //                   summed (the reference skips them, M:1555) and segment
@@ -104,44 +104,145 @@ __global__ void k_order(UIN len, const UIN *__restrict__ permi, const FPT *__res
   if (i < len) ord[permi[i]] = dis[i];
 }
 
-// AXT NOC tileH=1 (M:1385-1404): y[rwp[t]] += sum_k ax[16t+k] * ax[16t+8+k].
-// Each warp covers STEPS*4 consecutive tiles.
-constexpr int H1_STEPS = 8;
-__global__ void __launch_bounds__(TPB) k_axt_noc_h1(UIN tileNum, const FPT *__restrict__ ax,
-                                                    const UIN *__restrict__ rwp, FPT *__restrict__ y) {
-  const unsigned lane = threadIdx.x & 31u, lane8 = lane & 7u;
+// AXT with tileH = 1: NOC (M:1385-1404), y[rwp[t]] += sum_k ax[16t+k] *
+// ax[16t+8+k], and COM (M:1517-1566), true segmented sums.  A lane takes 4
+// consecutive slots (half a tile), so one segmented warp scan serves 128
+// slots: COM at n = 1M, 14.9M nonzeros: 53 us, with one slot per lane (25
+// shuffles per 32 slots) 80; the bytes alone take 46.  A slot with a row start
+// (NOC: a tile of another row than the one before; COM: a descriptor or a
+// block start) ends the open row: rows that start and end inside a lane are
+// added to y there, the others by the lane that ends them, from the scan.  A
+// warp walks SEG_STEPS steps, the next step's loads in flight, and carries
+// its open row along.  VEC: ax and rwp aligned for 16-byte loads.
+constexpr int SEG_STEPS = 4;
+constexpr int SEG_SLOTS_WARP = SEG_STEPS * 128;  // a multiple of every COM block size
+
+template <bool VEC>
+__device__ __forceinline__ void ld4(const double *p, double (&d)[4]) {
+  if (VEC) {
+    const double2 a = ld_stream(reinterpret_cast<const double2 *>(p)), b = ld_stream(reinterpret_cast<const double2 *>(p) + 1);
+    d[0] = a.x, d[1] = a.y, d[2] = b.x, d[3] = b.y;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++) d[k] = ld_stream(p + k);
+  }
+}
+template <bool VEC>
+__device__ __forceinline__ void ld4(const float *p, float (&d)[4]) {
+  if (VEC) {
+    const float4 a = ld_stream(reinterpret_cast<const float4 *>(p));
+    d[0] = a.x, d[1] = a.y, d[2] = a.z, d[3] = a.w;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++) d[k] = ld_stream(p + k);
+  }
+}
+
+template <bool COM, bool VEC>
+__global__ void __launch_bounds__(TPB) k_axt_h1(size_t slots, UIN bs, UIN lg, const FPT *__restrict__ ax,
+                                                const UIN *__restrict__ rwp, FPT *__restrict__ y) {
+  const unsigned lane = threadIdx.x & 31u;
   const size_t warp = ((size_t)blockIdx.x * TPB + threadIdx.x) >> 5;
-  const size_t t0 = warp * (size_t)(H1_STEPS * 4);
-  if (t0 >= tileNum) return;
-  UIN crow = NO_ROW;
+  const size_t p0 = warp * (size_t)SEG_SLOTS_WARP;
+  if (p0 >= slots) return;
+  const unsigned lt = (1u << lane) - 1u;
+  FPT a[4] = {}, b[4] = {};  // the step's values and x copies
+  UIN d[4] = {};             // COM: descriptors; NOC: d[0] the tile's row, d[1] the row before (NO_ROW: none)
+  auto load = [&](size_t p) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) a[k] = b[k] = (FPT)0;
+    if (COM) d[0] = d[1] = d[2] = d[3] = 0;
+    if (p >= slots) return;  // slots is a multiple of 8: a lane's four slots exist or not together
+    const FPT *q = ax + (p >> 3) * 16 + (p & 7u);
+    ld4<VEC>(q, a);
+    ld4<VEC>(q + 8, b);
+    if (COM) {
+      if (VEC) {
+        const uint4 u = ld_stream(reinterpret_cast<const uint4 *>(rwp + p));
+        d[0] = u.x, d[1] = u.y, d[2] = u.z, d[3] = u.w;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++) d[k] = ld_stream(rwp + p + k);
+      }
+    } else {
+      const size_t t = p >> 3;
+      d[0] = ldg(rwp + t);
+      d[1] = p > p0 ? ldg(rwp + t - 1) : NO_ROW;
+    }
+  };
+  load(p0 + 4 * lane);
+  UIN crow = NO_ROW;  // the row open at the end of the last step, and its sum
   double csum = 0.0;
-  for (int st = 0; st < H1_STEPS; st++) {
-    const size_t t = t0 + (size_t)st * 4 + (lane >> 3);
-    const bool live = t < tileNum;
-    double p = 0.0;
-    UIN r = NO_ROW;
-    if (live) {
-      p = (double)ld_stream(ax + t * 16 + lane8) * (double)ld_stream(ax + t * 16 + 8 + lane8);
-      r = rwp[t];
+#pragma unroll 1
+  for (int st = 0; st < SEG_STEPS; st++) {
+    const size_t p = p0 + (size_t)st * 128 + 4 * lane;
+    double v[4];
+    UIN hr[4];  // row starting at the slot
+    bool h[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      v[k] = (double)a[k] * (double)b[k];
+      if (COM) {
+        h[k] = p < slots && (d[k] != 0 || ((p + k) & (bs - 1)) == 0);
+        hr[k] = d[k] >> lg;
+      } else {
+        h[k] = k == 0 && p < slots && (p & 7u) == 0 && d[0] != d[1];
+        hr[k] = d[0];
+      }
     }
-    // within-tile sum (lane8 == 0 holds it)
-    p += __shfl_xor_sync(FULL, p, 4);
-    p += __shfl_xor_sync(FULL, p, 2);
-    p += __shfl_xor_sync(FULL, p, 1);
-    if (lane8) p = 0.0;
-    const UIN rprev = __shfl_up_sync(FULL, r, 1);
-    const bool head = (lane == 0) ? (r != crow) : (r != rprev);
-    if (lane == 0) {
-      if (!head) p += csum;
-      else if (crow != NO_ROW) atomicAdd(y + crow, (FPT)csum);  // the carried run ended last step
+    if (st + 1 < SEG_STEPS) load(p + 128);
+    double pre = 0.0, acc = 0.0;
+    UIN lr = NO_ROW;  // row of my last start
+    bool f = false;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (h[k]) {
+        if (f) atomicAdd(y + lr, (FPT)acc);  // a row that starts and ends in my four slots
+        else pre = acc;
+        f = true;
+        lr = hr[k];
+        acc = 0.0;
+      }
+      acc += v[k];
     }
-    const double s = warp_seg_scan(p, head);
-    const UIN rnext = __shfl_down_sync(FULL, r, 1);
-    if (lane < 31 && r != rnext && r != NO_ROW) atomicAdd(y + r, (FPT)s);
-    crow = __shfl_sync(FULL, r, 31);
-    csum = __shfl_sync(FULL, s, 31);
+    if (!f) {
+      pre = acc;
+      acc = 0.0;
+    }
+    if (lane == 0) pre += csum;
+    const unsigned F = __ballot_sync(FULL, f);
+    const unsigned below = F & lt;
+    const int from = (F & (lt | (1u << lane))) ? 31 - __clz(F & (lt | (1u << lane))) : 0;
+    const int reach = (int)lane - from;  // lanes between me and the last start at or before me
+    const int maxreach = (int)__reduce_max_sync(FULL, (unsigned)reach);
+    double I = f ? acc : pre;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+      if (k > maxreach) break;
+      const double u = __shfl_up_sync(FULL, I, k);
+      if (reach >= k) I += u;
+    }
+    double E = __shfl_up_sync(FULL, I, 1);
+    if (lane == 0) E = 0.0;
+    const UIN prow = __shfl_sync(FULL, lr, below ? 31 - __clz(below) : 0);
+    const UIN open = below ? prow : crow;  // the row open at my first slot
+    if (f && open != NO_ROW) atomicAdd(y + open, (FPT)(E + pre));
+    const UIN last = __shfl_sync(FULL, lr, F ? 31 - __clz(F) : 0);
+    if (F) crow = last;
+    csum = __shfl_sync(FULL, I, 31);
   }
   if (lane == 0 && crow != NO_ROW) atomicAdd(y + crow, (FPT)csum);
+}
+
+template <bool COM>
+int launch_axt_h1(size_t slots, UIN bs, UIN lg, const FPT *ax, const UIN *rwp, FPT *y, cudaStream_t s,
+                  const char *what) {
+  const size_t warps = (slots + SEG_SLOTS_WARP - 1) / SEG_SLOTS_WARP;
+  const unsigned g = (unsigned)((warps * 32 + TPB - 1) / TPB);
+  const bool vec = ((reinterpret_cast<uintptr_t>(ax) | (COM ? reinterpret_cast<uintptr_t>(rwp) : 0)) & 15u) == 0;
+  if (vec) k_axt_h1<COM, true><<<g, TPB, 0, s>>>(slots, bs, lg, ax, rwp, y);
+  else k_axt_h1<COM, false><<<g, TPB, 0, s>>>(slots, bs, lg, ax, rwp, y);
+  return check_launch(what);
 }
 
 // AXT NOC tileH>1 (M:1443-1474): one warp per tile.
@@ -163,52 +264,6 @@ __global__ void __launch_bounds__(TPB) k_axt_noc(UIN tileNum, UIN th, const FPT 
   const double v = warp_seg_scan(lane < 8 ? s : 0.0, head);
   const UIN rnext = __shfl_down_sync(FULL, r, 1);
   if (lane < 8 && r != rnext) atomicAdd(y + r, (FPT)v);
-}
-
-// AXT COM tileH=1 (M:1517-1566), true segmented sums.
-constexpr int COM_STEPS = 16;
-__global__ void __launch_bounds__(TPB) k_axt_com_h1(UIN bs, UIN lg, UIN lenRWP, const FPT *__restrict__ ax,
-                                                    const UIN *__restrict__ rwp, FPT *__restrict__ y) {
-  const unsigned lane = threadIdx.x & 31u;
-  const size_t warp = ((size_t)blockIdx.x * TPB + threadIdx.x) >> 5;
-  const size_t p0 = warp * (size_t)(COM_STEPS * 32);
-  if (p0 >= lenRWP) return;
-  UIN crow = NO_ROW;
-  double csum = 0.0;
-  for (int st = 0; st < COM_STEPS; st++) {
-    const size_t p = p0 + (size_t)st * 32 + lane;
-    const bool live = p < lenRWP;
-    double v = 0.0;
-    bool head = false;
-    UIN hrow = 0;
-    if (live) {
-      const size_t a = (p >> 3) * 16 + (p & 7);
-      v = (double)ld_stream(ax + a) * (double)ld_stream(ax + a + 8);
-      const UIN d = rwp[p];
-      head = (d != 0) || ((p & (bs - 1)) == 0);
-      hrow = d >> lg;
-    }
-    // row of each lane's run: the row of the latest head at or before it
-    int hl = head ? (int)lane : -1;
-#pragma unroll
-    for (unsigned d = 1; d < 32; d <<= 1) {
-      const int u = __shfl_up_sync(FULL, hl, d);
-      if (lane >= d) hl = max(hl, u);
-    }
-    const UIN hr = __shfl_sync(FULL, hrow, hl < 0 ? 0 : hl);
-    const UIN r = live ? (hl < 0 ? crow : hr) : NO_ROW;
-    const bool seg = (lane == 0) ? (head || r != crow) : (head || !live);
-    if (lane == 0) {
-      if (!seg) v += csum;
-      else if (crow != NO_ROW) atomicAdd(y + crow, (FPT)csum);  // the carried run ended last step
-    }
-    const double s = warp_seg_scan(v, seg);
-    const bool nexthead = __shfl_down_sync(FULL, (unsigned)(head || !live), 1) != 0;
-    if (lane < 31 && live && nexthead && r != NO_ROW) atomicAdd(y + r, (FPT)s);
-    crow = __shfl_sync(FULL, r, 31);
-    csum = __shfl_sync(FULL, s, 31);
-  }
-  if (lane == 0 && crow != NO_ROW) atomicAdd(y + crow, (FPT)csum);
 }
 
 inline unsigned blocks_for(size_t threads) { return (unsigned)((threads + TPB - 1) / TPB); }
@@ -261,9 +316,8 @@ ISPMV_API int ispmv_dev_int_k1p(unsigned char mask, UIN chunkNum, const FPT *val
 ISPMV_API int ispmv_dev_int_axt_noc_h1(UIN tileNum, const FPT *ax, const UIN *rwp, FPT *y, void *stream) {
   if (tileNum == 0) return ISPMV_OK;
   if (!ax || !rwp || !y) return ISPMV_ERR_ARG;
-  const size_t warps = ((size_t)tileNum + lit::H1_STEPS * 4 - 1) / (lit::H1_STEPS * 4);
-  lit::k_axt_noc_h1<<<lit::blocks_for(warps * 32), lit::TPB, 0, as_stream(stream)>>>(tileNum, ax, rwp, y);
-  return check_launch("ispmv_dev_int_axt_noc_h1");
+  return lit::launch_axt_h1<false>((size_t)tileNum * 8, 8, 0, ax, rwp, y, as_stream(stream),
+                                   "ispmv_dev_int_axt_noc_h1");
 }
 
 ISPMV_API int ispmv_dev_int_axt_noc(UIN tileNum, UIN tileHeight, const FPT *ax, const UIN *rwp, FPT *y,
@@ -283,9 +337,7 @@ ISPMV_API int ispmv_dev_int_axt_com_h1(UIN bn, UIN bs, UIN log, UIN thw, UIN tn,
   if ((uint64_t)tn * 8 != lenRWP || (uint64_t)tn * 16 != lenAX || (uint64_t)bn * bs < lenRWP) return ISPMV_ERR_ARG;
   if (lenRWP == 0) return ISPMV_OK;
   if (!ax || !rwp || !y) return ISPMV_ERR_ARG;
-  const size_t warps = ((size_t)lenRWP + lit::COM_STEPS * 32 - 1) / (lit::COM_STEPS * 32);
-  lit::k_axt_com_h1<<<lit::blocks_for(warps * 32), lit::TPB, 0, as_stream(stream)>>>(bs, log, lenRWP, ax, rwp, y);
-  return check_launch("ispmv_dev_int_axt_com_h1");
+  return lit::launch_axt_h1<true>(lenRWP, bs, log, ax, rwp, y, as_stream(stream), "ispmv_dev_int_axt_com_h1");
 }
 
 #ifndef ISPMV_FPT_FLOAT  // FP64 only

@@ -120,3 +120,43 @@ def test_windows_host_device(env, n):
         assert np.array_equal(a[k], b[k]), k
     assert np.all(a["win_lo"] % 2 == 0) and np.all(a["win_lo"].astype(int) + a["win_len"] <= n)
     check(env, row, col, val, dev, "f64")
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("nnz", [1, 7, 8, 127, 128, 129, 511, 512, 513, 1025, 30_001])
+def test_axt_kernels_steps(env, nnz, offset):
+    """The tileH = 1 kernels (x-baked arrays) around a warp's step (128 slots)
+    and range (512), 16-byte aligned arrays or not; the GPU's conversion of the
+    same matrix at tile heights that fill tiles in ax order and in slot order."""
+    torch, D, F, orc = env
+    n = max(3, nnz // 3)
+    rng = np.random.default_rng(nnz)
+    cuts = np.sort(rng.integers(0, nnz + 1, n - 1))
+    lengths = np.minimum(np.diff(np.concatenate([[0], cuts, [nnz]])), n)
+    row, col, val = rows_of(lengths, n, nnz)
+    x = rng.uniform(-1, 1, n)
+    csr = F.CSR(row, col, val)
+    ref, absax = orc.cf_csr(row, col, val, x), orc.abs_csr(row, col, val, x)
+
+    def up(a):  # a device copy that starts `offset` elements into its buffer
+        t = D.to_device(a)
+        buf = torch.zeros(t.numel() + offset, dtype=t.dtype, device="cuda")
+        buf[offset:] = t
+        return buf[offset:]
+
+    y = torch.zeros(n, dtype=torch.float64, device="cuda")
+    noc = F.getFormatDataAXT(0, 128, 8, 1, "NOC", csr, x)[1]
+    D.int_axt_noc_h1(noc.c.tileN, up(noc.ax), up(noc.sec), y)
+    assert_parity(y.cpu().numpy(), ref, absax, TOL_F64, "NOC")
+    for bs in (8, 512):
+        com = F.getFormatDataAXT(0, bs, 8, 1, "COM", csr, x)[1]
+        c = com.c
+        y.zero_()
+        D.int_axt_com_h1((c.lenSEC + bs - 1) // bs, bs, c.log, 8, c.tileN, c.lenAX, c.lenSEC, up(com.ax), up(com.sec), y)
+        assert_parity(y.cpu().numpy(), ref, absax, TOL_F64, f"COM {bs}")
+    dev = [D.to_device(a) for a in (row, col, val, x)]
+    for mode, th in (("COM", 1), ("NOC", 1), ("NOC", 3), ("NOC", 64), ("NOC", 65)):
+        got = D.DeviceAXT(*dev, th=th, mode=mode).to_host()
+        want = F.getFormatDataAXT(0, 128, 8, th, mode, csr, x)[1]
+        for k in ("con", "ax", "sec"):
+            assert np.array_equal(got[k], getattr(want, k)), (mode, th, k)
