@@ -1803,63 +1803,61 @@ bool tmem_plan(const ispmv_plan_s *p) {
   return p->opts.kernel == ISPMV_KERNEL_WIDE && wide_variant(p->opts.variant).tmem;
 }
 
+// Slots per group of the SpMM kernel, whole chunks (a multiple of 64): an even
+// share of as many loads of the GPU's `held` groups as keep it at 192 or less.
+// Longer parts spread the resident groups over more of the matrix (less of X
+// found in L2), shorter ones pay their start more often: k = 8 / 32 on
+// power-law rows 144 / 323 us at 128 slots, 138 / 330 at 192, 149 / 339 at 256.
+size_t spmm_part(size_t slots, size_t held) {
+  const size_t loads = std::max<size_t>(1, (slots + held * 192 - 1) / (held * 192));
+  return std::max<size_t>(64, ((slots + loads * held - 1) / (loads * held) + 63) / 64 * 64);
+}
+
 // One pass per block of CB = G*W right-hand sides (G lanes per group, W
 // columns per lane).
-template <int G, int W, typename VT, int SPL>
-int spmm_blocks(ispmv_plan_s *p, UIN k, const FPT *X, FPT *Y, cudaStream_t s) {
+template <int G, int W, int T, int MINB, bool VEC, typename VT>
+int spmm_blocks(ispmv_plan_s *p, UIN k, const FPT *X, FPT *Y, cudaStream_t s, const char *name) {
   constexpr int NG = 32 / G, CB = G * W;
-  const size_t nparts = p->nseg * NG, nrec = 2 * nparts;
+  const size_t part = spmm_part(p->slots_pad, (size_t)sm_count() * MINB * 8 * NG);
+  const size_t nparts = (p->slots_pad + part - 1) / part, ctas = (nparts + 8 * NG - 1) / (8 * NG), nrec = 2 * ctas;
   if (p->mm_rows_cap < nrec) {
-    TRY(dev_alloc(p, std::max<size_t>(1, nrec), &p->mm_row));
+    TRY(dev_alloc(p, nrec, &p->mm_row));
     p->mm_rows_cap = nrec;
   }
-  if (p->mm_cap < nrec * CB) {
-    TRY(dev_alloc(p, std::max<size_t>(1, nrec * CB), &p->mm_sum));
-    p->mm_cap = nrec * CB;
+  if (p->mm_cap < (nparts + nrec) * CB) {
+    TRY(dev_alloc(p, (nparts + nrec) * CB, &p->mm_sum));
+    p->mm_cap = (nparts + nrec) * CB;
   }
-  const VT *val = static_cast<const VT *>(p->val);
+  const unsigned spl = il_spl(p);
+  const mm::Stream st{p->slots, p->slots_pad, p->seg_slots, p->val, p->col, p->heads, p->segh,
+                      spl == 16 ? 4u : spl == 8 ? 3u : 0u};
   for (UIN j0 = 0; j0 < k; j0 += CB) {
-    mm::Out o{Y, p->rowmap, p->mm_row, p->mm_sum, k, j0, std::min<UIN>(CB, k - j0)};
-    const unsigned g = (unsigned)((p->nseg * 32 + 255) / 256);
-    mm::stream_spmm<G, W, VT, SPL><<<g, 256, 0, s>>>(p->slots, p->slots_pad, p->seg_slots, p->nseg, val, p->col,
-                                                     p->heads, p->segh, X, o);
-    TRY(check_launch("stream_spmm"));
+    mm::Out o{Y, p->rowmap, p->mm_sum, p->mm_row, p->mm_sum + nparts * CB, k, j0, std::min<UIN>(CB, k - j0)};
+    mm::stream_spmm<G, W, T, MINB, VEC, VT><<<(unsigned)ctas, 256, 0, s>>>(st, part, nparts, X, o);
+    TRY(check_launch(name));
     p->kname = last_launch();
-    const size_t work = std::max(nrec, p->nempty) * CB;
-    mm::spmm_fixup<CB><<<(unsigned)((work + 255) / 256), 256, 0, s>>>(nrec, p->mm_row, p->mm_sum, p->empty,
-                                                                      p->nempty, o);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((std::max(nrec, p->nempty) * CB + 255) / 256));
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    ISPMV_TRY(cudaLaunchKernelEx(&cfg, mm::spmm_fixup<CB>, nrec, (const UIN *)p->empty, p->nempty, o));
     TRY(check_launch("spmm_fixup"));
   }
   return ISPMV_OK;
 }
 
-// Four columns per lane: one pass per block of CB = 4G right-hand sides.
-template <int G, int T, int MINB, typename VT, int SPL>
-int spmm_blocks4(ispmv_plan_s *p, UIN k, const FPT *X, FPT *Y, cudaStream_t s) {
-  constexpr int NG = 32 / G, CB = 4 * G;
-  const size_t nparts = p->nseg * NG, nrec = 2 * nparts;
-  if (p->mm_rows_cap < nrec) {
-    TRY(dev_alloc(p, std::max<size_t>(1, nrec), &p->mm_row));
-    p->mm_rows_cap = nrec;
-  }
-  if (p->mm_cap < nrec * CB) {
-    TRY(dev_alloc(p, std::max<size_t>(1, nrec * CB), &p->mm_sum));
-    p->mm_cap = nrec * CB;
-  }
-  const VT *val = static_cast<const VT *>(p->val);
-  for (UIN j0 = 0; j0 < k; j0 += CB) {
-    mm::Out o{Y, p->rowmap, p->mm_row, p->mm_sum, k, j0, std::min<UIN>(CB, k - j0)};
-    const unsigned g = (unsigned)((p->nseg * 32 + 255) / 256);
-    mm::stream_spmm4<G, T, MINB, VT, SPL><<<g, 256, 0, s>>>(p->slots, p->slots_pad, p->seg_slots, p->nseg, val,
-                                                            p->col, p->heads, p->segh, X, o);
-    TRY(check_launch("stream_spmm4"));
-    p->kname = last_launch();
-    const size_t work = std::max(nrec, p->nempty) * CB;
-    mm::spmm_fixup<CB><<<(unsigned)((work + 255) / 256), 256, 0, s>>>(nrec, p->mm_row, p->mm_sum, p->empty,
-                                                                      p->nempty, o);
-    TRY(check_launch("spmm_fixup"));
-  }
-  return ISPMV_OK;
+// Two columns per lane: 16-byte X loads where k is even and X and Y are
+// 16-byte aligned, else column by column.
+template <int G, typename VT>
+int spmm_two(ispmv_plan_s *p, UIN k, const FPT *X, FPT *Y, cudaStream_t s) {
+  if ((k & 1u) == 0 && k < (1u << 29) && ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15u) == 0)
+    return spmm_blocks<G, 2, 8, 3, true, VT>(p, k, X, Y, s, "stream_spmm");
+  return spmm_blocks<G, 2, 8, 3, false, VT>(p, k, X, Y, s, "stream_spmm");
 }
 
 // RHS block 8, 16 or 32 columns (ispmv_plan_opts.rhs_block, else by k).
@@ -1868,35 +1866,23 @@ int spmm_blocks4(ispmv_plan_s *p, UIN k, const FPT *X, FPT *Y, cudaStream_t s) {
 // lanes per group); AUTO the four-column form for blocks of 16 and 32
 // columns where it applies, else two (on 8-column blocks the two-column
 // form is the faster with FP64 values).
-template <typename VT, int SPL>
-int spmm_run_spl(ispmv_plan_s *p, UIN k, const FPT *X, FPT *Y, cudaStream_t s) {
+template <typename VT>
+int spmm_run(ispmv_plan_s *p, UIN k, const FPT *X, FPT *Y, cudaStream_t s) {
   int g = p->opts.rhs_block;
   if (g != 8 && g != 16 && g != 32) g = k <= 8 ? 8 : k <= 16 ? 16 : 32;
-  const bool four_ok = (k & 3u) == 0 && ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 31u) == 0;
+  const bool four_ok = (k & 3u) == 0 && k < (1u << 29) && ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 31u) == 0;
   const int kind = p->opts.spmm_kernel;
   if (kind == ISPMV_KERNEL_WIDE && !four_ok)
     return fail(ISPMV_ERR_UNSUPPORTED,
                 "ispmv_plan_spmm: four columns per lane need k a multiple of 4 and X, Y 32-byte aligned");
   if (four_ok && (kind == ISPMV_KERNEL_WIDE || (kind == ISPMV_KERNEL_AUTO && g > 8))) {
-    if (g == 8) return spmm_blocks4<2, 8, 2, VT, SPL>(p, k, X, Y, s);
-    if (g == 16) return spmm_blocks4<4, 4, 3, VT, SPL>(p, k, X, Y, s);
-    return spmm_blocks4<8, 8, 2, VT, SPL>(p, k, X, Y, s);
+    if (g == 8) return spmm_blocks<2, 4, 4, 3, true, VT>(p, k, X, Y, s, "stream_spmm4");
+    if (g == 16) return spmm_blocks<4, 4, 8, 2, true, VT>(p, k, X, Y, s, "stream_spmm4");
+    return spmm_blocks<8, 4, 8, 2, true, VT>(p, k, X, Y, s, "stream_spmm4");
   }
-  if (g == 8) return spmm_blocks<4, 2, VT, SPL>(p, k, X, Y, s);
-  if (g == 16) return spmm_blocks<8, 2, VT, SPL>(p, k, X, Y, s);
-  return spmm_blocks<16, 2, VT, SPL>(p, k, X, Y, s);
-}
-
-// The plan's stream layout as a template argument: slot order, or lane-
-// interleaved with 8 or 16 slots per lane.
-template <typename VT>
-int spmm_run(ispmv_plan_s *p, UIN k, const FPT *X, FPT *Y, cudaStream_t s) {
-  switch (il_spl(p)) {
-    case 0: return spmm_run_spl<VT, 0>(p, k, X, Y, s);
-    case 8: return spmm_run_spl<VT, 8>(p, k, X, Y, s);
-    case 16: return spmm_run_spl<VT, 16>(p, k, X, Y, s);
-    default: return fail(ISPMV_ERR_UNSUPPORTED, "ispmv_plan_spmm: lane-interleaved plans of 8 or 16 slots per lane");
-  }
+  if (g == 8) return spmm_two<4, VT>(p, k, X, Y, s);
+  if (g == 16) return spmm_two<8, VT>(p, k, X, Y, s);
+  return spmm_two<16, VT>(p, k, X, Y, s);
 }
 }  // namespace
 

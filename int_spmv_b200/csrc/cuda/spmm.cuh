@@ -1,19 +1,37 @@
 // spmm.cuh - multi-RHS SpMM on the slot stream: Y = A X, X and Y row-major
-// n x k (FP64), one plan's slot stream read once for all k right-hand sides.
+// n x k (FP64), one plan's slot stream read once per block of up to 32
+// right-hand sides.
 //
-// A warp splits into 32/G groups of G lanes; lane jl of a group owns the W
-// columns j0 + W*jl .. of the current column block (G*W = 8, 16 or 32
-// columns).  Each group walks its own contiguous part of the warp's segment:
-// G slots' values and columns are loaded per step (one per lane, coalesced)
-// and broadcast with shuffles, each lane reads its W-wide piece of row
-// X[col] (the group reads a contiguous row piece of X) and accumulates.
-// Row starts come from the
-// stream's bitmap; a row that ends inside the group's part is written to Y
-// directly, the runs open at the part's two ends become G-wide records that
-// spmm_fixup adds per row.  Deterministic, no atomics.  SPL > 0 reads a
-// plan whose values and columns are stored lane-interleaved for stream_wide
-// (wide::il_pos_c with SPL slots per lane); SPL = 0 a plan in slot order.
+// A warp splits into NG = 32/G groups of G lanes; lane jl of a group owns the
+// W columns j0 + W*jl .. of the column block (G*W = 8, 16 or 32 columns).
+// Each group walks its own contiguous part of the slot stream.  Row starts
+// come from the stream's bitmap; a row that ends inside the part is written
+// to Y directly.  Rows that cross parts are joined at the CTA's end by the
+// group they start in; only the runs open at the CTA's two ends become
+// G*W-wide records that spmm_fixup adds per row.  Deterministic, no atomics.
+//
+// What bounds it: a slot costs G*W*8 bytes of X, gathered through L1 (a tag
+// lookup and 64 bytes per SM and cycle) and, past 126 MB of X, from DRAM.  The
+// kernel therefore keeps the other users of the L1 pipe small and as many X
+// pieces in flight as it can:
+//   - values and columns come in by cp.async, 16 bytes per lane, into a
+//     double-buffered chunk of 4G slots per group in shared memory, read back
+//     as broadcasts of 16 bytes (2 values, 4 columns); loading them slot by
+//     slot touched 24 lines per 32 nonzeros, three quarters of what X does;
+//   - no registers hold the stream, so 16-24 warps per SM keep 4 to 8 X pieces
+//     per lane in flight: four slots of a step are consumed, then the pieces of
+//     the same four slots of the next step are loaded into the registers freed
+//     (slot by slot, the loads outnumber the barriers a warp waits on, and the
+//     two-column form took 175 us where it takes 138 so);
+//   - parts are short (spmm_part): the warps resident at a time then work on
+//     neighbouring rows, whose columns' X rows stay in L2 (k = 32, 256 MB of
+//     X: 323 us at 128 slots, 413 at 512), and the joins inside the CTA keep
+//     the records few (records per part cost 12-44 us of fix-up).
+// Power-law n = 1M, 14.9M nonzeros, FP64, against one slot's value and column
+// per lane and step: k = 8 237 us -> 149, k = 32 434 -> 364 (fresh X each time).
 #pragma once
+#include <type_traits>
+
 #include "wide.cuh"
 
 namespace ispmv {
@@ -22,327 +40,281 @@ namespace mm {
 struct Out {
   FPT *Y;
   const UIN *rowmap;
-  UIN *rec_row;     // 2 per part
-  double *rec_sum;  // 2 * G per part
+  double *head;     // G*W per part: the sum of the run open at the part's start
+  UIN *rec_row;     // 2 per CTA
+  double *rec_sum;  // 2 * G*W per CTA
   UIN k, j0, kb;    // row stride, first column of the block, columns in the block
 };
 
 __device__ __forceinline__ UIN real_row(const Out &o, UIN r) { return o.rowmap ? o.rowmap[r] : r; }
 
-template <bool B>
-struct BoolC {
-  static constexpr bool value = B;
+// The plan's stream: `lspl` = log2 of the slots per lane of a lane-interleaved
+// plan (wide::il_pos), 0 for one in slot order.
+struct Stream {
+  size_t nslots, nslots_pad, seg_slots;
+  const void *val;
+  const UIN *col, *heads, *segh;
+  unsigned lspl;
 };
 
-// One slot of a step as the group reads it from shared memory: its value
-// and the column of the slot at the same place in the next step.
-struct alignas(16) SlotRec {
-  double v;
-  UIN c, pad;
-};
+// Position of the vector of 1 << lv elements that starts at slot s.
+__device__ __forceinline__ size_t il_vec(size_t s, unsigned lspl, unsigned lv) {
+  if (!lspl) return s;
+  const size_t bt = (size_t)32 << lspl;
+  const unsigned r = (unsigned)(s & (bt - 1)), l = r >> lspl, k = r & ((1u << lspl) - 1u);
+  return (s & ~(bt - 1)) + ((size_t)(k >> lv) << (5 + lv)) + (l << lv);
+}
 
-// G lanes per group, W (1 or 2) consecutive right-hand sides per lane: a
-// pass covers CB = G*W columns.  A step of the group covers T = G slots:
-// each lane loads one slot's value and column (coalesced), one step ahead
-// of their use, and the group then works through the step's slots (8 at a
-// time when G = 16) in two phases:
-// first the X rows of all 8 slots are loaded into registers (W-wide vector
-// loads of the group's contiguous piece of each row), then the row starts
-// are handled and the products accumulated.  The loads of a step are thus in
-// flight together, ahead of the stores that row ends make to Y, and the
-// values and columns of the next step arrive meanwhile.
-template <int G, int W, typename VT, int SPL>
-__global__ void __launch_bounds__(256) stream_spmm(size_t nslots, size_t nslots_pad, size_t seg_slots, size_t nseg,
-                                                   const VT *__restrict__ val, const UIN *__restrict__ col,
-                                                   const UIN *__restrict__ heads, const UIN *__restrict__ segh,
-                                                   const FPT *__restrict__ X, Out o) {
-  static_assert(W == 1 || W == 2, "one or two right-hand sides per lane");
-  constexpr int NG = 32 / G;            // groups per warp = parts per segment
-  constexpr int CB = G * W;             // columns of one pass
-  constexpr int R = 1;                  // slots per lane and step
-  constexpr int T = G * R;              // slots per step (4, 8 or 16: within one bitmap word)
-  constexpr int SUB = T < 8 ? T : 8;    // slots whose X rows are loaded together
-  const unsigned lane = threadIdx.x & 31u, grp = lane / G, jl = lane % G;
-  const unsigned gmask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << (grp * G));
-  const size_t segid = ((size_t)blockIdx.x * 256 + threadIdx.x) >> 5;
-  if (segid >= nseg) return;
-  const size_t s0 = segid * seg_slots;
-  const size_t seg_end = min(s0 + seg_slots, nslots_pad);
-  const size_t part = (seg_end - s0) / NG;  // a multiple of 32
-  const size_t a = s0 + grp * part, b = a + part;
-  const size_t pid = segid * NG + grp;
-  // compressed row of the run open at slot a: starts before a, minus one
-  UIN cr = segh[segid];
-  for (size_t w = s0 >> 5; w < (a >> 5); w++) cr += __popc(__ldg(heads + w));
-  const bool a_head = (__ldg(heads + (a >> 5)) & 1u) != 0;  // a is 32-aligned
-  const UIN row_a = a_head ? NO_ROW : cr - 1u;
-  UIN row = cr - 1u;    // current run's row (advanced at each start)
-  bool have = !a_head;  // the current run has slots in this part
-  const unsigned j = jl * W;  // my first column in the block
-  const int ncol = j < o.kb ? min(W, (int)(o.kb - j)) : 0;  // my live columns (0..W)
-  // W-wide loads and stores need 16-byte rows: k even, j0 even, X and Y aligned
-  const bool vec = W == 2 && ncol == 2 && ((o.k | o.j0) & 1u) == 0 &&
-                   ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(o.Y)) & 15u) == 0;
-  const size_t xoff = o.j0 + j;
-  double acc[W];
+__device__ __forceinline__ void cp_async16(void *smem, const void *g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tma::smem_addr(smem)), "l"(g) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// W consecutive doubles of a row of X (or to a row of Y): one access of 8*W
+// bytes when VEC (aligned, all W columns live), else those below ncol.
+template <int W, bool VEC>
+__device__ __forceinline__ void ld_x(const double *p, int ncol, double (&d)[W]) {
+  if constexpr (VEC && W == 4) {
+    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(d[0]), "=d"(d[1]), "=d"(d[2]), "=d"(d[3])
+                 : "l"(p));
+  } else if constexpr (VEC) {
+    static_assert(W == 2, "two or four columns per lane");
+    asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(d[0]), "=d"(d[1]) : "l"(p));
+  } else {
 #pragma unroll
-  for (int w = 0; w < W; w++) acc[w] = 0.0;
-  if (jl == 0) {
-    o.rec_row[2 * pid] = NO_ROW;
-    o.rec_row[2 * pid + 1] = NO_ROW;
+    for (int w = 0; w < W; w++) d[w] = w < ncol ? __ldg(p + w) : 0.0;
   }
-#pragma unroll
-  for (int w = 0; w < W; w++) {
-    if (w < ncol) {
-      o.rec_sum[(2 * pid) * CB + j + w] = 0.0;
-      o.rec_sum[(2 * pid + 1) * CB + j + w] = 0.0;
-    }
-  }
-  auto put = [&](UIN r) {  // the run of row r ends: Y or the part's head record
-#pragma unroll
-    for (int w = 0; w < W; w++) {
-      if (w < ncol) {
-        if (r == row_a) o.rec_sum[(2 * pid) * CB + j + w] = acc[w];
-        else o.Y[(size_t)real_row(o, r) * o.k + xoff + w] = acc[w];
-      }
-    }
-  };
-  // the step's slots: lane jl holds slots c0 + q*G + jl, q < R
-  VT nv[R];
-  UIN nc[R], nhw = 0;
-  auto load_step = [&](size_t c0) {
-#pragma unroll
-    for (int q = 0; q < R; q++) {
-      const size_t my = c0 + (size_t)q * G + jl;
-      nv[q] = val[wide::il_pos_c<SPL, 16u / sizeof(VT)>(my)];
-      nc[q] = col[wide::il_pos_c<SPL, 4u>(my)];
-    }
-    nhw = __ldg(heads + (c0 >> 5));
-  };
-  if (a < b) load_step(a);
-  for (size_t c0 = a; c0 < b; c0 += T) {
-    VT mv[R];
-    UIN mc[R];
-#pragma unroll
-    for (int q = 0; q < R; q++) {
-      mv[q] = nv[q];
-      mc[q] = nc[q];
-    }
-    const UIN hw = nhw;
-    if (c0 + T < b) load_step(c0 + T);
-#pragma unroll
-    for (int i0 = 0; i0 < T; i0 += SUB) {
-      double xv[SUB][W];
-      double vv[SUB];
-#pragma unroll
-      for (int u = 0; u < SUB; u++) {
-        const int i = i0 + u;  // slot c0 + i: lane i % G, register i / G
-        vv[u] = (double)__shfl_sync(gmask, mv[i / G], grp * G + i % G);
-        const UIN c = __shfl_sync(gmask, mc[i / G], grp * G + i % G);
-        const bool live = c0 + i < nslots;
-        const FPT *xr = X + (size_t)c * o.k + xoff;
-        if (vec) {
-          const double2 qx = live ? __ldg(reinterpret_cast<const double2 *>(xr)) : make_double2(0.0, 0.0);
-          xv[u][0] = qx.x;
-          xv[u][W - 1] = qx.y;
-        } else {
-#pragma unroll
-          for (int w = 0; w < W; w++) xv[u][w] = (live && w < ncol) ? __ldg(xr + w) : 0.0;
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < SUB; u++) {
-        const size_t s = c0 + i0 + u;
-        if ((hw >> (s & 31u)) & 1u) {  // a row starts at s: the current run ends
-          if (have) {
-            if (vec && row != row_a) {
-              *reinterpret_cast<double2 *>(o.Y + (size_t)real_row(o, row) * o.k + xoff) =
-                  make_double2(acc[0], acc[W - 1]);
-            } else {
-              put(row);
-            }
-            if (row == row_a && jl == 0) o.rec_row[2 * pid] = row;
-          }
-          row++;
-#pragma unroll
-          for (int w = 0; w < W; w++) acc[w] = 0.0;
-          have = true;
-        }
-#pragma unroll
-        for (int w = 0; w < W; w++) acc[w] = fma(vv[u], xv[u][w], acc[w]);
-      }
-    }
-  }
-  // the run open at the part's end
-  if (have) {
-    const bool is_a = row == row_a;
-    if (jl == 0) o.rec_row[2 * pid + (is_a ? 0 : 1)] = row;
+}
+template <int W, bool VEC>
+__device__ __forceinline__ void st_y(double *p, int ncol, const double (&d)[W]) {
+  if constexpr (VEC && W == 4) {
+    if (ncol > 0)
+      asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(d[0]), "d"(d[1]), "d"(d[2]), "d"(d[3])
+                   : "memory");
+  } else if constexpr (VEC) {
+    if (ncol > 0) *reinterpret_cast<double2 *>(p) = make_double2(d[0], d[1]);
+  } else {
 #pragma unroll
     for (int w = 0; w < W; w++)
-      if (w < ncol) o.rec_sum[(2 * pid + (is_a ? 0 : 1)) * CB + j + w] = acc[w];
+      if (w < ncol) p[w] = d[w];
   }
 }
 
-// 32-byte global accesses (sm_100): four consecutive doubles, the address
-// 32-byte aligned.
-__device__ __forceinline__ void ld4(const double *p, double (&d)[4]) {
-  asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-               : "=d"(d[0]), "=d"(d[1]), "=d"(d[2]), "=d"(d[3])
-               : "l"(p));
-}
-__device__ __forceinline__ void st4(double *p, const double (&d)[4]) {
-  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(d[0]), "d"(d[1]), "d"(d[2]), "d"(d[3])
-               : "memory");
-}
+// One chunk of 4G slots of a group in shared memory, padded so that the
+// groups' 16-byte broadcasts fall in different banks.
+template <int G, typename VT>
+struct alignas(16) Chunk {
+  VT v[4 * G + 16 / sizeof(VT)];
+  UIN c[4 * G + 4];
+};
 
-// Four right-hand sides per lane: a group of G lanes covers CB = 4G columns
-// (8, 16 or 32) with one 32-byte X load per lane and slot, and NG = 32 / G
-// groups per warp each walk their own part of the segment as in
-// stream_spmm.  A step takes T slots of the group; its X row pieces are
-// loaded while the step before is consumed, slot by slot, into the registers
-// that slot of the step before has just freed, so every lane keeps T loads
-// in flight all the time (not T at the start of a step and none while it is
-// consumed).  Values and columns of step s+1 are in registers during step
-// s, and those of step s+2 are loaded at its start; at a step's start each
-// lane writes its slots' values and next columns to the warp's records in
-// shared memory, which the group then reads as broadcasts.  Needs k and j0
-// multiples of 4 and X and Y 32-byte aligned (kb is then a multiple of 4
-// too); lanes past the block's last column load a piece of the block and
-// store nothing.  The last step of a part is compiled apart (no loads for a
-// next step), so a slot costs no test for it.
-template <int G, int T, int MINB, typename VT, int SPL>
+template <int G, int W, int T, int MINB, bool VEC, typename VT>
 __global__ void __launch_bounds__(256, MINB)
-    stream_spmm4(size_t nslots, size_t nslots_pad, size_t seg_slots, size_t nseg, const VT *__restrict__ val,
-                 const UIN *__restrict__ col, const UIN *__restrict__ heads, const UIN *__restrict__ segh,
-                 const FPT *__restrict__ X, Out o) {
-  static_assert(T % G == 0 && T <= 32 && 32 % T == 0, "a step is whole lanes and inside one bitmap word");
-  constexpr int W = 4, NG = 32 / G, CB = G * W, R = T / G;  // R: slots per lane whose value and column it loads
+    stream_spmm(Stream st, size_t part, size_t nparts, const FPT *__restrict__ X, Out o) {
+  constexpr int NG = 32 / G, CB = G * W, C = 4 * G, NU = C / T, V = 16 / (int)sizeof(VT), LV = V == 2 ? 1 : 2;
+  static_assert(T % 4 == 0 && C % T == 0 && (C <= 32 || C == 64), "whole 16-byte pieces, chunks inside bitmap words");
+  __shared__ Chunk<G, VT> chunks[8][2][NG];
+  pdl_trigger();  // the record fix-up may launch; it waits for this grid
   const unsigned lane = threadIdx.x & 31u, grp = lane / G, jl = lane % G;
-  const size_t segid = ((size_t)blockIdx.x * 256 + threadIdx.x) >> 5;
-  if (segid >= nseg) return;
-  const size_t s0 = segid * seg_slots;
-  const size_t seg_end = min(s0 + seg_slots, nslots_pad);
-  const size_t part = (seg_end - s0) / NG;  // a multiple of 32
-  const size_t a = s0 + grp * part, b = a + part;
-  const size_t pid = segid * NG + grp;
-  UIN cr = segh[segid];
-  for (size_t w = s0 >> 5; w < (a >> 5); w++) cr += __popc(__ldg(heads + w));
-  const bool a_head = (__ldg(heads + (a >> 5)) & 1u) != 0;
-  const UIN row_a = a_head ? NO_ROW : cr - 1u;
-  UIN row = cr - 1u;
-  bool have = !a_head;
-  const unsigned j = jl * W;
-  const bool live = j < o.kb;  // all four columns, or none
-  const FPT *xb = X + o.j0 + (live ? j : o.kb - W);
-  double acc[W] = {0.0, 0.0, 0.0, 0.0};
-  if (jl == 0) {
-    o.rec_row[2 * pid] = NO_ROW;
-    o.rec_row[2 * pid + 1] = NO_ROW;
-  }
-  if (live) {
-#pragma unroll
-    for (int w = 0; w < W; w++) {
-      o.rec_sum[(2 * pid) * CB + j + w] = 0.0;
-      o.rec_sum[(2 * pid + 1) * CB + j + w] = 0.0;
-    }
-  }
-  auto load_step = [&](size_t c0, VT (&lv)[R], UIN (&lc)[R], UIN &lw) {
-#pragma unroll
-    for (int q = 0; q < R; q++) {
-      const size_t my = c0 + (size_t)q * G + jl;
-      lv[q] = val[wide::il_pos_c<SPL, 16u / sizeof(VT)>(my)];
-      lc[q] = col[wide::il_pos_c<SPL, 4u>(my)];
-    }
-    lw = __ldg(heads + (c0 >> 5));
+  const size_t pid = (((size_t)blockIdx.x * 256 + threadIdx.x) >> 5) * NG + grp;
+  Chunk<G, VT> *const mine = &chunks[threadIdx.x >> 5][0][grp];  // and mine + NG
+  const bool has = pid < nparts;
+  const size_t a = has ? pid * part : 0, b = has ? min(a + part, st.nslots_pad) : 0;
+  const int ncol = jl * W < o.kb ? min(W, (int)(o.kb - jl * W)) : 0;  // my live columns
+  // lanes past the block's last column load a piece of the block and store nothing
+  const FPT *const xb = X + o.j0 + (VEC && !ncol ? o.kb - W : jl * W);
+  const UIN kb8 = o.k * 8u;  // row stride in bytes (VEC: k < 2^29)
+  auto x_row = [&](UIN c) {
+    if constexpr (VEC) return reinterpret_cast<const FPT *>(reinterpret_cast<const char *>(xb) + (uint64_t)c * kb8);
+    else return xb + (size_t)c * o.k;
   };
-  if (a >= b) return;
-  // step s in registers: values mv, bitmap word mw, X pieces xv; step s+1:
-  // values v1, columns c1, word w1; step s+2: v2, c2, w2 (in flight)
-  VT mv[R], v1[R] = {}, v2[R] = {};
-  UIN mc[R], c1[R] = {}, c2[R] = {}, mw, w1 = 0, w2 = 0;
-  double xv[T][W];
-  load_step(a, mv, mc, mw);
-  if (a + T < b) load_step(a + T, v1, c1, w1);
-#pragma unroll
-  for (int i = 0; i < T; i++) {
-    const UIN c = __shfl_sync(FULL, mc[i / G], grp * G + i % G);
-    ld4(xb + (size_t)c * o.k, xv[i]);
+  FPT *const yb = o.Y + o.j0 + jl * W;
+  // compressed row of the run open at slot a: row starts before a, minus one
+  UIN row = 0;
+  bool a_head = false;
+  if (has) {
+    const size_t sg = a / st.seg_slots;
+    for (size_t w = (sg * st.seg_slots >> 5) + jl; w < (a >> 5); w += G) row += __popc(__ldg(st.heads + w));
+    if (jl == 0) row += __ldg(st.segh + sg);
+    a_head = (__ldg(st.heads + (a >> 5)) & 1u) != 0;
   }
-  // a run that ends is stored to its Y row, or to the part's head record
-  // when it is the row open at the part's start (a select, not a branch);
-  // lanes past the block's last column store nothing
-  double *const head = o.rec_sum + (2 * pid) * CB + j;
-  // the warp's slot records: group g's slot i at g * (T + 1) + i (one
-  // record of padding per group, so the groups' broadcasts fall in
-  // different banks)
-  constexpr int RS = T + 1;
-  __shared__ SlotRec recs[8][NG * RS];
-  SlotRec *const wrec = recs[threadIdx.x >> 5];
-  const SlotRec *const grec = wrec + grp * RS;
-  auto step = [&](size_t c0, auto more_c) {
-    constexpr bool MORE = decltype(more_c)::value;  // step s+1 exists: load its X pieces
 #pragma unroll
-    for (int q = 0; q < R; q++) wrec[grp * RS + q * G + jl] = SlotRec{(double)mv[q], c1[q], 0u};
-    __syncwarp();
-    if (c0 + 2 * T < b) load_step(c0 + 2 * T, v2, c2, w2);
-    if (c0 + T > nslots) {  // the stream's zero padding adds nothing, whatever X holds
+  for (int d = 1; d < G; d <<= 1) row += __shfl_xor_sync(FULL, row, d);
+  row -= 1u;
+  const UIN row_a = a_head ? NO_ROW : row;
+
+  const VT *const val = static_cast<const VT *>(st.val);
+  // the group's chunk at c0: each lane copies 4/V value vectors and one
+  // column vector, neighbouring lanes neighbouring addresses
+  auto issue = [&](size_t c0, Chunk<G, VT> *dst) {
+    const unsigned lgl = st.lspl && (C >> st.lspl) > 1 ? 31 - __clz(C >> st.lspl) : 0;  // log2 lanes the chunk spans
 #pragma unroll
-      for (int i = 0; i < T; i++)
-        if (c0 + i >= nslots) {
-#pragma unroll
-          for (int w = 0; w < W; w++) xv[i][w] = 0.0;
-        }
+    for (int r = 0; r < 4 / V; r++) {
+      const unsigned rank = r * G + jl;
+      const unsigned m = ((rank & ((1u << lgl) - 1u)) << (st.lspl ? st.lspl - LV : 0)) + (rank >> lgl);
+      cp_async16(dst->v + V * m, val + il_vec(c0 + V * m, st.lspl, LV));
     }
-    const unsigned hs = mw >> (unsigned)(c0 & 31u);
+    const unsigned m = ((jl & ((1u << lgl) - 1u)) << (st.lspl ? st.lspl - 2 : 0)) + (jl >> lgl);
+    cp_async16(dst->c + 4 * m, st.col + il_vec(c0 + 4 * m, st.lspl, 2));
+  };
+  // row-start bits of the chunk at c0
+  using Bits = std::conditional_t<C == 64, unsigned long long, unsigned>;
+  auto bits_of = [&](size_t c0) {
+    Bits h = __ldg(st.heads + (c0 >> 5));
+    if constexpr (C == 64) h |= (Bits)__ldg(st.heads + (c0 >> 5) + 1) << 32;
+    else h >>= (unsigned)(c0 & 31u);
+    return h;
+  };
+
+  double xv[T][W], acc[W];
 #pragma unroll
-    for (int i = 0; i < T; i++) {
-      const SlotRec sr = grec[i];
-      const double v = sr.v;
-      if (hs & (1u << i)) {  // a row starts at slot c0 + i: the current run ends
-        const bool is_a = row == row_a;
-        double *dst = is_a ? head : o.Y + (size_t)real_row(o, row) * o.k + o.j0 + j;
-        if (have && live) st4(dst, acc);
-        if (have && is_a && jl == 0) o.rec_row[2 * pid] = row;
-        row++;
+  for (int w = 0; w < W; w++) acc[w] = 0.0;
+  double *const head = o.head + pid * CB + jl * W;
+  double *ydst = head;  // where the open run goes if it ends here: the part's head first
+  Bits hs = 0, hnext = 0;
+  if (a < b) {
+    issue(a, mine);
+    hnext = bits_of(a);
+  }
+  cp_async_wait();
+  __syncwarp();
+  if (a < b) {
 #pragma unroll
-        for (int w = 0; w < W; w++) acc[w] = 0.0;
-        have = true;
+    for (int i = 0; i < T; i++) ld_x<W, VEC>(x_row(mine->c[i]), ncol, xv[i]);
+  }
+  bool first = true;
+  const int nch = (int)(part / C);
+  for (int q = 0; q < nch; q++) {
+    const size_t c0 = a + (size_t)q * C;
+    const bool on = c0 < b, next = c0 + C < b;
+    const Chunk<G, VT> *cur = mine + (q & 1) * NG, *other = mine + (~q & 1) * NG;
+    hs = hnext;
+    if (next) {
+      issue(c0 + C, const_cast<Chunk<G, VT> *>(other));
+      hnext = bits_of(c0 + C);
+    }
+#pragma unroll 1
+    for (int u = 0; u < NU; u++) {
+      const UIN *cn = cur->c + (u + 1) * T;
+      bool more = on;
+      if (u == NU - 1) {  // the next step is the next chunk's first: it must have landed
+        cp_async_wait();
+        __syncwarp();
+        cn = other->c;
+        more = next;
       }
+      if (on) {
+        const size_t s = c0 + u * T;
+        if (s + T > st.nslots) {  // the stream's zero padding adds nothing, whatever X holds
 #pragma unroll
-      for (int w = 0; w < W; w++) acc[w] = fma(v, xv[i][w], acc[w]);
-      if constexpr (MORE) ld4(xb + (size_t)sr.c * o.k, xv[i]);  // slot i of step s+1, into the registers just freed
-    }
-    __syncwarp();  // every lane has read the records before the next step writes them
+          for (int i = 0; i < T; i++)
+            if (s + i >= st.nslots) {
 #pragma unroll
-    for (int q = 0; q < R; q++) {
-      mv[q] = v1[q];
-      c1[q] = c2[q];
-      v1[q] = v2[q];
+              for (int w = 0; w < W; w++) xv[i][w] = 0.0;
+            }
+        }
+#pragma unroll
+        for (int i0 = 0; i0 < T; i0 += 4) {
+          VT v[4];
+          UIN c[4];
+          if constexpr (V == 2) {
+            const double2 t0 = *reinterpret_cast<const double2 *>(cur->v + u * T + i0);
+            const double2 t1 = *reinterpret_cast<const double2 *>(cur->v + u * T + i0 + 2);
+            v[0] = t0.x, v[1] = t0.y, v[2] = t1.x, v[3] = t1.y;
+          } else {
+            const float4 t = *reinterpret_cast<const float4 *>(cur->v + u * T + i0);
+            v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+          }
+          {
+            const uint4 t = *reinterpret_cast<const uint4 *>(cn + i0);  // stale past the part's end: not used
+            c[0] = t.x, c[1] = t.y, c[2] = t.z, c[3] = t.w;
+          }
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            if (hs & 1u) {  // a row starts here: the open run ends (the part's first one, maybe empty, as a record)
+              st_y<W, VEC>(ydst, ncol, acc);
+              row++;
+              first = false;
+              ydst = o.rowmap ? yb + (size_t)o.rowmap[row] * o.k : yb + (size_t)row * o.k;
+#pragma unroll
+              for (int w = 0; w < W; w++) acc[w] = 0.0;
+            }
+            hs >>= 1;
+#pragma unroll
+            for (int w = 0; w < W; w++) acc[w] = fma((double)v[i], xv[i0 + i][w], acc[w]);
+            if (more && (i % 4) == 3) {
+#pragma unroll
+              for (int e = 0; e < 4; e++) ld_x<W, VEC>(x_row(c[i - 3 + e]), ncol, xv[i0 + i - 3 + e]);
+            }
+          }
+        }
+      }
     }
-    mw = w1;
-    w1 = w2;
+    __syncwarp();  // the chunk is read: its buffer may be filled again
+  }
+  // Join the rows that cross parts of this CTA.  flag of a part: it starts
+  // with a row (1), no row starts in it (2).
+  constexpr int CG = 8 * NG;  // parts of a CTA
+  __shared__ unsigned char flag[CG];
+  const unsigned gi = (threadIdx.x >> 5) * NG + grp;
+  if (has && first) st_y<W, VEC>(head, ncol, acc);
+  if (jl == 0) flag[gi] = (a_head ? 1 : 0) | (first ? 2 : 0);
+  __syncthreads();  // the CTA's heads and flags are written
+  const unsigned live = (unsigned)min((size_t)CG, nparts - (size_t)blockIdx.x * CG);
+  // adds to acc what the following parts hold of the row open at part i's
+  // end; true if the row ends in this CTA
+  auto follow = [&](unsigned i) {
+    for (unsigned j = i + 1; j < live; j++) {
+      const unsigned char f = flag[j];
+      if (f & 1u) return true;
+      const double *h = o.head + ((size_t)blockIdx.x * CG + j) * CB + jl * W;
+#pragma unroll
+      for (int w = 0; w < W; w++)
+        if (VEC ? ncol > 0 : w < ncol) acc[w] += h[w];
+      if (!(f & 2u)) return true;
+    }
+    return false;
   };
-  size_t c0 = a;
-  for (; c0 + T < b; c0 += T) step(c0, BoolC<true>{});
-  step(c0, BoolC<false>{});
-  if (have) {  // the run open at the part's end
-    const bool is_a = row == row_a;
-    if (jl == 0) o.rec_row[2 * pid + (is_a ? 0 : 1)] = row;
-    if (live) {
+  if (!has) return;
+  const size_t r2 = 2 * (size_t)blockIdx.x;
+  bool tail = false;  // the CTA's last run is mine, and goes to its tail record
+  if (!first) {
+    if (follow(gi)) {
+      st_y<W, VEC>(ydst, ncol, acc);
+    } else {
+      tail = true;
+      st_y<W, VEC>(o.rec_sum + (r2 + 1) * CB + jl * W, ncol, acc);
+    }
+  }
+  if (tail && jl == 0) o.rec_row[r2 + 1] = row;
+  if (gi == 0) {
+    // the CTA's head record: the run open at its start; no tail if that run never ends
+    bool whole = false;
+    if (!a_head) {
 #pragma unroll
-      for (int w = 0; w < W; w++) o.rec_sum[(2 * pid + (is_a ? 0 : 1)) * CB + j + w] = acc[w];
+      for (int w = 0; w < W; w++) acc[w] = (VEC ? ncol > 0 : w < ncol) ? head[w] : 0.0;
+      if (first) whole = !follow(0);
+      st_y<W, VEC>(o.rec_sum + r2 * CB + jl * W, ncol, acc);
+    }
+    if (jl == 0) {
+      o.rec_row[r2] = row_a;
+      if (whole) o.rec_row[r2 + 1] = NO_ROW;
     }
   }
 }
 
-// Record i (of 2 per part) writes its row if it is that row's last record,
-// adding the row's earlier records; rows with no slot get zeros.
-template <int G>  // G = columns of one pass
-__global__ void spmm_fixup(size_t nrec, const UIN *__restrict__ rec_row, const double *__restrict__ rec_sum,
-                           const UIN *__restrict__ empty, size_t nempty, Out o) {
+// Record i (of 2 per CTA) writes its row if it is that row's last record,
+// adding the row's earlier records; rows with no slot get zeros.  A
+// programmatic dependent of the main kernel.
+template <int CB>  // columns of one pass
+__global__ void spmm_fixup(size_t nrec, const UIN *__restrict__ empty, size_t nempty, Out o) {
+  pdl_wait();
+  const UIN *rec_row = after_wait((const UIN *)o.rec_row);
+  const double *rec_sum = after_wait((const double *)o.rec_sum);
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t i = t / G;
-  const unsigned j = t % G;
+  const size_t i = t / CB;
+  const unsigned j = t % CB;
   if (j >= o.kb) return;
   if (i < nempty) o.Y[(size_t)empty[i] * o.k + o.j0 + j] = 0.0;
   if (i >= nrec) return;
@@ -351,12 +323,12 @@ __global__ void spmm_fixup(size_t nrec, const UIN *__restrict__ rec_row, const d
   size_t q = i + 1;
   while (q < nrec && rec_row[q] == NO_ROW) q++;
   if (q < nrec && rec_row[q] == r) return;
-  double total = rec_sum[i * G + j];
+  double total = rec_sum[i * CB + j];
   for (size_t m = i; m-- > 0;) {
     const UIN rm = rec_row[m];
     if (rm == NO_ROW) continue;
     if (rm != r) break;
-    total += rec_sum[m * G + j];
+    total += rec_sum[m * CB + j];
   }
   o.Y[(size_t)real_row(o, r) * o.k + o.j0 + j] = total;
 }

@@ -160,3 +160,25 @@ def test_axt_kernels_steps(env, nnz, offset):
         want = F.getFormatDataAXT(0, 128, 8, th, mode, csr, x)[1]
         for k in ("con", "ax", "sec"):
             assert np.array_equal(got[k], getattr(want, k)), (mode, th, k)
+
+
+@pytest.mark.parametrize("k", [8, 16, 32, 11])
+@pytest.mark.parametrize("n,rl", [(40, 3), (64, 8), (3000, 1), (700, 37), (130, 129), (2, 1)])
+def test_spmm_parts(env, k, n, rl):
+    """SpMM parts of 64 slots and up: rows that start at part and CTA edges,
+    rows of a slot, rows over many parts, of whole CTAs, and the last part."""
+    torch, D, F, orc = env
+    rng = np.random.default_rng(n + rl)
+    lengths = np.full(n, rl)
+    lengths[n // 2:] = rng.integers(0, min(n, 2 * rl) + 1, n - n // 2)
+    if n == 3000:
+        lengths[77] = 2999  # one row over several CTAs
+    row, col, val = rows_of(lengths, n, n)
+    X = rng.uniform(-1, 1, (n, k))
+    for f, kw in ((None, {}), (None, dict(kernel="ldg")), (None, dict(kernel="wide", variant=0))):
+        plan = D.Plan(F.CSR(row, col, val), f, **kw)
+        Y = torch.full((n, k), 9.0, dtype=torch.float64, device="cuda")
+        plan.spmm(torch.from_numpy(X).cuda(), Y)
+        for j in range(k):
+            xj = np.ascontiguousarray(X[:, j])
+            assert_parity(Y[:, j].cpu().numpy(), orc.cf_csr(row, col, val, xj), orc.abs_csr(row, col, val, xj), TOL_F64)
