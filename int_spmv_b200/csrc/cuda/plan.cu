@@ -212,12 +212,19 @@ int empty_rows(ispmv_plan_s *p, const str_matCSR *csr) {
   return ISPMV_OK;
 }
 
-int alloc_records(ispmv_plan_s *p) {
-  TRY(dev_alloc(p, std::max<size_t>(1, 2 * p->nseg), &p->rec_row));
-  TRY(dev_alloc(p, std::max<size_t>(1, 2 * p->nseg), &p->rec_sum));
+// The work areas of a stream or unit plan, set on `s`; a builder on the
+// default stream waits here (products run on any stream).
+int alloc_records(ispmv_plan_s *p, cudaStream_t s = nullptr) {
+  const size_t nrec = std::max<size_t>(1, 2 * p->nseg);
+  TRY(dev_alloc(p, nrec, &p->rec_row));
+  TRY(dev_alloc(p, nrec, &p->rec_sum));
   TRY(dev_alloc(p, 1, &p->status));
-  ISPMV_TRY(cudaMemset(p->status, 0, sizeof(int)));
+  // no row: a staged kernel that gives up a wait leaves records unwritten,
+  // which the fix-up reads all the same
+  ISPMV_TRY(cudaMemsetAsync(p->rec_row, 0xFF, nrec * sizeof(UIN), s));
+  ISPMV_TRY(cudaMemsetAsync(p->status, 0, sizeof(int), s));
   TRY(dev_alloc(p, 1, &p->queue));
+  if (!s) ISPMV_TRY(cudaStreamSynchronize(s));
   return ISPMV_OK;
 }
 
@@ -1023,7 +1030,7 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
     p->xw.nwin = 1;
     p->xw.n = p->n;
   }
-  TRY(alloc_records(p));
+  TRY(alloc_records(p, s));
   if (wc.stg) p->xw.status = p->status;
   ISPMV_TRY(cudaMemcpyAsync(&hf.bad, bad, sizeof hf.bad, cudaMemcpyDeviceToHost, s));
   ISPMV_TRY(cudaStreamSynchronize(s));
