@@ -17,6 +17,9 @@
 //   rows    CSR row pointer (pk::csr_vec) and AXC brick pointer
 //           (pk::axc_rows): the row-parallel kernels.
 //   K1      val/col column-major per chunk, chp, nmc, permi (pk::k1_chunks).
+//   slices  16-bit-delta plans of equally long neighbouring rows: 32 rows side
+//           by side, values and deltas per element, row lengths
+//           (sl::slice_rows).
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -27,6 +30,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include "plan_tma.cuh"
+#include "slices.cuh"
 #include "spmm.cuh"
 #include "sss.cuh"
 #include "tmem.cuh"
@@ -35,7 +39,7 @@
 using namespace ispmv;
 
 enum PlanFormat { F_CSR = 0, F_AXC = 1, F_K1 = 2, F_K1P = 3, F_AXT_NOC = 4, F_AXT_COM = 5 };
-enum PlanPath { P_STREAM = 0, P_UNITS = 1, P_ROWS = 2, P_K1 = 3 };
+enum PlanPath { P_STREAM = 0, P_UNITS = 1, P_ROWS = 2, P_K1 = 3, P_SLICES = 4 };
 
 struct ispmv_plan_s {
   int fmt = 0;
@@ -44,6 +48,10 @@ struct ispmv_plan_s {
   UIN n = 0, nnz = 0, th = 1, bs = 0, lanes = 8;
   size_t slots = 0, slots_pad = 0, nunits = 0;
   bool no_win = false;  // staged variants: empty x windows
+  bool chosen = false;  // kernel and variant by AUTO
+  uint2 *slices = nullptr;  // P_SLICES: first element column and base column of each slice, and the end
+  uint8_t *slen = nullptr;  // P_SLICES: row lengths
+  UIN slice_w = 0;          // P_SLICES: the widest slice
   size_t fslots = 0;  // the format's slots, padding included (stream path: slots holds none)
   size_t seg_slots = 0, nseg = 0;
   UIN useg = 0;
@@ -151,7 +159,7 @@ void finish_info(ispmv_plan_s *p, const char *name) {
   ispmv_plan_info &i = p->info;
   i.nrows = p->n;
   i.nnz = p->nnz;
-  i.slots = p->path == P_STREAM ? p->fslots : p->slots;
+  i.slots = p->path == P_STREAM || p->path == P_SLICES ? p->fslots : p->slots;
   i.format = p->fmt;
   i.val_kind = p->opts.val_kind;
   i.col_kind = p->opts.col_kind;
@@ -165,6 +173,7 @@ void finish_info(ispmv_plan_s *p, const char *name) {
     const double B = (double)p->d16_batch, batches = (double)(p->slots_pad / p->d16_batch);
     bi = 2.0 + (4.0 * batches + B * 4.0 * (double)p->esc_batches) / std::max(1.0, (double)p->nnz);
   }
+  if (p->path == P_SLICES) bi = 2.0 + (8.0 * ((p->n + 31) / 32) + (double)p->n) / std::max(1.0, (double)p->nnz);
   i.alg_bytes = (double)p->nnz * (bv + bi) + (double)p->n * 16.0 + 4.0 * ((double)p->n + 1.0);
   snprintf(i.name, sizeof i.name, "%s", name);
 }
@@ -349,6 +358,7 @@ void auto_wide(ispmv_plan_s *p, const str_matCSR *csr) {
   if (p->opts.variant != 0) return;
   p->opts.variant = auto_variant(p, (double)csr->nnz >= 16.0 * (double)p->n, random_far_fraction(csr) >= 0.05);
   p->no_win = csr->nnz < WIN_MIN_NNZ;
+  p->chosen = true;
 }
 
 // The per-CTA x windows of the staged stream_wide variants: CTA t walks
@@ -453,6 +463,62 @@ void pack_rows(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v, s
   p->slots = csr->nnz;
 }
 
+// Slices of 32 rows (sl::slice_rows) for AUTO's 16-bit-delta plans, where the
+// rows of a slice are nearly equally long (at most 8% padding: the bytes it
+// adds are then less than the kernel saves) and short (a row is one lane's
+// work: at most 48 elements), and every slice's columns span less than 65536.
+// v, c: the rows back to back.  Returns false where a slice does not fit.
+bool slice_fit(const ispmv_plan_s *p, const str_matCSR *csr, const std::vector<UIN> &c, std::vector<uint2> &meta) {
+  const UIN ns = (p->n + 31) / 32;
+  meta.assign((size_t)ns + 1, uint2{0, 0});
+  uint64_t cols = 0;
+  for (UIN s = 0; s < ns; s++) {
+    const UIN r0 = s * 32, r1 = std::min<UIN>(p->n, r0 + 32);
+    UIN w = 0;
+    for (UIN r = r0; r < r1; r++) w = std::max(w, csr->row[r + 1] - csr->row[r]);
+    if (w > 48) return false;
+    UIN lo = 0xFFFFFFFFu, hi = 0;
+    for (UIN q = csr->row[r0]; q < csr->row[r1]; q++) {
+      lo = std::min(lo, c[q]);
+      hi = std::max(hi, c[q]);
+    }
+    if (w && hi - lo > 0xFFFFu) return false;
+    meta[s] = {(UIN)cols, w ? lo : 0};
+    cols += w;
+  }
+  meta[ns] = {(UIN)cols, 0};
+  return cols * 32 <= csr->nnz + csr->nnz / 12 + 1024 && cols * 32 <= 0xFFFFFFFFull;
+}
+
+int setup_slices(ispmv_plan_s *p, const str_matCSR *csr, const std::vector<double> &v, const std::vector<UIN> &c,
+                 const std::vector<uint2> &meta) {
+  p->path = P_SLICES;
+  p->slots_pad = (size_t)meta.back().x * 32;
+  std::vector<double> sv(p->slots_pad, 0.0);
+  std::vector<uint16_t> sd(p->slots_pad, 0);
+  std::vector<uint8_t> len(p->n);
+#pragma omp parallel for schedule(static)
+  for (long long r = 0; r < (long long)p->n; r++) {
+    const uint2 m = meta[r / 32];
+    const UIN a = csr->row[r], l = csr->row[r + 1] - a;
+    len[r] = (uint8_t)l;
+    for (UIN k = 0; k < l; k++) {
+      const size_t q = ((size_t)m.x + k) * 32 + r % 32;
+      sv[q] = v[a + k];
+      sd[q] = (uint16_t)(c[a + k] - m.y);
+    }
+  }
+  uint16_t *d;
+  TRY(upload_values(p, sv));
+  TRY(dev_upload(p, sd.data(), sd.size(), &d));
+  TRY(dev_upload(p, meta.data(), meta.size(), &p->slices));
+  TRY(dev_upload(p, len.data(), len.size(), &p->slen));
+  p->narrow.col16 = d;
+  p->info.device_bytes = (uint64_t)p->slots_pad * (vbytes(p) + 2) + meta.size() * 8 + p->n;
+  for (size_t s = 0; s + 1 < meta.size(); s++) p->slice_w = std::max(p->slice_w, meta[s + 1].x - meta[s].x);
+  return ISPMV_OK;
+}
+
 // The stream path: `v`/`c` the slot streams (length p->slots), `start[r]`
 // the first slot of row r (rows with no slot are skipped).
 int setup_stream(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v, std::vector<UIN> &c,
@@ -460,6 +526,11 @@ int setup_stream(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v,
   p->path = P_STREAM;
   p->fslots = p->slots;
   if (p->slots != csr->nnz) pack_rows(p, csr, v, c, start);
+  if (p->chosen && p->opts.col_kind == ISPMV_COL_D16 && p->opts.val_kind != ISPMV_VAL_F32_LO16 &&
+      p->opts.units_per_warp <= 0 && p->slots) {
+    std::vector<uint2> meta;
+    if (slice_fit(p, csr, c, meta)) return setup_slices(p, csr, v, c, meta);
+  }
   p->slots_pad = std::max(SS, (p->slots + SS - 1) / SS * SS);
   if (p->opts.kernel == ISPMV_KERNEL_WIDE && wide_variant(p->opts.variant).tmem) {
     // whole CTAs: every consumer warp of stream_tmem walks a full segment
@@ -1657,6 +1728,13 @@ int run_main(ispmv_plan_s *p, const FPT *x, FPT *y, int beta, cudaStream_t s) {
       }
       return check_launch("csr_vec");
     }
+    case P_SLICES: {
+      const UIN ns = (p->n + 31) / 32;
+      auto *k = p->slice_w <= 5 ? sl::slice_rows<VT, 5> : sl::slice_rows<VT, 9>;
+      k<<<(ns + pk::TPB / 32 - 1) / (pk::TPB / 32), pk::TPB, 0, s>>>(p->n, ns, p->slices, p->slen, p->narrow.col16,
+                                                                     val, x, y, beta);
+      return check_launch("stream_wide<rows32,d16>");
+    }
     case P_K1: {
       const unsigned g = (unsigned)pk::k1_ctas(p->chunkNum, p->k1_cta, p->k1_long);
       if (p->fmt == F_K1P) {
@@ -1699,7 +1777,7 @@ ISPMV_API int ispmv_plan_spmv_graph(ispmv_plan p, const FPT *x, FPT *y, int beta
     // work areas a product allocates on first use, allocated before the
     // capture (no allocation may happen inside it): the FP32 copy of x of
     // FP32-value plans on the lane-interleaved kernel
-    if (p->opts.val_kind != ISPMV_VAL_F64 && p->opts.kernel == ISPMV_KERNEL_WIDE && !p->x32)
+    if (p->opts.val_kind != ISPMV_VAL_F64 && p->opts.kernel == ISPMV_KERNEL_WIDE && p->path == P_STREAM && !p->x32)
       TRY(dev_alloc(p, p->n, &p->x32));
     ISPMV_TRY(cudaStreamBeginCapture(p->cap_stream, cudaStreamCaptureModeThreadLocal));
     p->capturing = true;

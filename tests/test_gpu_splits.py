@@ -182,3 +182,38 @@ def test_spmm_parts(env, k, n, rl):
         for j in range(k):
             xj = np.ascontiguousarray(X[:, j])
             assert_parity(Y[:, j].cpu().numpy(), orc.cf_csr(row, col, val, xj), orc.abs_csr(row, col, val, xj), TOL_F64)
+
+
+@pytest.mark.parametrize("val_kind", ["f64", "f32"])
+@pytest.mark.parametrize("n,w,span", [(1, 1, 0), (31, 3, 40), (32, 48, 60), (33, 9, 100), (4000, 10, 65_000), (70_000, 19, 65_535),
+                                      (70_000, 19, 65_536), (5000, 49, 300)])
+def test_slices_of_rows(env, val_kind, n, w, span):
+    """16-bit-delta plans of 32 equally long rows side by side: unfilled last
+    slices, remainders of the unrolled loop, shorter and empty rows, the widest
+    rows (48) and columns (65535) they take and the first they do not, no read
+    of x for padding."""
+    torch, D, F, orc = env
+    rng = np.random.default_rng(n + w)
+    lengths = np.full(n, min(w, n))
+    if n > 100:
+        lengths[rng.integers(0, n, n // 300)] = 0
+        lengths[rng.integers(0, n, n // 200)] = w - 1
+    row = np.zeros(n + 1, np.uint32)
+    row[1:] = np.cumsum(lengths)
+    k = np.arange(int(row[-1])) - np.repeat(row[:-1], lengths)
+    r = np.repeat(np.arange(n), lengths) // 32 * 32
+    lo = np.minimum(r, max(0, n - 1 - span))
+    col = np.minimum(lo + np.where(k == w - 1, span, k), n - 1).astype(np.uint32)
+    val = rng.standard_normal(len(col))
+    csr = F.CSR(row, col, val)
+    for f in (None, F.getFormatDataAXT(0, 128, 8, 4, "NOC", csr, np.zeros(n))[1]):
+        plan = D.Plan(csr, f, val=val_kind, col="d16")
+        assert plan.info["col_kind"] == 1
+        check(env, row, col, val, plan, val_kind)
+        assert ("rows32" in plan.kernel_name()) == (w <= 48 and span <= 65_535)
+        x = torch.rand(n, dtype=torch.float64, device="cuda")
+        y = torch.empty_like(x)
+        a = plan.spmv(x, y).clone()
+        assert torch.equal(plan.spmv_graph(x, y), a)
+    with pytest.raises(Exception):
+        plan.spmm(torch.zeros((n, 8), dtype=torch.float64, device="cuda"))
