@@ -43,10 +43,12 @@ int sm_count();
   } while (0)
 
 // ---- device side --------------------------------------------------------
-// Programmatic dependent launch: a main kernel lets the launch that follows
-// it in the stream (the row fix-up, K1's reorder) start now; that kernel
-// waits (pdl_wait) for the whole main grid and its writes before it reads
-// anything.  Both are no-ops for ordinary launches.
+// Programmatic dependent launch: a kernel lets the launch that follows it in
+// the stream start now (the row fix-up after a main kernel, the next
+// product's main kernel after that); that kernel waits (pdl_wait) for the
+// whole earlier grid and its writes before it reads or writes anything but the
+// plan's own constant arrays - x, y, records and work areas come after the
+// wait.  Both are no-ops for ordinary launches.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A pointer (or texture handle) to what the awaited grid wrote, for use after

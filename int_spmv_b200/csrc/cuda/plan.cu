@@ -1405,6 +1405,26 @@ int launch_staged_w(K kernel, size_t smem, size_t nseg, int ctas_per_sm, cudaStr
   return check_launch(what);
 }
 
+// A launch that may start while the launches before it in the stream finish
+// (its kernel waits for them before it touches anything but the plan's
+// constant arrays), unless a timing event sits between.
+template <typename... KA, typename... A>
+int launch_dependent(const ispmv_plan_s *p, const char *name, void (*k)(KA...), size_t grid, unsigned block,
+                     size_t smem, cudaStream_t s, A... a) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = !p->tcap || p->capturing ? 1 : 0;
+  ISPMV_TRY(cudaLaunchKernelEx(&cfg, k, static_cast<KA>(a)...));
+  return check_launch(name);
+}
+
 // A linear texture over `src` (bytes long, FP64 read as int2 or FP32),
 // cached on the plan for the same buffer; 0 when the buffer does not meet
 // the texture alignment or size limits (the caller then gathers with loads).
@@ -1448,38 +1468,23 @@ int launch_wide(ispmv_plan_s *p, const FPT *x, seg::Out &o, cudaStream_t s, cons
     // FP32 values: gather from an FP32 copy of x (the value the FP32 multiply uses)
     if (!p->x32) TRY(dev_alloc(p, p->n, &p->x32));
     const unsigned gc = (unsigned)std::min<size_t>(((size_t)p->n / 2 + 255) / 256, (size_t)sm_count() * 8) + 1;
-    if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) wide::x_to_f32<true><<<gc, 256, 0, s>>>(p->n, x, p->x32);
-    else wide::x_to_f32<false><<<gc, 256, 0, s>>>(p->n, x, p->x32);
-    TRY(check_launch("x_to_f32"));
+    auto *kx = (reinterpret_cast<uintptr_t>(x) & 15u) == 0 ? wide::x_to_f32<true> : wide::x_to_f32<false>;
+    TRY(launch_dependent(p, "x_to_f32", kx, gc, 256, 0, s, p->n, x, p->x32));
     const cudaTextureObject_t tx = TEX ? x_texture(p, p->x32, (size_t)p->n * 4, true) : 0;
     if (TEX && !tx) return launch_wide<VT, SPL, MINB, D16, false>(p, x, o, s, "stream_wide<tex: x gathered with loads>");
-    // a programmatic dependent of x_to_f32: its CTAs load their first
-    // batch while x is rounded, and wait for x_to_f32 before they gather
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((p->nseg + WIDE_WARPS - 1) / WIDE_WARPS));
-    cfg.blockDim = dim3(WIDE_WARPS * 32);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    ISPMV_TRY(cudaLaunchKernelEx(&cfg, wide::stream_wide<VT, float, SPL, 0, WIDE_WARPS, MINB, D16, TEX, false, false, PFC>,
-                                 p->slots, p->slots_pad, p->seg_slots, p->nseg, static_cast<const VT *>(p->val),
-                                 (const UIN *)p->col, (const UIN *)p->heads, (const UIN *)p->segh, p->xw,
-                                 (const float *)p->x32, o, p->narrow, tx));
-    return check_launch(name);
+    return launch_dependent(p, name, wide::stream_wide<VT, float, SPL, 0, WIDE_WARPS, MINB, D16, TEX, false, false, PFC>,
+                            (p->nseg + WIDE_WARPS - 1) / WIDE_WARPS, WIDE_WARPS * 32, 0, s, p->slots, p->slots_pad,
+                            p->seg_slots, p->nseg, static_cast<const VT *>(p->val), p->col, p->heads, p->segh, p->xw,
+                            p->x32, o, p->narrow, tx);
   } else {
     const cudaTextureObject_t tx = TEX ? x_texture(p, x, (size_t)p->n * 8, false) : 0;
     if (TEX && !tx) return launch_wide<VT, SPL, MINB, D16, false>(p, x, o, s, "stream_wide<tex: x gathered with loads>");
     auto *k = wide::stream_wide<VT, double, SPL, NW, WIDE_WARPS, MINB, D16, TEX, STG, LO, PFC>;
     const size_t smem = STG ? (size_t)p->xw.cap * sizeof(double) : 0;
     if (smem) ISPMV_TRY(cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned g = (unsigned)((p->nseg + WIDE_WARPS - 1) / WIDE_WARPS);
-    k<<<g, WIDE_WARPS * 32, smem, s>>>(p->slots, p->slots_pad, p->seg_slots, p->nseg, static_cast<const VT *>(p->val),
-                                        p->col, p->heads, p->segh, p->xw, x, o, p->narrow, tx);
-    return check_launch(name);
+    return launch_dependent(p, name, k, (p->nseg + WIDE_WARPS - 1) / WIDE_WARPS, WIDE_WARPS * 32, smem, s, p->slots,
+                            p->slots_pad, p->seg_slots, p->nseg, static_cast<const VT *>(p->val), p->col, p->heads,
+                            p->segh, p->xw, x, o, p->narrow, tx);
   }
 }
 
@@ -1495,6 +1500,8 @@ int launch_wide_tma(ispmv_plan_s *p, const FPT *x, seg::Out &o, cudaStream_t s, 
   if (p->opts.ctas_per_sm > 0) per_sm = std::min(per_sm, p->opts.ctas_per_sm);
   const size_t want = (p->nseg + W - 1) / W;
   const unsigned g = (unsigned)std::max<size_t>(1, std::min(want, (size_t)sm_count() * (size_t)std::max(1, per_sm)));
+  // an ordinary launch: starting before the launch before it ends gave
+  // nothing here (32 FEM blocks 54.8 / 54.6 us) and 1% away at 160^3
   k<<<g, W * 32, smem, s>>>(p->slots, p->slots_pad, p->seg_slots, p->nseg, static_cast<const VT *>(p->val), p->col,
                             p->heads, p->segh, x, o, p->status);
   return check_launch(name);
@@ -1731,20 +1738,16 @@ int run_main(ispmv_plan_s *p, const FPT *x, FPT *y, int beta, cudaStream_t s) {
     case P_SLICES: {
       const UIN ns = (p->n + 31) / 32;
       auto *k = p->slice_w <= 5 ? sl::slice_rows<VT, 5> : sl::slice_rows<VT, 9>;
-      k<<<(ns + pk::TPB / 32 - 1) / (pk::TPB / 32), pk::TPB, 0, s>>>(p->n, ns, p->slices, p->slen, p->narrow.col16,
-                                                                     val, x, y, beta);
-      return check_launch("stream_wide<rows32,d16>");
+      return launch_dependent(p, "stream_wide<rows32,d16>", k, (ns + pk::TPB / 32 - 1) / (pk::TPB / 32), pk::TPB, 0, s,
+                              p->n, ns, p->slices, p->slen, p->narrow.col16, val, x, y, beta);
     }
     case P_K1: {
       const unsigned g = (unsigned)pk::k1_ctas(p->chunkNum, p->k1_cta, p->k1_long);
-      if (p->fmt == F_K1P) {
-        pk::k1_chunks<VT, true><<<g, pk::TPB, 0, s>>>(p->n, p->chunkNum, p->k1_cta, p->k1_long, p->chp, p->nmc, p->permi,
-                                                      p->col, val, x, y, beta);
-        return check_launch("k1_chunks<scatter>");
-      }
-      pk::k1_chunks<VT, false><<<g, pk::TPB, 0, s>>>(p->n, p->chunkNum, p->k1_cta, p->k1_long, p->chp, p->nmc, p->permi,
-                                                     p->col, val, x, p->res, beta);
-      return check_launch("k1_chunks");
+      if (p->fmt == F_K1P)
+        return launch_dependent(p, "k1_chunks<scatter>", pk::k1_chunks<VT, true>, g, pk::TPB, 0, s, p->n, p->chunkNum,
+                                p->k1_cta, p->k1_long, p->chp, p->nmc, p->permi, p->col, val, x, y, beta);
+      return launch_dependent(p, "k1_chunks", pk::k1_chunks<VT, false>, g, pk::TPB, 0, s, p->n, p->chunkNum, p->k1_cta,
+                              p->k1_long, p->chp, p->nmc, p->permi, p->col, val, x, p->res, beta);
     }
     case P_STREAM:
     case P_UNITS: {
@@ -1921,17 +1924,8 @@ int spmm_blocks(ispmv_plan_s *p, UIN k, const FPT *X, FPT *Y, cudaStream_t s, co
     mm::stream_spmm<G, W, T, MINB, VEC, VT><<<(unsigned)ctas, 256, 0, s>>>(st, part, nparts, X, o);
     TRY(check_launch(name));
     p->kname = last_launch();
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((std::max(nrec, p->nempty) * CB + 255) / 256));
-    cfg.blockDim = dim3(256);
-    cfg.stream = s;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    ISPMV_TRY(cudaLaunchKernelEx(&cfg, mm::spmm_fixup<CB>, nrec, (const UIN *)p->empty, p->nempty, o));
-    TRY(check_launch("spmm_fixup"));
+    TRY(launch_dependent(p, "spmm_fixup", mm::spmm_fixup<CB>, (std::max(nrec, p->nempty) * CB + 255) / 256, 256, 0, s,
+                         nrec, p->empty, p->nempty, o));
   }
   return ISPMV_OK;
 }

@@ -101,7 +101,7 @@ __device__ __forceinline__ float2 ld_pair(const float *p) { return ld_stream(rei
 // of a chunk of m columns at slot `off`.
 template <typename VT, int STRIDE>
 __device__ __forceinline__ double2 k1_sum(const VT *__restrict__ val, const UIN *__restrict__ col,
-                                          const FPT *__restrict__ x, size_t off, UIN kp0, UIN m, unsigned lane8) {
+                                          const FPT *x, size_t off, UIN kp0, UIN m, unsigned lane8) {
   using V2 = decltype(ld_pair((const VT *)nullptr));
   double a0[K1_U], a1[K1_U];
 #pragma unroll
@@ -121,8 +121,8 @@ __device__ __forceinline__ double2 k1_sum(const VT *__restrict__ val, const UIN 
     double x0[K1_U], x1[K1_U];
 #pragma unroll
     for (int u = 0; u < K1_U; u++) {
-      x0[u] = ldg(x + c[u].x);
-      x1[u] = ldg(x + c[u].y);
+      x0[u] = x[c[u].x];
+      x1[u] = x[c[u].y];
     }
 #pragma unroll
     for (int u = 0; u < K1_U; u++) {
@@ -146,8 +146,8 @@ __device__ __forceinline__ double2 k1_sum(const VT *__restrict__ val, const UIN 
 #pragma unroll
     for (int u = 0; u < K1_U - 1; u++) {
       if (k + (UIN)(u * STRIDE) < np) {
-        x0[u] = ldg(x + c[u].x);
-        x1[u] = ldg(x + c[u].y);
+        x0[u] = x[c[u].x];
+        x1[u] = x[c[u].y];
       }
     }
 #pragma unroll
@@ -165,9 +165,11 @@ template <typename VT, bool SCATTER>
 __global__ void __launch_bounds__(TPB) k1_chunks(UIN n, UIN chunkNum, UIN ncta, UIN nlong,
                                                  const UIN *__restrict__ chp, const UIN *__restrict__ nmc,
                                                  const UIN *__restrict__ permi, const UIN *__restrict__ col,
-                                                 const VT *__restrict__ val, const FPT *__restrict__ x,
-                                                 FPT *__restrict__ out, int beta) {
+                                                 const VT *__restrict__ val, const FPT *x_, FPT *out_, int beta) {
   pdl_trigger();
+  pdl_wait();  // the launch before this one wrote x, or still reads or writes out
+  const FPT *x = after_wait(x_);
+  FPT *out = after_wait(out_);
   __shared__ double2 part[TPB / 32][4];
   const unsigned lane = threadIdx.x & 31u, lane8 = lane & 7u, wib = threadIdx.x >> 5;
   size_t c;
@@ -235,6 +237,7 @@ inline size_t k1_ctas(UIN chunkNum, UIN ncta, UIN nlong) {
 // result; a programmatic dependent launch of k1_chunks where the stream
 // allows it, so it first waits for that grid and its writes.
 __global__ void k1_order(UIN n, const UIN *__restrict__ permi, const FPT *res_, FPT *y_, int beta) {
+  pdl_trigger();
   pdl_wait();
   const FPT *res = after_wait(res_);
   FPT *y = after_wait(y_);

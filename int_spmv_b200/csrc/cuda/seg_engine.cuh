@@ -105,6 +105,7 @@ __device__ __forceinline__ void finish(const State &st, const Out &o, size_t seg
 // returns at once for an ordinary launch).
 __global__ void fixup(size_t nrec, const UIN *rec_row_, const double *rec_sum_, const UIN *__restrict__ rowmap,
                       const UIN *__restrict__ empty, size_t nempty, FPT *y_, int beta) {
+  pdl_trigger();  // the next product's main kernel may launch; it waits for this grid
   pdl_wait();
   const UIN *rec_row = after_wait(rec_row_);
   const double *rec_sum = after_wait(rec_sum_);

@@ -29,8 +29,8 @@ namespace sl {
 template <typename VT, int U>
 __global__ void __launch_bounds__(pk::TPB, sizeof(VT) == 8 ? 4 : 5)
     slice_rows(UIN n, UIN nslices, const uint2 *__restrict__ meta, const uint8_t *__restrict__ len,
-               const uint16_t *__restrict__ d16, const VT *__restrict__ val, const FPT *__restrict__ x,
-               FPT *__restrict__ y, int beta) {
+               const uint16_t *__restrict__ d16, const VT *__restrict__ val, const FPT *x, FPT *y_, int beta) {
+  pdl_trigger();
   const UIN s = blockIdx.x * (pk::TPB / 32) + (threadIdx.x >> 5);
   if (s >= nslices) return;
   const unsigned lane = threadIdx.x & 31u;
@@ -39,7 +39,9 @@ __global__ void __launch_bounds__(pk::TPB, sizeof(VT) == 8 ? 4 : 5)
   const UIN r = s * 32u + lane;
   const UIN l = r < n ? (UIN)__ldg(len + r) : 0u;
   const bool full = __all_sync(FULL, l == w);
-  const FPT *const xb = x + m.y;
+  pdl_wait();
+  const FPT *const xb = after_wait(x + m.y);
+  FPT *const y = after_wait(y_);
   size_t p = (size_t)m.x * 32 + lane;
   double acc = 0.0;
   auto elements = [&](UIN k0, auto rest_c) {
@@ -55,7 +57,7 @@ __global__ void __launch_bounds__(pk::TPB, sizeof(VT) == 8 ? 4 : 5)
       }
 #pragma unroll
     for (int u = 0; u < U; u++)
-      if (!REST || k0 + u < w) xv[u] = ldg(xb + c[u]);
+      if (!REST || k0 + u < w) xv[u] = xb[c[u]];
 #pragma unroll
     for (int u = 0; u < U; u++)
       if (!REST || k0 + u < w) {

@@ -41,16 +41,23 @@ __device__ __forceinline__ void emit(const seg::Out &o, const Run &st, UIN row, 
   }
 }
 
-__device__ __forceinline__ void begin(Run &st, const seg::Out &o, size_t segid, UIN rbase, UIN first_word) {
+// A segment's state (writes nothing), and its head record's first value.
+__device__ __forceinline__ void begin_state(Run &st, size_t segid, UIN rbase, UIN first_word) {
   st.seg = (UIN)segid;
   st.rbase = rbase;
   st.carry = false;
   st.csum = 0.0;
   st.row_a = (first_word & 1u) ? NO_ROW : rbase - 1u;
+}
+__device__ __forceinline__ void begin_record(const seg::Out &o, size_t segid) {
   if ((threadIdx.x & 31u) == 0) {
     o.rec_row[2 * segid] = NO_ROW;
     o.rec_sum[2 * segid] = 0.0;
   }
+}
+__device__ __forceinline__ void begin(Run &st, const seg::Out &o, size_t segid, UIN rbase, UIN first_word) {
+  begin_state(st, segid, rbase, first_word);
+  begin_record(o, segid);
 }
 
 // Bitmap words of one batch of 32*SPL slots.

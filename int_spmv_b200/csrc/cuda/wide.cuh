@@ -127,8 +127,11 @@ __device__ __forceinline__ double madd(float v, float x, double acc) { return ac
 // then move 4 bytes per slot and an L1 line serves 32 columns.  VEC: x and
 // x32 are 16- and 8-byte aligned, two elements per thread and step.
 template <bool VEC>
-__global__ void __launch_bounds__(256) x_to_f32(size_t n, const FPT *__restrict__ x, float *__restrict__ x32) {
+__global__ void __launch_bounds__(256) x_to_f32(size_t n, const FPT *x_, float *x32_) {
   pdl_trigger();  // the product's main kernel may start loading its stream now
+  pdl_wait();     // the launch before this one wrote x, or still reads x32
+  const FPT *x = after_wait(x_);
+  float *x32 = after_wait(x32_);
   const size_t stride = (size_t)gridDim.x * 256;
   size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if constexpr (VEC) {
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(256) x_to_f32(size_t n, const FPT *__restrict_
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && (n & 1)) x32[n - 1] = __double2float_rn(x[n - 1]);
   } else {
-    for (; i < n; i += stride) x32[i] = __double2float_rn(__ldg(x + i));
+    for (; i < n; i += stride) x32[i] = __double2float_rn(x[i]);
   }
 }
 
@@ -155,9 +158,9 @@ struct Bands {
 // runs on the lanes whose column is in the window, the global load on the
 // others.
 template <int NW>
-__device__ __forceinline__ double gather(const Bands<NW> &w, uint32_t sx_addr, const FPT *__restrict__ x, UIN c) {
+__device__ __forceinline__ double gather(const Bands<NW> &w, uint32_t sx_addr, const FPT *x, UIN c) {
   if constexpr (NW == 0) {
-    return __ldg(x + c);
+    return x[c];
   } else {
     uint32_t in = 0, off = 0;
 #pragma unroll
@@ -173,7 +176,7 @@ __device__ __forceinline__ double gather(const Bands<NW> &w, uint32_t sx_addr, c
         ".reg .pred p;\n"
         "setp.ne.u32 p, %3, 0;\n"
         "@p ld.shared.f64 %0, [%1];\n"
-        "@!p ld.global.nc.f64 %0, [%2];\n"
+        "@!p ld.global.f64 %0, [%2];\n"
         "}\n"
         : "=d"(v)
         : "r"(sx_addr + 8u * off), "l"(x + c), "r"(in));
@@ -317,9 +320,12 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
       tma::fence_barrier_init();
     }
     __syncthreads();
-    if (threadIdx.x == 0 && len) {
-      tma::bar_expect_tx(&wbar, len * 8u);
-      tma::bulk_g2s(sx, x + lo, len * 8u, &wbar);
+    if (threadIdx.x < 32) {
+      pdl_wait();  // x may be written by the launch before this one
+      if (lane == 0 && len) {
+        tma::bar_expect_tx(&wbar, len * 8u);
+        tma::bulk_g2s(sx, after_wait(x) + lo, len * 8u, &wbar);
+      }
     }
     // each warp waits for the window just before its first gathers, so that
     // its first batch's values and columns load during the copy.  Warp 0
@@ -336,7 +342,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
   const size_t s1 = min(s0 + seg_slots, nslots_pad);
   const int nbat = (int)((s1 - s0) / BT);
   sss::Run st;
-  sss::begin(st, o, segid, segh[segid], __ldg(heads + (s0 >> 5)));
+  sss::begin_state(st, segid, segh[segid], __ldg(heads + (s0 >> 5)));
   UIN lo_base = NO_ROW;
   if constexpr (LO) lo_base = __ldg(nw.lo_off + segid);
   Cols<SPL> cnext;  // PFC: the columns of batch j + 1
@@ -372,16 +378,17 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
       for (int k = 0; k < SPL; k++) c[k] = e[k];
     }
     const unsigned bits = (__ldg(heads + (b >> 5) + ((SPL * lane) >> 5)) >> ((SPL * lane) & 31u)) & MASK;
-    const XT *xg = x;
-    cudaTextureObject_t tg = xtex;
-    if constexpr (sizeof(XT) == 4) {
-      // FP32 x is written by x_to_f32, of which this kernel is a programmatic
-      // dependent: its first batch's values and columns are loaded, now wait
-      // for that grid and its writes before the first gather
-      if (j == 0) pdl_wait();
-      xg = after_wait(xg);
-      if constexpr (TEX) tg = after_wait(tg);
+    // x may be written (FP32 copies: by x_to_f32) and y and the records still
+    // be used by the launches before this one, of which this kernel is a
+    // programmatic dependent: its first batch's values and columns are
+    // loaded, now wait for those grids and their writes
+    if (j == 0) {
+      pdl_wait();
+      sss::begin_record(o, segid);
     }
+    const XT *const xg = after_wait(x);  // written while this kernel may already run: no read-only loads
+    cudaTextureObject_t tg = xtex;
+    if constexpr (TEX) tg = after_wait(tg);
     if constexpr (STG) {
       if (wlen) {  // first batch: the window must have landed (bounded wait)
         wlen = 0;
@@ -398,7 +405,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
 #pragma unroll
     for (int k = 0; k < SPL; k++) {
       if constexpr (NW > 0) {
-        xv[k] = gather<NW>(w, sxa, x, c[k]);
+        xv[k] = gather<NW>(w, sxa, xg, c[k]);
       } else if constexpr (TEX) {
         if constexpr (sizeof(XT) == 8) {
           const int2 t = tex1Dfetch<int2>(tg, (int)c[k]);
@@ -406,10 +413,8 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
         } else {
           xv[k] = tex1Dfetch<float>(tg, (int)c[k]);
         }
-      } else if constexpr (sizeof(XT) == 4) {
-        xv[k] = xg[c[k]];  // written while this kernel may already run: no read-only load
       } else {
-        xv[k] = __ldg(x + c[k]);
+        xv[k] = xg[c[k]];
       }
     }
     VT vv[SPL];

@@ -42,3 +42,66 @@ def test_f32_products_beside_other_work(variant):
         torch.cuda.current_stream().synchronize()
         wrong += not torch.equal(y, alone[i % 3])
     assert wrong == 0
+
+
+CHAINS = [("CSR", {}), ("CSR", dict(kernel="wide", variant=26)), ("CSR", dict(kernel="wide", variant=4)),
+          ("CSR", dict(kernel="wide", variant=11)), ("CSR", dict(kernel="wide", variant=16)),
+          ("CSR", dict(val="f32")), ("CSR", dict(val="f32", kernel="wide", variant=16)),
+          ("CSR", dict(val="f32lo")), ("CSR", dict(col="d16", kernel="wide", variant=9)), ("STENCIL", dict(col="d16")),
+          ("STENCIL", dict(val="f32", col="d16")), ("STENCIL", {}), ("K1", {}), ("K1P", {}), ("CSR", dict(kernel="ldg"))]
+
+
+@pytest.mark.parametrize("fmt,kw", CHAINS)
+@pytest.mark.parametrize("spmm", [0, 8, 11, 32])
+def test_products_in_a_chain(fmt, kw, spmm):
+    """Products whose x is the y of the product before (through one more
+    kernel, or directly), enqueued without a wait on a GPU that other work
+    keeps busy: each may start while the one before it finishes, and gives the
+    bits it gives alone."""
+    import numpy as np
+    import torch
+
+    from int_spmv_b200 import device as D
+    from int_spmv_b200 import formats as F
+    from int_spmv_b200 import matrices as M
+    if spmm and (fmt.startswith("K1") or "d16" in kw.values() or kw.get("val") == "f32lo"):
+        pytest.skip("SpMM needs a slot-stream plan with u32 columns")
+    row, col, val = M.stencil27(30) if fmt == "STENCIL" else M.random_csr(40_000, 5, rl_max=24, empty_frac=0.05)
+    if fmt != "STENCIL":
+        col = col.copy()
+    csr = F.CSR(row, col, val / np.abs(val).max() * 0.1)
+    f = F.getFormatDataK1(8, csr, np.zeros(csr.n))[1] if fmt.startswith("K1") else None
+    plan = D.Plan(csr, f, **({"reorder": fmt == "K1P"} if f is not None else {}), **kw)
+    shape = (csr.n, spmm) if spmm else (csr.n,)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x0 = torch.rand(shape, dtype=torch.float64, device="cuda", generator=g)
+
+    def chain(wait):
+        a, b = x0.clone(), torch.ones_like(x0)
+        for i in range(24):
+            if spmm:
+                plan.spmm(a, b)
+            elif i % 8 == 7:
+                plan.spmv_graph(a, b)
+            else:
+                plan.spmv(a, b, beta=i % 3 == 1)
+            if wait:
+                torch.cuda.synchronize()
+            if i % 2:
+                b.mul_(0.5).add_(a, alpha=0.25)
+            a, b = b, a
+            if wait:
+                torch.cuda.synchronize()
+        return a
+
+    alone = chain(True).clone()
+    torch.cuda.synchronize()
+    m = torch.randn(2048, 2048, device="cuda")
+    side = torch.cuda.Stream()
+    for _ in range(6):
+        with torch.cuda.stream(side):
+            for _ in range(8):
+                m @ m
+        got = chain(False)
+        torch.cuda.synchronize()
+        assert torch.equal(got, alone)
