@@ -281,28 +281,38 @@ WideCfg wide_variant(int v) {
 }
 
 // Slots per warp segment of a lane-interleaved plan of `slots` slots: the
-// variant's segment at most, and short enough that every warp the GPU holds
-// at once has one.  A warp works its batches of 32*spl slots one after the
-// other, about 1.5 us each when little else runs, so a matrix below one full
-// load of warps takes the time of its longest warp.  Near one load and above
-// it, the segments are cut so that the last load is nearly full (3% slack):
-// 1.24 loads of 3072 slots take 30.9 us where 0.93 of 4096 take 25.6
-// (27-point stencil, 80^3, FP32 values).  The bulk-copy staged kernel's
-// persistent warps take segments in turn: 2.3 each leave a quarter of the
-// warps idle in the last turn.  Measured against the variants' fixed segments:
-// 5-point 512^2 15.6 -> 10.6 us (from 2048 slots, padding dropped), power-law n =
-// 30,000 17.8 -> 8.4 us, 32 FEM blocks of 22M nonzeros in one graph 57.2 ->
-// 54.8 us (staged, from 4096).
+// variant's segment at most, and short enough that the warps fill the GPU.  A
+// warp works its batches of 32*spl slots one after the other, about 1.5 us
+// each when little else runs, so a matrix below one full load of warps (as
+// many as the GPU holds at once) takes the time of its longest warp, and one
+// a little above a whole number of loads pays for the next one: 1.24 loads of
+// 3072 slots take 30.9 us where 0.93 of 4096 take 25.6 and 1.85 of 2048 26.9
+// (27-point stencil, 80^3, FP32 values).  The longest segments whose last load
+// is at least 0.9 full are taken, else the ones that fill it best; beyond
+// four loads the last one hardly shows.  The bulk-copy staged kernel's
+// persistent warps take segments in turn, 8 or more each.  Measured against
+// the variants' fixed segments: 5-point 512^2 15.6 -> 10.6 us (from 2048
+// slots, padding dropped), power-law n = 30,000 17.8 -> 8.4 us, 32 FEM blocks
+// of 22M nonzeros in one graph 57.2 -> 54.8 us (staged, from 4096).
 size_t wide_seg(const WideCfg &w, size_t slots) {
   if (w.tmem) return w.seg;
-  if (w.tma) {  // persistent warps, segments dealt in turn: at least 8 per warp
+  if (w.tma) {
     const size_t s = slots / ((size_t)sm_count() * 4 * w.warps * 8);
     return std::min(w.seg, std::max(SS, (s + SS - 1) / SS * SS));
   }
-  const size_t held = (size_t)sm_count() * w.minb * WIDE_WARPS * 97 / 100;
-  const size_t loads = std::max<size_t>(1, (slots + held * w.seg - 1) / (held * w.seg));
-  const size_t s = (slots + loads * held - 1) / (loads * held);
-  return std::min(w.seg, std::max(SS, (s + SS - 1) / SS * SS));
+  const double held = (double)sm_count() * w.minb * WIDE_WARPS;
+  size_t best = w.seg;
+  double best_fill = 0.0;
+  for (size_t s = w.seg; s >= SS; s -= SS) {
+    const double loads = std::ceil((double)slots / (double)s) / held;
+    const double fill = std::max(loads / std::ceil(loads), loads > 4.0 ? 0.93 : 0.0);
+    if (fill > best_fill) {
+      best = s;
+      best_fill = fill;
+    }
+    if (fill >= 0.9) break;
+  }
+  return best;
 }
 
 // Fraction of a deterministic sample of the nonzeros whose column lies
