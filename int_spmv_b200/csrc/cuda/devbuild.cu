@@ -12,8 +12,8 @@
 // (row << log2 bs) | min(left - 1, bs - 1 - s%bs) at row and block starts.
 // Padding is zero.  The arrays are bit-identical to the host builder's.
 //
-// Steps: row slot counts -> exclusive prefix (three scan kernels over u64)
-// -> sizes read back to the host (one synchronisation, to allocate) ->
+// Steps: row slot counts -> exclusive prefix (three scan kernels over u64;
+// COM: the row pointer is the prefix) -> sizes read back to the host (one synchronisation, to allocate) ->
 // a CTA per 256 rows writes their slots.
 //
 // The K1 arrays of getFormatDataK1 (M:841-905) likewise: rows sorted by
@@ -47,6 +47,17 @@ __global__ void row_slots(UIN n, const UIN *__restrict__ row, UIN grp, int noc, 
   }
   const uint64_t l = row[r + 1] - row[r];
   cnt[r] = noc ? (l + grp - 1) / grp * grp : l;
+}
+
+// COM mode's slots are the CSR's own (row[r] - row[0]): no prefix, only this
+// check.  found = {row[0], row[n], 1 if the row pointer decreases}.
+__global__ void check_rows(UIN n, const UIN *__restrict__ row, UIN *__restrict__ found) {
+  const size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  const UIN a = row[r], e = row[r + 1];
+  if (e < a) found[2] = 1;
+  if (r == 0) found[0] = a;
+  if (r == n - 1) found[1] = e;
 }
 
 // Exclusive prefix of one block's SB items; bsum[b] = the block's total.
@@ -154,20 +165,22 @@ __global__ void __launch_bounds__(256) fill_axt(UIN n, const UIN *__restrict__ r
                                                 const uint64_t *__restrict__ off, UIN slots, UIN th, UIN bs, UIN lg,
                                                 UIN *__restrict__ con, FPT *__restrict__ ax, UIN *__restrict__ sec) {
   __shared__ UIN soff[FILL_ROWS], srow[FILL_ROWS], slen[FILL_ROWS], send;
-  const UIN total = (UIN)off[n];
+  const UIN first = off ? 0 : row[0];
+  auto start = [&](size_t r) { return off ? (UIN)off[r] : row[r] - first; };  // COM: no prefix needed
+  const UIN total = start(n);
   const size_t r0 = (size_t)blockIdx.x * FILL_ROWS;
   const bool tail = r0 >= n;  // the slots past the last row's
   {
     const size_t r = r0 + threadIdx.x;
     soff[threadIdx.x] = 0xFFFFFFFFu;
     if (r < n) {
-      const UIN s0 = (UIN)off[r], j0 = row[r];
+      const UIN s0 = start(r), j0 = row[r];
       soff[threadIdx.x] = s0;
       srow[threadIdx.x] = j0;
       slen[threadIdx.x] = row[r + 1] - j0;
       con[r] = axt_pos(s0, th);
     }
-    if (threadIdx.x == 0) send = tail ? slots : (UIN)off[min(r0 + FILL_ROWS, (size_t)n)];
+    if (threadIdx.x == 0) send = tail ? slots : start(min(r0 + FILL_ROWS, (size_t)n));
   }
   __syncthreads();
   const UIN a = tail ? total : soff[0], e = send, ths = 8 * th;
@@ -331,20 +344,36 @@ ISPMV_API int ispmv_dev_build_axt(UIN bs, UIN thw, UIN th, const char *mode, UIN
   } while (0)
   DB_TRY(cudaEventCreate(&e0));
   DB_TRY(cudaEventCreate(&e1));
-  DB_ALLOC(cnt, len * sizeof(uint64_t));
-  DB_ALLOC(off, len * sizeof(uint64_t));
-  DB_ALLOC(bsum, nb * sizeof(uint64_t));
-  DB_TRY(cudaEventRecord(e0, s));
-  row_slots<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(n, d_row, grp, noc, cnt);
-  if ((st = check_launch("row_slots"))) goto done;
-  scan_block<<<(unsigned)nb, ST, 0, s>>>(len, cnt, off, bsum);
-  if ((st = check_launch("scan_block"))) goto done;
-  scan_totals<<<1, ST, 0, s>>>(nb, bsum);
-  if ((st = check_launch("scan_totals"))) goto done;
-  add_block_offsets<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(len, off, bsum);
-  if ((st = check_launch("add_block_offsets"))) goto done;
-  DB_TRY(cudaMemcpyAsync(&slots, off + n, sizeof slots, cudaMemcpyDeviceToHost, s));
-  DB_TRY(cudaStreamSynchronize(s));
+  if (com) {
+    UIN found[3] = {0, 0, 0};
+    DB_ALLOC(bsum, sizeof found);
+    DB_TRY(cudaEventRecord(e0, s));
+    DB_TRY(cudaMemsetAsync(bsum, 0, sizeof found, s));
+    check_rows<<<(unsigned)(((size_t)n + 255) / 256), 256, 0, s>>>(n, d_row, reinterpret_cast<UIN *>(bsum));
+    if ((st = check_launch("check_rows"))) goto done;
+    DB_TRY(cudaMemcpyAsync(found, bsum, sizeof found, cudaMemcpyDeviceToHost, s));
+    DB_TRY(cudaStreamSynchronize(s));
+    if (found[2] || found[1] < found[0]) {  // row lengths that wrap
+      st = ISPMV_ERR_OVERFLOW;
+      goto done;
+    }
+    slots = found[1] - found[0];
+  } else {
+    DB_ALLOC(cnt, len * sizeof(uint64_t));
+    DB_ALLOC(off, len * sizeof(uint64_t));
+    DB_ALLOC(bsum, nb * sizeof(uint64_t));
+    DB_TRY(cudaEventRecord(e0, s));
+    row_slots<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(n, d_row, grp, noc, cnt);
+    if ((st = check_launch("row_slots"))) goto done;
+    scan_block<<<(unsigned)nb, ST, 0, s>>>(len, cnt, off, bsum);
+    if ((st = check_launch("scan_block"))) goto done;
+    scan_totals<<<1, ST, 0, s>>>(nb, bsum);
+    if ((st = check_launch("scan_totals"))) goto done;
+    add_block_offsets<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(len, off, bsum);
+    if ((st = check_launch("add_block_offsets"))) goto done;
+    DB_TRY(cudaMemcpyAsync(&slots, off + n, sizeof slots, cudaMemcpyDeviceToHost, s));
+    DB_TRY(cudaStreamSynchronize(s));
+  }
   {
     // every row's slot count is a multiple of th in NOC mode and th == 1 in COM mode
     const uint64_t columns = slots / th, tiles = (columns + thw - 1) / thw;

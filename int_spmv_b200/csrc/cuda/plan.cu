@@ -289,7 +289,7 @@ WideCfg wide_variant(int v) {
 // 3072 slots take 30.9 us where 0.93 of 4096 take 25.6 and 1.85 of 2048 26.9
 // (27-point stencil, 80^3, FP32 values).  The longest segments whose last load
 // is at least 0.9 full are taken, else the ones that fill it best; beyond
-// four loads the last one hardly shows.  The bulk-copy staged kernel's
+// three loads the last one hardly shows.  The bulk-copy staged kernel's
 // persistent warps take segments in turn, 8 or more each.  Measured against
 // the variants' fixed segments: 5-point 512^2 15.6 -> 10.6 us (from 2048
 // slots, padding dropped), power-law n = 30,000 17.8 -> 8.4 us, 32 FEM blocks
@@ -305,7 +305,7 @@ size_t wide_seg(const WideCfg &w, size_t slots) {
   double best_fill = 0.0;
   for (size_t s = w.seg; s >= SS; s -= SS) {
     const double loads = std::ceil((double)slots / (double)s) / held;
-    const double fill = std::max(loads / std::ceil(loads), loads > 4.0 ? 0.93 : 0.0);
+    const double fill = std::max(loads / std::ceil(loads), loads > 3.0 ? 0.93 : 0.0);
     if (fill > best_fill) {
       best = s;
       best_fill = fill;
@@ -398,7 +398,7 @@ WinGeom win_geom(UIN n, UIN cap) {
   g.w2 = std::max<UIN>(1, g.W >> g.s2);
   return g;
 }
-__host__ __device__ inline bool win_sampled(size_t slot) { return ((slot >> 3) & 3u) == 0; }
+__host__ __device__ inline bool win_sampled(size_t slot) { return ((slot >> 3) & 7u) == 0; }
 
 // The first start of the `w` neighbouring bins with the most counts.
 UIN best_run(const UIN *h, UIN nb, UIN w) {
@@ -962,7 +962,7 @@ __device__ UIN cta_best_run(UIN *h, UIN nb, UIN w, unsigned long long *red) {
   return 0xFFFFFFFFu - (UIN)best;
 }
 
-// One CTA per plan CTA tile: stage_windows' choice.  Reads a quarter of the
+// One CTA per plan CTA tile: stage_windows' choice.  Reads an eighth of the
 // columns (twice, the second time from L2); a sort of every tile's columns
 // and a search for the densest interval took 690 us of the 860 a plan's
 // kernels did at n = 1M, 14.9M nonzeros.
@@ -974,9 +974,9 @@ __global__ void __launch_bounds__(256) dcsr_windows(WinGeom g, size_t T, size_t 
   auto count = [&](UIN nb, UIN lo, UIN s) {
     for (UIN i = threadIdx.x; i < WH(nb) + 1; i += 256) h[i] = 0;
     __syncthreads();
-    // groups of 8 slots 0, 4, 8, ... of the tile (T is a multiple of 32)
+    // groups of 8 slots 0, 8, 16, ... of the tile (T is a multiple of 64)
     for (size_t k = threadIdx.x;; k += 256) {
-      const size_t q = a + (k >> 3) * 32 + (k & 7u);
+      const size_t q = a + (k >> 3) * 64 + (k & 7u);
       if (q >= e) break;
       const UIN c = col[q];
       if (c >= lo && ((c - lo) >> s) < nb) atomicAdd(&h[WH((c - lo) >> s)], 1u);

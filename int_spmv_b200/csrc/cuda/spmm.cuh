@@ -106,7 +106,7 @@ __device__ __forceinline__ void st_y(double *p, int ncol, const double (&d)[W]) 
 template <int G, typename VT>
 struct alignas(16) Chunk {
   VT v[4 * G + 16 / sizeof(VT)];
-  UIN c[4 * G + 4];
+  UIN c[4 * G + (G == 2 ? 8 : 4)];
 };
 
 template <int G, int W, int T, int MINB, bool VEC, typename VT>
