@@ -154,7 +154,7 @@ __device__ __forceinline__ UIN axt_pos(UIN s, UIN th) {
 // steps), so neighbouring threads read and write neighbouring slots whatever
 // the rows' lengths.  Bound by the bytes it moves: at power-law n = 1M,
 // 14.9M nonzeros, one warp per row after two memsets took 270 us and 60, this
-// takes 132 (477 MB, 74 us at the copy rate; x is gathered).  A last CTA, past the rows, fills the last tile.
+// takes 124 (477 MB, 74 us at the copy rate; x is gathered).  A last CTA, past the rows, fills the last tile.
 // TILES (th > 1): slots in ax order (tile, sub-row, column), so that the
 // writes are contiguous; only the CTA's own slots of its first and last tile.
 constexpr int FILL_ROWS = 256;
@@ -184,50 +184,84 @@ __global__ void __launch_bounds__(256) fill_axt(UIN n, const UIN *__restrict__ r
   }
   __syncthreads();
   const UIN a = tail ? total : soff[0], e = send, ths = 8 * th;
-  auto slot = [&](UIN s, UIN p) {
-    if (tail) {
-      ax[p] = (FPT)0;
-      ax[p + 8] = (FPT)0;
-      if (COM) sec[s] = 0;
-      else if (s % th == 0 && (th > 1 || (s & 7u) == 0)) sec[th == 1 ? s >> 3 : s / th] = 0;
-      return;
-    }
-    UIN q = 0;  // the last row that starts at or before s (empty rows before it start there too)
+  // a slot past the last row: zeros
+  auto pad = [&](UIN s, UIN p) {
+    ax[p] = (FPT)0;
+    ax[p + 8] = (FPT)0;
+    if (COM) sec[s] = 0;
+    else if (s % th == 0 && (th > 1 || (s & 7u) == 0)) sec[th == 1 ? s >> 3 : s / th] = 0;
+  };
+  // U slots at positions p: their rows, then values and columns, then x, then
+  // the writes, so that the loads of all U are in flight together
+  constexpr int U = 4;
+  auto slots_of = [&](const UIN (&s)[U], const UIN (&p)[U], const bool (&on)[U]) {
+    UIN q[U], k[U];
+    FPT v[U], xv[U];
+    UIN c[U];
+    bool in[U];
 #pragma unroll
-    for (UIN d = FILL_ROWS / 2; d > 0; d >>= 1)
-      if (soff[q + d] <= s) q += d;
-    const UIN k = s - soff[q], len = slen[q];
-    FPT v = (FPT)0, xv = (FPT)0;
-    if (COM || k < len) {
-      const UIN j = srow[q] + k;
-      v = ld_stream(val + j);
-      xv = ldg(x + ld_stream(col + j));
+    for (int i = 0; i < U; i++) {
+      q[i] = 0;  // the last row that starts at or before s (empty rows before it start there too)
+#pragma unroll
+      for (UIN d = FILL_ROWS / 2; d > 0; d >>= 1)
+        if (soff[q[i] + d] <= s[i]) q[i] += d;
+      k[i] = s[i] - soff[q[i]];
+      in[i] = on[i] && (COM || k[i] < slen[q[i]]);
     }
-    ax[p] = v;
-    ax[p + 8] = xv;
-    const UIN r = (UIN)r0 + q;
-    if (COM) {
-      UIN d = 0;
-      if (k == 0 || (s & (bs - 1)) == 0) {
-        const UIN q1 = len - k - 1, q2 = bs - 1 - (s & (bs - 1));
-        d = (r << lg) | min(q1, q2);
+#pragma unroll
+    for (int i = 0; i < U; i++) {
+      const size_t j = in[i] ? (size_t)srow[q[i]] + k[i] : 0;
+      v[i] = in[i] ? ld_stream(val + j) : (FPT)0;
+      c[i] = in[i] ? ld_stream(col + j) : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < U; i++) xv[i] = in[i] ? ldg(x + c[i]) : (FPT)0;
+#pragma unroll
+    for (int i = 0; i < U; i++) {
+      if (!on[i]) continue;
+      ax[p[i]] = v[i];
+      ax[p[i] + 8] = xv[i];
+      const UIN r = (UIN)r0 + q[i];
+      if (COM) {
+        UIN d = 0;
+        if (k[i] == 0 || (s[i] & (bs - 1)) == 0) {
+          const UIN q1 = slen[q[i]] - k[i] - 1, q2 = bs - 1 - (s[i] & (bs - 1));
+          d = (r << lg) | min(q1, q2);
+        }
+        sec[s[i]] = d;
+      } else if (th == 1) {
+        if ((s[i] & 7u) == 0) sec[s[i] >> 3] = r;
+      } else if (s[i] % th == 0) {
+        sec[s[i] / th] = r;
       }
-      sec[s] = d;
-    } else if (th == 1) {
-      if ((s & 7u) == 0) sec[s >> 3] = r;
-    } else if (s % th == 0) {
-      sec[s / th] = r;
     }
   };
-  if (TILES) {
-    for (uint64_t i = (uint64_t)(a / ths) * ths + threadIdx.x; i < ((uint64_t)e + ths - 1) / ths * ths; i += 256) {
+  // item i of the CTA: a slot, or (TILES) a place in ax order
+  const uint64_t i0 = TILES ? (uint64_t)(a / ths) * ths : a;
+  const uint64_t i1 = TILES ? ((uint64_t)e + ths - 1) / ths * ths : e;
+  auto place = [&](uint64_t i, UIN &s, UIN &p) {
+    if (TILES) {
       const UIN T = (UIN)(i / ths), w = (UIN)i - T * ths, R = w >> 3, C = w & 7u;
-      const UIN s = T * ths + C * th + R;
-      if (s >= a && s < e) slot(s, T * 2 * ths + R * 16 + C);
+      s = T * ths + C * th + R;
+      p = T * 2 * ths + R * 16 + C;
+      return i < i1 && s >= a && s < e;
     }
-  } else {
-#pragma unroll 4
-    for (uint64_t s = (uint64_t)a + threadIdx.x; s < e; s += 256) slot((UIN)s, axt_pos((UIN)s, th));
+    s = (UIN)i;
+    p = axt_pos(s, th);
+    return i < i1;
+  };
+  for (uint64_t i = i0 + threadIdx.x; i < i1; i += 256 * U) {
+    UIN s[U], p[U];
+    bool on[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) on[u] = place(i + 256 * u, s[u], p[u]);
+    if (tail) {
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (on[u]) pad(s[u], p[u]);
+    } else {
+      slots_of(s, p, on);
+    }
   }
 }
 
