@@ -415,7 +415,8 @@ typedef struct {
   int units_per_warp;/* work granule of one warp; 0 = library default */
   double lo_tol;     /* F32_LO16: rows whose FP32 rounding error bound exceeds
                         lo_tol relative carry a lo-word; 0 = default 1e-6 */
-  int variant;       /* kernel variant (prefetch depth / register budget); 0 = default;
+  int variant;       /* kernel variant (prefetch depth / register budget; WIDE: the slots per warp
+                        segment are the variant's at most, fewer on small matrices); 0 = default;
                         ISPMV_VARIANT_QUEUE = persistent warps pulling segments
                         from a device work queue */
   int rhs_block;     /* SpMM right-hand sides per pass: 8, 16 or 32; 0 = by k */
@@ -429,7 +430,9 @@ typedef struct {
 void ispmv_plan_opts_default(ispmv_plan_opts *o);
 
 /* Plans from host-built formats.  The host arrays are only read during the
- * call; the plan owns its device copies.  `csr` must have rl filled. */
+ * call; the plan owns its device copies.  `csr` must have rl filled.  The
+ * slot-stream kernels' plans hold the rows back to back, without the padding
+ * of AXC bricks and AXT tiles (info.slots counts the format's slots). */
 int ispmv_plan_csr(const str_matCSR *csr, const ispmv_plan_opts *o, ispmv_plan *out);
 int ispmv_plan_axc(const str_matCSR *csr, const str_matAXC *axc, const UIN *axi,
                    const ispmv_plan_opts *o, ispmv_plan *out);

@@ -1051,6 +1051,8 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
   const WideCfg wc = wide_variant(p->opts.variant);
   if (!wc.ok || wc.tmem)
     return fail(ISPMV_ERR_UNSUPPORTED, "plan from a device CSR: the lane-interleaved kernel without TMEM staging");
+  if (wc.stg && nnz > 0x7FFFFFFFu)
+    return fail(ISPMV_ERR_UNSUPPORTED, "plan from a device CSR: per-CTA x windows up to 2^31 - 1 nonzeros");
   p->fmt = F_CSR;
   p->path = P_STREAM;
   p->slots = p->fslots = nnz;
@@ -1415,12 +1417,12 @@ int launch_staged_w(K kernel, size_t smem, size_t nseg, int ctas_per_sm, cudaStr
   return check_launch(what);
 }
 
-// A launch that may start while the launches before it in the stream finish
-// (its kernel waits for them before it touches anything but the plan's
+// A launch; `early`: it may start while the launches before it in the stream
+// finish (its kernel waits for them before it touches anything but the plan's
 // constant arrays), unless a timing event sits between.
 template <typename... KA, typename... A>
 int launch_dependent(const ispmv_plan_s *p, const char *name, void (*k)(KA...), size_t grid, unsigned block,
-                     size_t smem, cudaStream_t s, A... a) {
+                     size_t smem, cudaStream_t s, bool early, A... a) {
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -1430,7 +1432,7 @@ int launch_dependent(const ispmv_plan_s *p, const char *name, void (*k)(KA...), 
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = at;
-  cfg.numAttrs = !p->tcap || p->capturing ? 1 : 0;
+  cfg.numAttrs = early && (!p->tcap || p->capturing) ? 1 : 0;
   ISPMV_TRY(cudaLaunchKernelEx(&cfg, k, static_cast<KA>(a)...));
   return check_launch(name);
 }
@@ -1474,26 +1476,29 @@ template <typename VT, int SPL, int MINB, bool D16 = false, bool TEX = false, bo
           bool PFC = false>
 int launch_wide(ispmv_plan_s *p, const FPT *x, seg::Out &o, cudaStream_t s, const char *name) {
   constexpr int NW = STG ? 1 : 0;
+  const size_t ctas = (p->nseg + WIDE_WARPS - 1) / WIDE_WARPS;
+  const bool early = STG || ctas <= (size_t)sm_count() * MINB;  // one load of CTAs: stream_wide's DEP form
   if constexpr (sizeof(VT) == 4 && !STG && !LO) {
     // FP32 values: gather from an FP32 copy of x (the value the FP32 multiply uses)
     if (!p->x32) TRY(dev_alloc(p, p->n, &p->x32));
     const unsigned gc = (unsigned)std::min<size_t>(((size_t)p->n / 2 + 255) / 256, (size_t)sm_count() * 8) + 1;
     auto *kx = (reinterpret_cast<uintptr_t>(x) & 15u) == 0 ? wide::x_to_f32<true> : wide::x_to_f32<false>;
-    TRY(launch_dependent(p, "x_to_f32", kx, gc, 256, 0, s, p->n, x, p->x32));
+    TRY(launch_dependent(p, "x_to_f32", kx, gc, 256, 0, s, true, p->n, x, p->x32));
     const cudaTextureObject_t tx = TEX ? x_texture(p, p->x32, (size_t)p->n * 4, true) : 0;
     if (TEX && !tx) return launch_wide<VT, SPL, MINB, D16, false>(p, x, o, s, "stream_wide<tex: x gathered with loads>");
-    return launch_dependent(p, name, wide::stream_wide<VT, float, SPL, 0, WIDE_WARPS, MINB, D16, TEX, false, false, PFC>,
-                            (p->nseg + WIDE_WARPS - 1) / WIDE_WARPS, WIDE_WARPS * 32, 0, s, p->slots, p->slots_pad,
-                            p->seg_slots, p->nseg, static_cast<const VT *>(p->val), p->col, p->heads, p->segh, p->xw,
-                            p->x32, o, p->narrow, tx);
+    auto *k = early ? wide::stream_wide<VT, float, SPL, 0, WIDE_WARPS, MINB, D16, TEX, false, false, PFC, true>
+                    : wide::stream_wide<VT, float, SPL, 0, WIDE_WARPS, MINB, D16, TEX, false, false, PFC, false>;
+    return launch_dependent(p, name, k, ctas, WIDE_WARPS * 32, 0, s, early, p->slots, p->slots_pad, p->seg_slots,
+                            p->nseg, static_cast<const VT *>(p->val), p->col, p->heads, p->segh, p->xw, p->x32, o,
+                            p->narrow, tx);
   } else {
     const cudaTextureObject_t tx = TEX ? x_texture(p, x, (size_t)p->n * 8, false) : 0;
     if (TEX && !tx) return launch_wide<VT, SPL, MINB, D16, false>(p, x, o, s, "stream_wide<tex: x gathered with loads>");
-    auto *k = wide::stream_wide<VT, double, SPL, NW, WIDE_WARPS, MINB, D16, TEX, STG, LO, PFC>;
+    auto *k = early ? wide::stream_wide<VT, double, SPL, NW, WIDE_WARPS, MINB, D16, TEX, STG, LO, PFC, true>
+                    : wide::stream_wide<VT, double, SPL, NW, WIDE_WARPS, MINB, D16, TEX, STG, LO, PFC, STG>;
     const size_t smem = STG ? (size_t)p->xw.cap * sizeof(double) : 0;
     if (smem) ISPMV_TRY(cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return launch_dependent(p, name, k, (p->nseg + WIDE_WARPS - 1) / WIDE_WARPS, WIDE_WARPS * 32, smem, s, p->slots,
-                            p->slots_pad, p->seg_slots, p->nseg, static_cast<const VT *>(p->val), p->col, p->heads,
+    return launch_dependent(p, name, k, ctas, WIDE_WARPS * 32, smem, s, early, p->slots, p->slots_pad, p->seg_slots, p->nseg, static_cast<const VT *>(p->val), p->col, p->heads,
                             p->segh, p->xw, x, o, p->narrow, tx);
   }
 }
@@ -1749,14 +1754,14 @@ int run_main(ispmv_plan_s *p, const FPT *x, FPT *y, int beta, cudaStream_t s) {
       const UIN ns = (p->n + 31) / 32;
       auto *k = p->slice_w <= 5 ? sl::slice_rows<VT, 5> : sl::slice_rows<VT, 9>;
       return launch_dependent(p, "stream_wide<rows32,d16>", k, (ns + pk::TPB / 32 - 1) / (pk::TPB / 32), pk::TPB, 0, s,
-                              p->n, ns, p->slices, p->slen, p->narrow.col16, val, x, y, beta);
+                              true, p->n, ns, p->slices, p->slen, p->narrow.col16, val, x, y, beta);
     }
     case P_K1: {
       const unsigned g = (unsigned)pk::k1_ctas(p->chunkNum, p->k1_cta, p->k1_long);
       if (p->fmt == F_K1P)
-        return launch_dependent(p, "k1_chunks<scatter>", pk::k1_chunks<VT, true>, g, pk::TPB, 0, s, p->n, p->chunkNum,
+        return launch_dependent(p, "k1_chunks<scatter>", pk::k1_chunks<VT, true>, g, pk::TPB, 0, s, true, p->n, p->chunkNum,
                                 p->k1_cta, p->k1_long, p->chp, p->nmc, p->permi, p->col, val, x, y, beta);
-      return launch_dependent(p, "k1_chunks", pk::k1_chunks<VT, false>, g, pk::TPB, 0, s, p->n, p->chunkNum, p->k1_cta,
+      return launch_dependent(p, "k1_chunks", pk::k1_chunks<VT, false>, g, pk::TPB, 0, s, true, p->n, p->chunkNum, p->k1_cta,
                               p->k1_long, p->chp, p->nmc, p->permi, p->col, val, x, p->res, beta);
     }
     case P_STREAM:
@@ -1935,7 +1940,7 @@ int spmm_blocks(ispmv_plan_s *p, UIN k, const FPT *X, FPT *Y, cudaStream_t s, co
     TRY(check_launch(name));
     p->kname = last_launch();
     TRY(launch_dependent(p, "spmm_fixup", mm::spmm_fixup<CB>, (std::max(nrec, p->nempty) * CB + 255) / 256, 256, 0, s,
-                         nrec, p->empty, p->nempty, o));
+                         true, nrec, p->empty, p->nempty, o));
   }
   return ISPMV_OK;
 }

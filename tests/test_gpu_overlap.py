@@ -105,3 +105,66 @@ def test_products_in_a_chain(fmt, kw, spmm):
         got = chain(False)
         torch.cuda.synchronize()
         assert torch.equal(got, alone)
+
+
+@pytest.mark.parametrize("kw", [dict(kernel="wide", variant=26), dict(kernel="wide", variant=11), dict(val="f32"),
+                                dict(col="d16"), dict(fmt="K1P"), dict(fmt="K1")])
+@pytest.mark.parametrize("before", ["kernel", "memset", "copy", "join", "nothing"])
+def test_products_in_a_captured_graph(kw, before):
+    """Products captured into a caller's CUDA graph after a kernel, a memset, a
+    copy, the join of another stream, or as its first node: replays give what
+    the same calls give outside."""
+    import numpy as np
+    import torch
+
+    from int_spmv_b200 import device as D
+    from int_spmv_b200 import formats as F
+    from int_spmv_b200 import matrices as M
+    kw = dict(kw)
+    fmt = kw.pop("fmt", "CSR")
+    row, col, val = M.stencil27(24)
+    csr = F.CSR(row, col, val / 60.0)
+    f = F.getFormatDataK1(8, csr, np.zeros(csr.n))[1] if fmt != "CSR" else None
+    plan = D.Plan(csr, f, **({"reorder": fmt == "K1P"} if f is not None else {}), **kw)
+    src = torch.rand(csr.n, dtype=torch.float64, device="cuda")
+    x, y, z = src.clone(), torch.zeros_like(src), torch.zeros_like(src)
+    side = torch.cuda.Stream()
+
+    def step():
+        if before == "kernel":
+            x.mul_(0.5).add_(1.0)
+        elif before == "memset":
+            y.zero_()
+        elif before == "copy":
+            x.copy_(src)
+        elif before == "join":
+            s = torch.cuda.current_stream()
+            side.wait_stream(s)
+            with torch.cuda.stream(side):
+                x.mul_(0.75)
+            s.wait_stream(side)
+        plan.spmv(x, y)
+        plan.spmv(y, z, beta=1)
+        x.add_(z, alpha=0.125)
+
+    def start():
+        x.copy_(src), y.zero_(), z.zero_()
+
+    start()
+    torch.cuda.synchronize()
+    for _ in range(5):
+        step()
+        torch.cuda.synchronize()
+    want = [t.clone() for t in (x, y, z)]
+    start()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    start()
+    torch.cuda.synchronize()
+    for _ in range(5):
+        graph.replay()
+    torch.cuda.synchronize()
+    for got, ref in zip((x, y, z), want):
+        assert torch.equal(got, ref)
