@@ -291,7 +291,7 @@ WideCfg wide_variant(int v) {
 // is at least 0.9 full are taken, else the ones that fill it best; beyond
 // three loads the last one hardly shows.  The bulk-copy staged kernel's
 // persistent warps take segments in turn, 8 or more each.  Measured against
-// the variants' fixed segments: 5-point 512^2 15.6 -> 10.6 us (from 2048
+// the variants' fixed segments: 5-point 512^2 15.2 -> 10.1 us (from 2048
 // slots, padding dropped), power-law n = 30,000 17.8 -> 8.4 us, 32 FEM blocks
 // of 22M nonzeros in one graph 57.2 -> 54.8 us (staged, from 4096).
 size_t wide_seg(const WideCfg &w, size_t slots) {
@@ -454,7 +454,7 @@ int stage_windows(ispmv_plan_s *p, const std::vector<UIN> &c) {
 // Drops the formats' row padding (AXC bricks, AXT tiles: rows padded to 8
 // slots, or to tileH) from the slot streams: the kernels find rows by their
 // start bits and need none, and every slot costs its 12 bytes and a gather of
-// x[0].  On power-law rows (14.9 nonzeros) tileH = 8 pads 24%: 61.1 -> 54.8
+// x[0].  On power-law rows (14.9 nonzeros) tileH = 8 pads 24%: 61.1 -> 53.2
 // us at n = 1M (beta = 1); on 5-point rows 8 slots hold 5.
 void pack_rows(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v, std::vector<UIN> &c,
                std::vector<size_t> &start) {

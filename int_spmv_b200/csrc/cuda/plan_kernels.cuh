@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(TPB) axc_rows(UIN n, const UIN *__restrict__ b
 // other).  SCATTER writes y[permi] (K1 with integrated reordering), else res
 // in chunk order (then k1_order).  Measured on power-law rows (n = 1M, 14.9M
 // nonzeros, longest row 1,100-3,000, FP64, K1p): 147.7 us with the long
-// chunks on one warp each and the remainders serial, 67.3 us so; the L1's one
+// chunks on one warp each and the remainders serial, 64.0 us so; the L1's one
 // tag lookup per gather and cycle alone takes 52 us.
 constexpr UIN K1_LONG = 64;   // columns from which a chunk gets a warp
 constexpr UIN K1_CTA = 256;   // columns from which a chunk gets a CTA

@@ -9,8 +9,8 @@
 //   - records its first run (head) and last run (tail) - which may continue
 //     into a neighbouring segment - as (row, partial) pairs;
 // and a fix-up kernel then adds each row's partials in segment order and
-// writes y.  No atomics: y is overwritten (beta = 0) or accumulated
-// (beta = 1) deterministically, and every row is written exactly once.
+// writes y.  y is overwritten (beta = 0) or accumulated (beta = 1, by one
+// reduction per row) deterministically: every row is written exactly once.
 #pragma once
 #include "common.cuh"
 

@@ -11,8 +11,8 @@
 //
 // Bound by latency and L1 capacity: of 27 elements a row, U = 9 are loaded
 // and then gathered together (14 or 27 hold more lines than L1 keeps: 60-100
-// us).  27-point stencil, 101^3: FP32 values 44.5 us by the slot stream, 39.6
-// so (28.5 at the copy rate); FP64 values 50.2 (45.0).  At small sizes the
+// us).  27-point stencil, 101^3: FP32 values 44.5 us by the slot stream, 38.2
+// so (28.5 at the copy rate); FP64 values 65.7 and 49.8 (45.0).  At small sizes the
 // two launches saved count: 40^3 8.2 us, 5-point 800^2 9.0.  Slices staged by
 // bulk copies into shared memory take L1 from the gathers and were no faster.
 #pragma once
