@@ -51,13 +51,13 @@ int sm_count();
 // wait.  Both are no-ops for ordinary launches.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// A pointer (or texture handle) to what the awaited grid wrote, for use after
+// A pointer to what the awaited grid wrote, for use after
 // pdl_wait.  The compiler may move loads through a const __restrict__
 // parameter (read-only for the kernel's lifetime, as far as it is told) above
 // the wait; loads through the value returned here depend on this point.
 template <typename T>
 __device__ __forceinline__ T after_wait(T p) {
-  static_assert(sizeof(T) == 8, "a pointer or a texture handle");
+  static_assert(sizeof(T) == 8, "a pointer");
   asm volatile("" : "+l"(p)::"memory");
   return p;
 }

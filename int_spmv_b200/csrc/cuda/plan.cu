@@ -1477,7 +1477,8 @@ template <typename VT, int SPL, int MINB, bool D16 = false, bool TEX = false, bo
 int launch_wide(ispmv_plan_s *p, const FPT *x, seg::Out &o, cudaStream_t s, const char *name) {
   constexpr int NW = STG ? 1 : 0;
   const size_t ctas = (p->nseg + WIDE_WARPS - 1) / WIDE_WARPS;
-  const bool early = STG || ctas <= (size_t)sm_count() * MINB;  // one load of CTAs: stream_wide's DEP form
+  // one load of CTAs: stream_wide's DEP form; never with texture gathers
+  const bool early = STG || (!TEX && ctas <= (size_t)sm_count() * MINB);
   if constexpr (sizeof(VT) == 4 && !STG && !LO) {
     // FP32 values: gather from an FP32 copy of x (the value the FP32 multiply uses)
     if (!p->x32) TRY(dev_alloc(p, p->n, &p->x32));
@@ -1486,7 +1487,7 @@ int launch_wide(ispmv_plan_s *p, const FPT *x, seg::Out &o, cudaStream_t s, cons
     TRY(launch_dependent(p, "x_to_f32", kx, gc, 256, 0, s, true, p->n, x, p->x32));
     const cudaTextureObject_t tx = TEX ? x_texture(p, p->x32, (size_t)p->n * 4, true) : 0;
     if (TEX && !tx) return launch_wide<VT, SPL, MINB, D16, false>(p, x, o, s, "stream_wide<tex: x gathered with loads>");
-    auto *k = early ? wide::stream_wide<VT, float, SPL, 0, WIDE_WARPS, MINB, D16, TEX, false, false, PFC, true>
+    auto *k = early ? wide::stream_wide<VT, float, SPL, 0, WIDE_WARPS, MINB, D16, TEX, false, false, PFC, !TEX>
                     : wide::stream_wide<VT, float, SPL, 0, WIDE_WARPS, MINB, D16, TEX, false, false, PFC, false>;
     return launch_dependent(p, name, k, ctas, WIDE_WARPS * 32, 0, s, early, p->slots, p->slots_pad, p->seg_slots,
                             p->nseg, static_cast<const VT *>(p->val), p->col, p->heads, p->segh, p->xw, p->x32, o,
@@ -1494,7 +1495,7 @@ int launch_wide(ispmv_plan_s *p, const FPT *x, seg::Out &o, cudaStream_t s, cons
   } else {
     const cudaTextureObject_t tx = TEX ? x_texture(p, x, (size_t)p->n * 8, false) : 0;
     if (TEX && !tx) return launch_wide<VT, SPL, MINB, D16, false>(p, x, o, s, "stream_wide<tex: x gathered with loads>");
-    auto *k = early ? wide::stream_wide<VT, double, SPL, NW, WIDE_WARPS, MINB, D16, TEX, STG, LO, PFC, true>
+    auto *k = early ? wide::stream_wide<VT, double, SPL, NW, WIDE_WARPS, MINB, D16, TEX, STG, LO, PFC, !TEX>
                     : wide::stream_wide<VT, double, SPL, NW, WIDE_WARPS, MINB, D16, TEX, STG, LO, PFC, STG>;
     const size_t smem = STG ? (size_t)p->xw.cap * sizeof(double) : 0;
     if (smem) ISPMV_TRY(cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -284,6 +284,9 @@ __device__ __forceinline__ void batch(const VT (&v)[SPL], const XT (&xv)[SPL], u
 // TEX: x is gathered with texture fetches (tex1Dfetch on `xtex`, a linear
 // texture over x) instead of global loads: the texture pipe of L1TEX serves
 // the gathers while the load/store pipe streams values and columns.
+// Texture fetches, like read-only loads, are defined only for what was written
+// before the launch, so this form is never a dependent (DEP): the lines it
+// finds may be those of x (or of x's FP32 copy) before it was written anew.
 // STG: one window per CTA chosen by the plan (xw.tlo/xw.tlen: the densest
 // interval of the CTA's columns), copied into shared memory by one bulk copy
 // (cp.async.bulk, no multicast) on an mbarrier; x must be 16-byte aligned
@@ -309,6 +312,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
   static_assert(!STG || sizeof(XT) == 8, "the window holds FP64 x");
   static_assert(!LO || (sizeof(VT) == 4 && sizeof(XT) == 8), "lo-words correct FP32 values against FP64 x");
   static_assert(DEP || !STG, "the window's copy waits for x");
+  static_assert(!(DEP && TEX), "texture fetches need x written before the launch");
   static_assert(!(PFC && D16), "column prefetch reads u32 columns");
   constexpr int BT = 32 * SPL;
   constexpr unsigned MASK = SPL == 32 ? 0xffffffffu : (1u << SPL) - 1u;
@@ -358,7 +362,6 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
     if (nbat > 0) cnext.get(col, s0, lane);
   }
   const XT *xg = x;
-  cudaTextureObject_t tg = xtex;
   for (int j = 0; j < nbat; j++) {
     const size_t b = s0 + (size_t)j * BT;
     Vals<VT, SPL> v;
@@ -396,7 +399,6 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
         pdl_wait();
         sss::begin_record(o, segid);
         xg = after_wait(x);  // no read-only loads through it: written while this kernel may already run
-        if constexpr (TEX) tg = after_wait(tg);
       }
     }
     if constexpr (STG) {
@@ -418,10 +420,10 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
         xv[k] = gather<NW>(w, sxa, xg, c[k]);
       } else if constexpr (TEX) {
         if constexpr (sizeof(XT) == 8) {
-          const int2 t = tex1Dfetch<int2>(tg, (int)c[k]);
+          const int2 t = tex1Dfetch<int2>(xtex, (int)c[k]);
           xv[k] = __hiloint2double(t.y, t.x);
         } else {
-          xv[k] = tex1Dfetch<float>(tg, (int)c[k]);
+          xv[k] = tex1Dfetch<float>(xtex, (int)c[k]);
         }
       } else if constexpr (DEP) {
         xv[k] = xg[c[k]];

@@ -168,3 +168,44 @@ def test_products_in_a_captured_graph(kw, before):
     torch.cuda.synchronize()
     for got, ref in zip((x, y, z), want):
         assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("kw", [dict(variant=16), dict(variant=16, val="f32"), dict(variant=16, col="d16"),
+                                dict(variant=16, val="f32", col="d16")])
+def test_texture_products_back_to_back(kw):
+    """Texture gathers, product after product with no other kernel between
+    and x, y swapped: every third product reads anew a buffer whose lines an
+    SM may still hold from the product before last."""
+    import numpy as np
+    import torch
+
+    from int_spmv_b200 import device as D
+    from int_spmv_b200 import formats as F
+    from int_spmv_b200 import matrices as M
+    row, col, val = M.random_csr(40_000, 5, rl_max=24, empty_frac=0.05)
+    csr = F.CSR(row, col, val / np.abs(val).max() * 0.1)
+    plan = D.Plan(csr, None, kernel="wide", **kw)
+    x0 = torch.rand(csr.n, dtype=torch.float64, device="cuda")
+
+    def chain(wait):
+        a, b = x0.clone(), torch.ones_like(x0)
+        for _ in range(12):
+            plan.spmv(a, b)
+            if wait:
+                torch.cuda.synchronize()
+            a, b = b, a
+        return a
+
+    alone = chain(True).clone()
+    torch.cuda.synchronize()
+    assert "tex" in plan.kernel_name(), plan.kernel_name()
+    m = torch.randn(2048, 2048, device="cuda")
+    side = torch.cuda.Stream()
+    for i in range(12):
+        if i % 2:
+            with torch.cuda.stream(side):
+                for _ in range(8):
+                    m @ m
+        got = chain(False)
+        torch.cuda.synchronize()
+        assert torch.equal(got, alone)
