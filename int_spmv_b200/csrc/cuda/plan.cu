@@ -203,7 +203,15 @@ int begin(const ispmv_plan_opts *o, ispmv_plan_s **out) {
   return ISPMV_OK;
 }
 
-int done(ispmv_plan_s *p, int st, ispmv_plan *out) {
+// A host builder's copies are waited for here (a small copy from pageable
+// memory may return before it has reached the device): products run on any
+// stream, and read the plan's arrays before they wait for the launches before
+// them.  `waited`: the builder has waited for its own stream.
+int done(ispmv_plan_s *p, int st, ispmv_plan *out, bool waited = false) {
+  if (st == ISPMV_OK && !waited) {
+    const cudaError_t e = cudaStreamSynchronize(nullptr);
+    if (e != cudaSuccess) st = cuda_status(e, "cudaStreamSynchronize");
+  }
   if (st != ISPMV_OK) {
     ispmv_plan_destroy(p);
     return st;
@@ -221,8 +229,7 @@ int empty_rows(ispmv_plan_s *p, const str_matCSR *csr) {
   return ISPMV_OK;
 }
 
-// The work areas of a stream or unit plan, set on `s`; a builder on the
-// default stream waits here (products run on any stream).
+// The work areas of a stream or unit plan, set on `s`.
 int alloc_records(ispmv_plan_s *p, cudaStream_t s = nullptr) {
   const size_t nrec = std::max<size_t>(1, 2 * p->nseg);
   TRY(dev_alloc(p, nrec, &p->rec_row));
@@ -233,7 +240,6 @@ int alloc_records(ispmv_plan_s *p, cudaStream_t s = nullptr) {
   ISPMV_TRY(cudaMemsetAsync(p->rec_row, 0xFF, nrec * sizeof(UIN), s));
   ISPMV_TRY(cudaMemsetAsync(p->status, 0, sizeof(int), s));
   TRY(dev_alloc(p, 1, &p->queue));
-  if (!s) ISPMV_TRY(cudaStreamSynchronize(s));
   return ISPMV_OK;
 }
 
@@ -1132,7 +1138,7 @@ ISPMV_API int ispmv_plan_dev_csr(UIN n, UIN nnz, const UIN *d_row, const UIN *d_
   TRY(begin(o, &p));
   const int st = dev_csr_stream(p, n, nnz, d_row, d_col, d_val, as_stream(stream));
   finish_info(p, "CSR");
-  return done(p, st, out);
+  return done(p, st, out, true);
 }
 
 ISPMV_API int ispmv_plan_get_layout(ispmv_plan p, ispmv_plan_layout *l) {

@@ -209,3 +209,43 @@ def test_texture_products_back_to_back(kw):
         got = chain(False)
         torch.cuda.synchronize()
         assert torch.equal(got, alone)
+
+
+@pytest.mark.parametrize("kind", ["slices", "slices_f32", "K1", "K1P", "rows", "axc_rows", "noc4_ldg", "auto", "f32lo"])
+def test_product_on_another_stream_right_after_the_plan(kind):
+    """A host-built plan's arrays are on the device when the builder returns:
+    a product at once, on a stream the default stream does not order, on blocks
+    that held another matrix's arrays."""
+    import numpy as np
+    import torch
+
+    from int_spmv_b200 import device as D
+    from int_spmv_b200 import formats as F
+    from int_spmv_b200 import matrices as M
+    from oracle import Oracle
+    from paritylib import assert_parity
+    orc = Oracle()
+    mats = []
+    for seed in (1, 2):  # two matrices of the same size
+        row, col, val = M.stencil27(12)
+        val = np.random.default_rng(seed).standard_normal(len(val))
+        x = M.uniform_x(len(row) - 1, seed)
+        csr = F.CSR(row, col, val)
+        z = np.zeros(csr.n)
+        f = F.getFormatDataK1(8, csr, z)[1] if kind.startswith("K1") else \
+            F.getFormatDataAXC(0, csr, z)[1] if kind == "axc_rows" else \
+            F.getFormatDataAXT(0, 128, 8, 4, "NOC", csr, z)[1] if kind == "noc4_ldg" else None
+        mats.append((csr, f, torch.from_numpy(x).cuda(), orc.cf_csr(row, col, val, x), orc.abs_csr(row, col, val, x)))
+    kw = {"slices": dict(col="d16"), "slices_f32": dict(col="d16", val="f32"), "K1": dict(reorder=False),
+          "rows": dict(kernel="rows"), "axc_rows": dict(kernel="rows"), "noc4_ldg": dict(kernel="ldg"),
+          "f32lo": dict(val="f32lo")}.get(kind, {})
+    side = torch.cuda.Stream()
+    y = torch.empty_like(mats[0][2])
+    torch.cuda.synchronize()
+    for i in range(20):
+        csr, f, x, ref, absax = mats[i % 2]
+        plan = D.Plan(csr, f, **kw)
+        plan.spmv(x, y, stream=side)
+        side.synchronize()
+        assert_parity(y.cpu().numpy(), ref, absax, 1e-6 if "f32" in kind else 1e-12, what=f"{kind} {i}")
+        del plan
