@@ -26,8 +26,8 @@ int fail(int status, const char *text);
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 // Device memory from the library's pool (mempool.cu): alloc as cudaMalloc; free
 // keeps the blocks for later requests once no work can use them: `idle` says
-// that the caller has synchronised the stream they were used on, else the
-// device is synchronised.
+// that the caller has synchronised the stream they were used on, else all work
+// on the device is waited for, as cudaFree does.
 int pool_alloc(void **out, size_t bytes);
 void pool_free(void *const *ptrs, size_t count, bool idle);
 // Id of the calling thread's current context; 0 when there is none yet or

@@ -9,9 +9,9 @@
 //     first.  ispmv_pool_trim gives them back on demand, and a failing
 //     cudaMalloc empties the pool and tries again.
 //   - A block is kept only once no work can use it any more: the caller has
-//     synchronised the stream it was used on (idle = true), or the device is
-//     synchronised here, as cudaFree did.  Whatever that returns an error
-//     for (a capture under way, a context that is gone) is left to cudaFree.
+//     synchronised the stream it was used on (idle = true), or all work on the
+//     device is waited for here with a cudaFree, as dropping a plan always did
+//     (wait_for_work).  Where that fails the block itself goes to cudaFree.
 //   - Blocks belong to the context they were allocated in: ones of a context
 //     that was destroyed (cudaDeviceReset) are forgotten.
 //   - One lock; the pool lives until the process ends.
@@ -61,6 +61,7 @@ struct Pool {
   std::vector<Block> kept;                  // oldest first
   size_t kept_bytes = 0;
   std::unordered_map<void *, Block> live;   // blocks handed out
+  std::vector<unsigned long long> anchors;  // contexts that hold wait_for_work's anchor
 };
 Pool &pool() {
   static Pool *p = new Pool();  // never destroyed: plans may outlive static objects
@@ -73,6 +74,29 @@ size_t rounded(size_t n) {
   size_t step = 512;
   while (step * 16 <= n) step *= 2;
   return std::max<size_t>(1, (n + step - 1) / step) * step;
+}
+
+// Waits for all work on the current device, on every stream, by freeing an
+// allocation of no use: cudaFree waits for it.  cudaDeviceSynchronize waits
+// too, but it is prohibited while any stream of the device is being captured
+// and ends that capture, whatever its mode; cudaFree is allowed beside another
+// thread's thread-local or relaxed capture.  `anchors` holds one allocation
+// per context beside it, so that the small pages stay mapped: 10 us for the
+// pair, 700 us where they are mapped and unmapped each time.
+bool wait_for_work(Pool &p) {
+  const unsigned long long ctx = current_ctx_id();
+  void *a = nullptr, *t = nullptr;
+  bool ok = true;
+  {
+    std::lock_guard<std::mutex> g(p.mu);
+    if (std::find(p.anchors.begin(), p.anchors.end(), ctx) == p.anchors.end()) {
+      ok = cudaMalloc(&a, 512) == cudaSuccess;
+      if (ok) p.anchors.push_back(ctx);
+    }
+  }
+  ok = ok && cudaMalloc(&t, 512) == cudaSuccess && cudaFree(t) == cudaSuccess;
+  if (!ok) (void)cudaGetLastError();
+  return ok;
 }
 
 // Frees kept blocks, oldest first, until at most `keep` bytes are kept.
@@ -165,7 +189,7 @@ void pool_free(void *const *ptrs, size_t count, bool idle) {
     bool keep = b.ptr && b.ctx && b.bytes <= POOL_MAX && cur >= 0;
     if (keep && synced != b.dev) {
       keep = (cur == b.dev || cudaSetDevice(b.dev) == cudaSuccess) &&
-             (idle || cudaDeviceSynchronize() == cudaSuccess);
+             (idle || wait_for_work(p));
       ctx = keep ? current_ctx_id() : 0;
       if (keep) synced = b.dev;
       else (void)cudaGetLastError();

@@ -90,3 +90,57 @@ def test_threads(env):
     for t in ts:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("mode", ["thread_local", "relaxed"])
+def test_dropped_beside_a_capture(env, mode):
+    """Plans and GPU-built formats dropped by one thread while another
+    captures a graph: the capture goes on, and its graph runs."""
+    torch, D, _, _ = env
+    (row, col, val, x), ref, absax = make(env, 20_000, 5)
+    plan, y = D.Plan.from_device_csr(row, col, val), torch.empty_like(x)
+    for _ in range(2):  # also the memory the drops need, once
+        drop = [D.Plan.from_device_csr(row, col, val), D.DeviceAXT(row, col, val, x), D.DeviceK1(row, col, val)]
+        plan.spmv(x, y)
+        torch.cuda.synchronize()
+        s, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s, capture_error_mode=mode):
+            plan.spmv(x, y)
+            t = threading.Thread(target=drop.clear)
+            t.start()
+            t.join()
+            y.mul_(2.0)
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert_parity(0.5 * y.cpu().numpy(), ref, absax)
+
+
+def test_graph_products_beside_drops(env):
+    """spmv_graph captures anew for each pair of x and y while another thread
+    builds and drops plans."""
+    torch, D, _, _ = env
+    (row, col, val, x), ref, absax = make(env, 20_000, 6)
+    plan, ys = D.Plan.from_device_csr(row, col, val), [torch.empty_like(x) for _ in range(2)]
+    torch.cuda.synchronize()
+    stop, built = threading.Event(), []
+
+    def churn():
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            while not stop.is_set():
+                D.Plan.from_device_csr(row, col, val)
+                built.append(1)
+
+    t = threading.Thread(target=churn)
+    t.start()
+    try:
+        for i in range(200):
+            plan.spmv_graph(x, ys[i % 2])
+    finally:
+        stop.set()
+        t.join()
+    torch.cuda.synchronize()
+    assert built
+    for y in ys:
+        assert_parity(y.cpu().numpy(), ref, absax)
