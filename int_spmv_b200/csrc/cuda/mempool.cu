@@ -12,8 +12,9 @@
 //     synchronised the stream it was used on (idle = true), or all work on the
 //     device is waited for here with a cudaFree, as dropping a plan always did
 //     (wait_for_work).  Where that fails the block itself goes to cudaFree.
-//   - Blocks belong to the context they were allocated in: ones of a context
-//     that was destroyed (cudaDeviceReset) are forgotten.
+//   - Blocks belong to the context they were allocated in: they are given out
+//     and freed in it alone; those of a context that was destroyed
+//     (cudaDeviceReset) are forgotten.
 //   - One lock; the pool lives until the process ends.
 #include <cuda.h>
 
@@ -29,24 +30,33 @@ namespace {
 
 constexpr size_t POOL_MAX = (size_t)2 << 30;
 
-// cuCtxGetCurrent / cuCtxGetId through the runtime's driver entry points, so
-// the library links no driver library.  Null when unavailable.
+// Driver calls through the runtime's entry points, so the library links no
+// driver library.  Null when unavailable.
 typedef CUresult(CUDAAPI *CtxGetCurrentFn)(CUcontext *);
 typedef CUresult(CUDAAPI *CtxGetIdFn)(CUcontext, unsigned long long *);
+typedef CUresult(CUDAAPI *CtxPushFn)(CUcontext);
+typedef CUresult(CUDAAPI *CtxPopFn)(CUcontext *);
+typedef CUresult(CUDAAPI *PtrGetAttrFn)(void *, CUpointer_attribute, CUdeviceptr);
 CtxGetCurrentFn g_ctx_current = nullptr;
 CtxGetIdFn g_ctx_id = nullptr;
+CtxPushFn g_ctx_push = nullptr;
+CtxPopFn g_ctx_pop = nullptr;
+PtrGetAttrFn g_ptr_attr = nullptr;
 std::once_flag g_ctx_fns_once;
 
-void find_ctx_fns() {
+template <typename F>
+void find_fn(const char *name, F *fn) {
   void *f = nullptr;
   cudaDriverEntryPointQueryResult q;
-  if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
-      q == cudaDriverEntryPointSuccess)
-    g_ctx_current = reinterpret_cast<CtxGetCurrentFn>(f);
-  f = nullptr;
-  if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
-      q == cudaDriverEntryPointSuccess)
-    g_ctx_id = reinterpret_cast<CtxGetIdFn>(f);
+  if (cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+    *fn = reinterpret_cast<F>(f);
+}
+void find_ctx_fns() {
+  find_fn("cuCtxGetCurrent", &g_ctx_current);
+  find_fn("cuCtxGetId", &g_ctx_id);
+  find_fn("cuCtxPushCurrent", &g_ctx_push);
+  find_fn("cuCtxPopCurrent", &g_ctx_pop);
+  find_fn("cuPointerGetAttribute", &g_ptr_attr);
   (void)cudaGetLastError();
 }
 
@@ -99,17 +109,30 @@ bool wait_for_work(Pool &p) {
   return ok;
 }
 
-// Frees kept blocks, oldest first, until at most `keep` bytes are kept.
+// Gives a kept block back, in the context it was allocated in, whatever the
+// calling thread's device and context are.  The driver names the context that
+// owns the address now: another one than the block's, or none, means that the
+// block's context was destroyed and its memory with it.
+void give_back(const Block &b) {
+  CUcontext c = nullptr, popped;
+  unsigned long long id = 0;
+  if (!g_ctx_push || !g_ctx_pop || !g_ptr_attr) {  // no driver entry points: no context to choose
+    if (cudaFree(b.ptr) != cudaSuccess) (void)cudaGetLastError();
+    return;
+  }
+  if (g_ptr_attr(&c, CU_POINTER_ATTRIBUTE_CONTEXT, (CUdeviceptr)(uintptr_t)b.ptr) != CUDA_SUCCESS || !c ||
+      g_ctx_id(c, &id) != CUDA_SUCCESS || id != b.ctx || g_ctx_push(c) != CUDA_SUCCESS)
+    return;
+  if (cudaFree(b.ptr) != cudaSuccess) (void)cudaGetLastError();
+  (void)g_ctx_pop(&popped);
+}
+
+// Gives kept blocks back, oldest first, until at most `keep` bytes are kept.
 void trim_locked(Pool &p, size_t keep) {
   size_t k = 0;
-  const unsigned long long ctx = p.kept_bytes > keep ? current_ctx_id() : 0;
   for (; k < p.kept.size() && p.kept_bytes > keep; k++) {
-    const Block &b = p.kept[k];
-    p.kept_bytes -= b.bytes;
-    int dev = 0;
-    // a block of this device but another context: that context is gone
-    if (cudaGetDevice(&dev) == cudaSuccess && dev == b.dev && ctx != b.ctx) continue;
-    if (cudaFree(b.ptr) != cudaSuccess) (void)cudaGetLastError();
+    p.kept_bytes -= p.kept[k].bytes;
+    give_back(p.kept[k]);
   }
   p.kept.erase(p.kept.begin(), p.kept.begin() + k);
 }

@@ -144,3 +144,37 @@ def test_graph_products_beside_drops(env):
     assert built
     for y in ys:
         assert_parity(y.cpu().numpy(), ref, absax)
+
+
+@pytest.mark.parametrize("where", ["new_thread", "other_context"])
+def test_trim_gives_memory_back(env, where):
+    """ispmv_pool_trim frees what it no longer counts, from a thread that has
+    no context yet and from one whose current context is another one of the
+    device's."""
+    import ctypes as C
+    torch, D, _, _ = env
+    D.trim_pool(0)
+    n = 2_000_000
+    row = torch.arange(0, 8 * n + 1, 8, dtype=torch.int32, device="cuda")
+    col = torch.randint(0, n, (8 * n,), dtype=torch.int32, device="cuda")
+    val = torch.rand(8 * n, dtype=torch.float64, device="cuda")
+    D.Plan.from_device_csr(row, col, val)
+    torch.cuda.synchronize()
+    kept = D.trim_pool(1 << 40)
+    assert kept > 100 << 20
+    before = torch.cuda.mem_get_info()[0]
+    left, cu = [], C.CDLL("libcuda.so.1")
+
+    def trim():
+        ctx = C.c_void_p()
+        if where == "other_context":
+            assert cu.cuCtxCreate_v2(C.byref(ctx), 0, 0) == 0
+        left.append(D.trim_pool(0))
+        if where == "other_context":
+            assert cu.cuCtxDestroy_v2(ctx) == 0
+
+    t = threading.Thread(target=trim)
+    t.start()
+    t.join()
+    assert left == [0]
+    assert torch.cuda.mem_get_info()[0] - before > 0.9 * kept
