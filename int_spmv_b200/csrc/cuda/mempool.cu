@@ -78,11 +78,14 @@ Pool &pool() {
   return *p;
 }
 
-// Requests are rounded up to steps of 1/8 of their power of two (512 bytes
-// at least), so that a matrix of nearly the same size finds the same blocks.
+// Requests are rounded up to steps of 1/8 of their power of two (512 bytes at
+// least, STEP_MAX at most), so that a matrix of nearly the same size finds the
+// same blocks; those too large to be kept are left as they are.
+constexpr size_t STEP_MAX = (size_t)8 << 20;
 size_t rounded(size_t n) {
   size_t step = 512;
-  while (step * 16 <= n) step *= 2;
+  while (step * 16 <= n && step < STEP_MAX) step *= 2;
+  if (n > POOL_MAX) step = 512;
   return std::max<size_t>(1, (n + step - 1) / step) * step;
 }
 

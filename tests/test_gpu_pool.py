@@ -178,3 +178,20 @@ def test_trim_gives_memory_back(env, where):
     t.join()
     assert left == [0]
     assert torch.cuda.mem_get_info()[0] - before > 0.9 * kept
+
+
+def test_large_plan_takes_its_bytes(env):
+    """Blocks of gigabytes are not rounded up by a share of their size: a plan
+    takes the device memory its info names (and work areas, and pages)."""
+    torch, D, _, _ = env
+    n = 37_800_000  # 302.4M nonzeros: 2.42 GB of values, 1.21 GB of columns, both just above a step of 1/8
+    row = torch.arange(0, 8 * n + 1, 8, dtype=torch.int32, device="cuda")
+    col = torch.randint(0, n, (8 * n,), dtype=torch.int32, device="cuda")
+    val = torch.rand(8 * n, dtype=torch.float64, device="cuda")
+    D.trim_pool(0)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    plan = D.Plan.from_device_csr(row, col, val)
+    D.trim_pool(0)
+    used = before - torch.cuda.mem_get_info()[0]
+    assert used <= 1.01 * plan.info["device_bytes"] + (64 << 20), (used, plan.info["device_bytes"])
