@@ -49,6 +49,7 @@ struct ispmv_plan_s {
   size_t slots = 0, slots_pad = 0, nunits = 0;
   bool no_win = false;  // staged variants: empty x windows
   bool chosen = false;  // kernel and variant by AUTO
+  bool long_rows = false;  // stream and unit plans: a row of more than seg::FIX_LONG segments (seg::fixup's form)
   uint2 *slices = nullptr;  // P_SLICES: first element column and base column of each slice, and the end
   uint8_t *slen = nullptr;  // P_SLICES: row lengths
   UIN slice_w = 0;          // P_SLICES: the widest slice
@@ -220,10 +221,14 @@ int done(ispmv_plan_s *p, int st, ispmv_plan *out, bool waited = false) {
   return ISPMV_OK;
 }
 
+// The list of empty rows, and whether a row spans many segments.
 int empty_rows(ispmv_plan_s *p, const str_matCSR *csr) {
   std::vector<UIN> e;
-  for (UIN r = 0; r < csr->nrows; r++)
-    if (csr->row[r + 1] == csr->row[r]) e.push_back(r);
+  for (UIN r = 0; r < csr->nrows; r++) {
+    const UIN l = csr->row[r + 1] - csr->row[r];
+    if (!l) e.push_back(r);
+    if (l > seg::FIX_LONG * p->seg_slots) p->long_rows = true;
+  }
   p->nempty = e.size();
   if (!e.empty()) TRY(dev_upload(p, e.data(), e.size(), &p->empty));
   return ISPMV_OK;
@@ -829,17 +834,20 @@ __global__ void dcsr_check_rows(UIN n, UIN nnz, const UIN *__restrict__ row, UIN
 // Row-start bits, the compressed -> real map and the empty-row list from the
 // prefix `pos` of the non-empty flags; and segh[g] = row starts at slots
 // below g*seg = pos[first r with row[r] >= g*seg], written by that r's thread
-// (n's, past the last row).
+// (n's, past the last row); *long_rows = 1 for a row of more than
+// seg::FIX_LONG segments.
 __global__ void dcsr_rows(UIN n, const UIN *__restrict__ row, const UIN *__restrict__ pos, UIN *__restrict__ heads,
                           UIN *__restrict__ rowmap, UIN *__restrict__ empty, size_t nseg, UIN seg,
-                          UIN *__restrict__ segh) {
+                          UIN *__restrict__ segh, int *__restrict__ long_rows) {
   const size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r > n) return;
   const UIN a = row[r], q = pos[r];
   const size_t g1 = r == n ? nseg : min((size_t)(a / seg) + 1, nseg);
   for (size_t g = r == 0 ? 0 : (size_t)(row[r - 1] / seg) + 1; g < g1; g++) segh[g] = q;
   if (r == n) return;
-  if (row[r + 1] > a) {
+  const UIN e = row[r + 1];
+  if (e > a) {
+    if (e - a > seg::FIX_LONG * seg) *long_rows = 1;
     atomicOr(&heads[a >> 5], 1u << (a & 31u));
     if (rowmap) rowmap[q] = (UIN)r;
   } else if (empty) {
@@ -1014,7 +1022,7 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
   struct Found {
     unsigned long long far;
     UIN nonempty;
-    int bad;
+    int bad, long_rows;
   } *found, hf{};
   DevTmp tmp(s);
   p->n = n;
@@ -1095,7 +1103,8 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
   }
   TRY(check_launch("dcsr_interleave"));
   dcsr_rows<<<(unsigned)(((size_t)n + 1 + 255) / 256), 256, 0, s>>>(n, row, pos, p->heads, p->rowmap, p->empty,
-                                                                      p->nseg, (UIN)p->seg_slots, p->segh);
+                                                                      p->nseg, (UIN)p->seg_slots, p->segh,
+                                                                      &found->long_rows);
   TRY(check_launch("dcsr_rows"));
   size_t nt = 0;
   if (wc.stg) {
@@ -1121,9 +1130,10 @@ int dev_csr_stream(ispmv_plan_s *p, UIN n, UIN nnz, const UIN *row, const UIN *c
   }
   TRY(alloc_records(p, s));
   if (wc.stg) p->xw.status = p->status;
-  ISPMV_TRY(cudaMemcpyAsync(&hf.bad, bad, sizeof hf.bad, cudaMemcpyDeviceToHost, s));
+  ISPMV_TRY(cudaMemcpyAsync(&hf, found, sizeof hf, cudaMemcpyDeviceToHost, s));
   ISPMV_TRY(cudaStreamSynchronize(s));
   if (hf.bad) return fail(ISPMV_ERR_ARG, malformed);
+  p->long_rows = hf.long_rows != 0;
   p->info.device_bytes = (uint64_t)(8 * nt) + (uint64_t)p->slots_pad * (vbytes(p) + 4) + p->slots_pad / 8;
   return ISPMV_OK;
 }
@@ -1714,7 +1724,7 @@ int run(ispmv_plan_s *p, const FPT *x, FPT *y, int beta, cudaStream_t s) {
       cfg.stream = s;
       cfg.attrs = at;
       cfg.numAttrs = pdl ? 1 : 0;
-      ISPMV_TRY(cudaLaunchKernelEx(&cfg, seg::fixup, nrec, (const UIN *)p->rec_row, (const double *)p->rec_sum,
+      ISPMV_TRY(cudaLaunchKernelEx(&cfg, p->long_rows ? seg::fixup<true> : seg::fixup<false>, nrec, (const UIN *)p->rec_row, (const double *)p->rec_sum,
                                    (const UIN *)p->rowmap, (const UIN *)p->empty, p->nempty, y, beta));
       return check_launch("fixup");
     }

@@ -103,8 +103,18 @@ __device__ __forceinline__ void finish(const State &st, const Out &o, size_t seg
 // overlaps the main kernel's last CTAs: griddepcontrol.wait then blocks until
 // the main kernel has completed and its records and rows are visible (it
 // returns at once for an ordinary launch).
-__global__ void fixup(size_t nrec, const UIN *rec_row_, const double *rec_sum_, const UIN *__restrict__ rowmap,
-                      const UIN *__restrict__ empty, size_t nempty, FPT *y_, int beta) {
+// LONG (a plan with a row of more than FIX_LONG segments): a thread walks
+// FIX_WALK records back by itself, and the rest of a longer row's are added by
+// its warp, 32 * FIX_U at a time, in an order that depends on the records
+// alone.  One row of 1M nonzeros among 10,000 short ones (2,000 segments):
+// 492.7 us a product with the records added one by one, 17.5 so.  Without
+// such a row the warp's part only costs: 52.0 -> 52.4 us (power-law n = 1M).
+constexpr size_t FIX_LONG = 8;
+constexpr int FIX_WALK = 16, FIX_U = 8;
+template <bool LONG>
+__global__ void __launch_bounds__(256) fixup(size_t nrec, const UIN *rec_row_, const double *rec_sum_,
+                                             const UIN *__restrict__ rowmap, const UIN *__restrict__ empty,
+                                             size_t nempty, FPT *y_, int beta) {
   pdl_trigger();  // the next product's main kernel may launch; it waits for this grid
   pdl_wait();
   const UIN *rec_row = after_wait(rec_row_);
@@ -112,18 +122,57 @@ __global__ void fixup(size_t nrec, const UIN *rec_row_, const double *rec_sum_, 
   FPT *y = after_wait(y_);
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < nempty && !beta) y[empty[i]] = 0.0;
-  if (i >= nrec) return;
-  const UIN r = rec_row[i];
-  if (r == NO_ROW) return;
-  size_t j = i + 1;
-  while (j < nrec && rec_row[j] == NO_ROW) j++;
-  if (j < nrec && rec_row[j] == r) return;
-  double total = rec_sum[i];
-  for (size_t k = i; k-- > 0;) {
-    const UIN rk = rec_row[k];
-    if (rk == NO_ROW) continue;
-    if (rk != r) break;
-    total += rec_sum[k];
+  UIN r = i < nrec ? rec_row[i] : NO_ROW;
+  if (!LONG && r == NO_ROW) return;
+  if (r != NO_ROW) {
+    size_t j = i + 1;
+    while (j < nrec && rec_row[j] == NO_ROW) j++;
+    if (j < nrec && rec_row[j] == r) r = NO_ROW;  // not the row's last record
+  }
+  if (!LONG && r == NO_ROW) return;
+  double total = 0.0;
+  size_t k = i;       // records [0, k) are left
+  bool more = false;  // and some of them may be the row's
+  if (r != NO_ROW) {
+    total = rec_sum[i];
+    more = true;
+    for (int t = 0; more && (!LONG || t < FIX_WALK); t++) {
+      more = false;
+      if (!k) break;
+      const UIN rk = rec_row[--k];
+      more = rk == NO_ROW || rk == r;
+      if (rk == r) total += rec_sum[k];
+    }
+  }
+  if constexpr (LONG) {
+    const unsigned lane = threadIdx.x & 31u;
+    for (unsigned need = __ballot_sync(FULL, more); need; need &= need - 1) {
+      const int src = __ffs(need) - 1;
+      const UIN rs = __shfl_sync(FULL, r, src);
+      unsigned long long e = __shfl_sync(FULL, (unsigned long long)k, src);
+      double part = 0.0;
+      for (bool go = true; go && e;) {
+        UIN rk[FIX_U];
+        double v[FIX_U];
+#pragma unroll
+        for (int u = 0; u < FIX_U; u++) {
+          const unsigned long long d = 32u * u + lane + 1u;  // record e - d
+          rk[u] = d <= e ? rec_row[e - d] : NO_ROW;
+          v[u] = d <= e ? rec_sum[e - d] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < FIX_U; u++) {
+          const unsigned other = __ballot_sync(FULL, rk[u] != rs && rk[u] != NO_ROW);
+          if (go && rk[u] == rs && lane < (other ? (unsigned)__ffs(other) - 1u : 32u)) part += v[u];
+          if (other) go = false;
+        }
+        e = e > 32u * FIX_U ? e - 32u * FIX_U : 0;
+      }
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(FULL, part, d);
+      if ((int)lane == src) total += part;
+    }
+    if (r == NO_ROW) return;
   }
   const UIN rr = rowmap ? rowmap[r] : r;
   y[rr] = beta ? total + y[rr] : total;

@@ -217,3 +217,50 @@ def test_slices_of_rows(env, val_kind, n, w, span):
         assert torch.equal(plan.spmv_graph(x, y), a)
     with pytest.raises(Exception):
         plan.spmm(torch.zeros((n, 8), dtype=torch.float64, device="cuda"))
+
+
+@pytest.mark.parametrize("kw", [{}, dict(val="f32"), dict(kernel="wide", variant=0), dict(kernel="ldg")])
+@pytest.mark.parametrize("segs", [1, 7, 8, 9, 16, 17, 60, 128, 129, 137])
+def test_rows_over_many_segments(env, kw, segs):
+    """Rows of more records than one thread adds up, next to short and empty
+    rows and to one another: the records before and after the row are others',
+    none, or a whole pass of the warp's."""
+    _, D, F, _ = env
+    n, k = 80_000, 512 * segs
+    lengths = np.zeros(n, int)
+    lengths[100:3000] = 3
+    lengths[[0, 1, 50, 3000, 3002, n - 1]] = [k, k + 1, k - 1, k + 255, k, k]
+    row = np.zeros(n + 1, np.uint32)
+    row[1:] = np.cumsum(lengths)
+    j = np.arange(int(row[-1])) - np.repeat(row[:-1], lengths)
+    col = (np.repeat((np.arange(n) * 7) % (n - lengths.max()), lengths) + j).astype(np.uint32)
+    val = np.random.default_rng(segs).standard_normal(len(col))
+    check(env, row, col, val, D.Plan(F.CSR(row, col, val), None, **kw), kw.get("val", "f64"))
+
+
+def test_one_very_long_row(env):
+    """A matrix with one row of a million nonzeros takes a few times what as
+    many in short rows take, not what adding its records one by one does."""
+    torch, D, _, _ = env
+    def us(lengths):
+        n = len(lengths)
+        row = torch.zeros(n + 1, dtype=torch.int32, device="cuda")
+        row[1:] = torch.from_numpy(lengths).cuda().cumsum(0)
+        nnz = int(row[-1])
+        col = torch.randint(0, n, (nnz,), dtype=torch.int32, device="cuda")
+        plan = D.Plan.from_device_csr(row, col, torch.rand(nnz, dtype=torch.float64, device="cuda"))
+        x = torch.rand(n, dtype=torch.float64, device="cuda")
+        y, best = torch.empty_like(x), 1e9
+        for _ in range(6):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            for _ in range(20):
+                plan.spmv(x, y)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 50)
+        return best
+
+    short = us(np.full(70_000, 15))
+    one = us(np.concatenate([np.full(5_000, 5), [1_000_000], np.full(5_000, 5)]))
+    assert one < 6 * short, (one, short)
