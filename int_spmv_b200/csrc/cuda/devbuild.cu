@@ -13,8 +13,9 @@
 // Padding is zero.  The arrays are bit-identical to the host builder's.
 //
 // Steps: row slot counts -> exclusive prefix (three scan kernels over u64;
-// COM: the row pointer is the prefix) -> sizes read back to the host (one synchronisation, to allocate) ->
-// a CTA per 256 rows writes their slots.
+// COM: the row pointer is the prefix), con and the row of every chunk of slots
+// -> sizes read back to the host (one synchronisation, to allocate) -> a CTA
+// per chunk writes its slots.
 //
 // The K1 arrays of getFormatDataK1 (M:841-905) likewise: rows sorted by
 // length, descending, equal lengths in ascending row order (the order of the
@@ -49,15 +50,43 @@ __global__ void row_slots(UIN n, const UIN *__restrict__ row, UIN grp, int noc, 
   cnt[r] = noc ? (l + grp - 1) / grp * grp : l;
 }
 
+// Slot s's value position in ax.  lenAX < 2^32 (checked before the fill),
+// so slots and positions fit in 32 bits.
+__device__ __forceinline__ UIN axt_pos(UIN s, UIN th) {
+  if (th == 1) return (s >> 3) * 16 + (s & 7u);
+  const UIN ths = 8 * th, T = s / ths, w = s - T * ths;
+  return T * 2 * ths + (w % th) * 16 + w / th;
+}
+
+// A fill CTA takes `chunk` slots; row_of[g] = the row that holds the first slot
+// of chunk g (of the first `cap` ones).
+struct Chunks {
+  UIN chunk, cap;
+  UIN *row_of;
+};
+// Row r, slots [s0, s1): its con, and the chunks whose first slot it holds.
+__device__ __forceinline__ void place_row(UIN r, uint64_t s0, uint64_t s1, UIN th, UIN *__restrict__ con, Chunks c) {
+  if (s1 > 0xFFFFFFFFull) return;  // more slots than the arrays can hold: refused after this pass
+  con[r] = axt_pos((UIN)s0, th);
+  if (s0 == s1) return;
+  for (UIN g = (UIN)(s1 - 1) / c.chunk;; g--) {  // the last chunk that starts before s1, downwards
+    if ((uint64_t)g * c.chunk < s0) return;
+    if (g < c.cap) c.row_of[g] = r;
+    if (!g) return;
+  }
+}
+
 // COM mode's slots are the CSR's own (row[r] - row[0]): no prefix, only this
 // check.  found = {row[0], row[n], 1 if the row pointer decreases}.
-__global__ void check_rows(UIN n, const UIN *__restrict__ row, UIN *__restrict__ found) {
+__global__ void check_rows(UIN n, const UIN *__restrict__ row, UIN *__restrict__ found, UIN *__restrict__ con,
+                           Chunks c) {
   const size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
-  const UIN a = row[r], e = row[r + 1];
-  if (e < a) found[2] = 1;
+  const UIN a = row[r], e = row[r + 1], first = row[0];
   if (r == 0) found[0] = a;
   if (r == n - 1) found[1] = e;
+  if (e < a || a < first) found[2] = 1;
+  else place_row((UIN)r, a - first, e - first, 1, con, c);
 }
 
 // Exclusive prefix of one block's SB items; bsum[b] = the block's total.
@@ -140,50 +169,47 @@ __global__ void add_block_offsets(size_t len, uint64_t *__restrict__ out, const 
   if (i < len) out[i] += bsum[i / SB];
 }
 
-// Slot s's value position in ax.  lenAX < 2^32 (checked before the fill),
-// so slots and positions fit in 32 bits.
-__device__ __forceinline__ UIN axt_pos(UIN s, UIN th) {
-  if (th == 1) return (s >> 3) * 16 + (s & 7u);
-  const UIN ths = 8 * th, T = s / ths, w = s - T * ths;
-  return T * 2 * ths + (w % th) * 16 + w / th;
+// The same for an AXT in NOC mode, and what follows from a row's slots.
+__global__ void axt_rows(UIN n, const uint64_t *__restrict__ cnt, uint64_t *__restrict__ off,
+                         const uint64_t *__restrict__ bsum, UIN th, UIN *__restrict__ con, Chunks c) {
+  const size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r > n) return;
+  const uint64_t s0 = off[r] + bsum[r / SB];
+  off[r] = s0;
+  if (r < n) place_row((UIN)r, s0, s0 + cnt[r], th, con, c);
 }
 
-// A CTA per FILL_ROWS rows: con, and every word of ax and sec of the rows'
-// slots, padding included, written once (no memset before).  The CTA's row
-// starts sit in shared memory; each thread finds the row of its slot there (8
-// steps), so neighbouring threads read and write neighbouring slots whatever
-// the rows' lengths.  Bound by the bytes it moves: at power-law n = 1M,
-// 14.9M nonzeros, one warp per row after two memsets took 270 us and 60, this
-// takes 124 (477 MB, 74 us at the copy rate; x is gathered).  A last CTA, past the rows, fills the last tile.
+// Every word of ax and sec, padding included, written once (no memset before).
+// A CTA per `chunk` slots, whatever rows they belong to: it starts at the row
+// that holds its first slot, takes FILL_ROWS rows' starts into shared memory at
+// a time, and each thread finds the row of its slot there (8 steps), so
+// neighbouring threads read and write neighbouring slots whatever the rows'
+// lengths.  (A CTA per 256 rows left 2000 rows of 5000 nonzeros to 8 CTAs:
+// 2,500 us, 81 so.)
+// Bound by the bytes it moves: a conversion at power-law n = 1M, 14.9M nonzeros
+// (477 MB, 74 us at the copy rate; x is gathered) took 330 us with one warp per
+// row after two memsets, 140 with a CTA per 256 rows, 120 so.
 // TILES (th > 1): slots in ax order (tile, sub-row, column), so that the
-// writes are contiguous; only the CTA's own slots of its first and last tile.
+// writes are contiguous; only the rows' own slots of their first and last tile.
+// 6 CTAs per SM there (40 registers) and 5 elsewhere: left to the compiler the
+// NOC forms take 5-10% longer.
 constexpr int FILL_ROWS = 256;
-constexpr UIN TILES_MAX_TH = 64;  // taller tiles span several CTAs' rows: slot order
+constexpr uint64_t FILL_SLOTS = 2048, FILL_SMALL = 1024;
+constexpr UIN TILES_MAX_TH = 64;  // taller tiles span several CTAs: slot order
 template <bool COM, bool TILES>
-__global__ void __launch_bounds__(256) fill_axt(UIN n, const UIN *__restrict__ row, const UIN *__restrict__ col,
+__global__ void __launch_bounds__(256, TILES ? 6 : 5) fill_axt(UIN n, const UIN *__restrict__ row, const UIN *__restrict__ col,
                                                 const FPT *__restrict__ val, const FPT *__restrict__ x,
-                                                const uint64_t *__restrict__ off, UIN slots, UIN th, UIN bs, UIN lg,
-                                                UIN *__restrict__ con, FPT *__restrict__ ax, UIN *__restrict__ sec) {
+                                                const uint64_t *__restrict__ off, UIN slots, Chunks ch, UIN th, UIN bs,
+                                                UIN lg, FPT *__restrict__ ax, UIN *__restrict__ sec) {
   __shared__ UIN soff[FILL_ROWS], srow[FILL_ROWS], slen[FILL_ROWS], send;
+  bool search = blockIdx.x >= ch.cap;  // the row of slot a is not known
+  UIN r0 = search ? 0 : ch.row_of[blockIdx.x];  // the first of the rows in shared memory
   const UIN first = off ? 0 : row[0];
   auto start = [&](size_t r) { return off ? (UIN)off[r] : row[r] - first; };  // COM: no prefix needed
-  const UIN total = start(n);
-  const size_t r0 = (size_t)blockIdx.x * FILL_ROWS;
-  const bool tail = r0 >= n;  // the slots past the last row's
-  {
-    const size_t r = r0 + threadIdx.x;
-    soff[threadIdx.x] = 0xFFFFFFFFu;
-    if (r < n) {
-      const UIN s0 = start(r), j0 = row[r];
-      soff[threadIdx.x] = s0;
-      srow[threadIdx.x] = j0;
-      slen[threadIdx.x] = row[r + 1] - j0;
-      con[r] = axt_pos(s0, th);
-    }
-    if (threadIdx.x == 0) send = tail ? slots : start(min(r0 + FILL_ROWS, (size_t)n));
-  }
-  __syncthreads();
-  const UIN a = tail ? total : soff[0], e = send, ths = 8 * th;
+  const UIN total = start(n), ths = 8 * th;
+  const UIN c0 = blockIdx.x * ch.chunk, c1 = ch.chunk < slots - c0 ? c0 + ch.chunk : slots;
+  const UIN e_rows = min(c1, total);  // slots [c0, e_rows) are rows', the rest padding
+  UIN a = c0, e = 0;                  // slots of the rows in shared memory
   // a slot past the last row: zeros
   auto pad = [&](UIN s, UIN p) {
     ax[p] = (FPT)0;
@@ -221,7 +247,7 @@ __global__ void __launch_bounds__(256) fill_axt(UIN n, const UIN *__restrict__ r
       if (!on[i]) continue;
       ax[p[i]] = v[i];
       ax[p[i] + 8] = xv[i];
-      const UIN r = (UIN)r0 + q[i];
+      const UIN r = r0 + q[i];
       if (COM) {
         UIN d = 0;
         if (k[i] == 0 || (s[i] & (bs - 1)) == 0) {
@@ -236,32 +262,59 @@ __global__ void __launch_bounds__(256) fill_axt(UIN n, const UIN *__restrict__ r
       }
     }
   };
-  // item i of the CTA: a slot, or (TILES) a place in ax order
-  const uint64_t i0 = TILES ? (uint64_t)(a / ths) * ths : a;
-  const uint64_t i1 = TILES ? ((uint64_t)e + ths - 1) / ths * ths : e;
-  auto place = [&](uint64_t i, UIN &s, UIN &p) {
+  // item i of slots [a, e): a slot, or (TILES) a place in ax order
+  auto place = [&](UIN i, UIN i1, UIN &s, UIN &p) {
     if (TILES) {
-      const UIN T = (UIN)(i / ths), w = (UIN)i - T * ths, R = w >> 3, C = w & 7u;
+      const UIN T = i / ths, w = i - T * ths, R = w >> 3, C = w & 7u;
       s = T * ths + C * th + R;
       p = T * 2 * ths + R * 16 + C;
       return i < i1 && s >= a && s < e;
     }
-    s = (UIN)i;
+    s = i;
     p = axt_pos(s, th);
     return i < i1;
   };
-  for (uint64_t i = i0 + threadIdx.x; i < i1; i += 256 * U) {
-    UIN s[U], p[U];
-    bool on[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) on[u] = place(i + 256 * u, s[u], p[u]);
-    if (tail) {
-#pragma unroll
-      for (int u = 0; u < U; u++)
-        if (on[u]) pad(s[u], p[u]);
+  for (; a < c1; a = e) {
+    const bool pad_now = a >= e_rows;
+    if (pad_now) {
+      e = c1;
     } else {
-      slots_of(s, p, on);
+      if (search)  // the last row at or after r0 that starts at or before slot a
+        for (UIN hi = n; hi - r0 > 1;) {
+          const UIN step = (hi - r0 - 1) / 256 + 1;
+          const size_t r = r0 + (size_t)(threadIdx.x + 1) * step;
+          r0 += step * (UIN)__syncthreads_count(r < hi && start(r) <= a);
+          hi = hi - r0 > step ? r0 + step : hi;
+        }
+      __syncthreads();  // the rows before these are done with
+      const size_t r = (size_t)r0 + threadIdx.x;
+      soff[threadIdx.x] = 0xFFFFFFFFu;
+      if (r < n) {
+        const UIN j0 = row[r];
+        soff[threadIdx.x] = start(r);
+        srow[threadIdx.x] = j0;
+        slen[threadIdx.x] = row[r + 1] - j0;
+      }
+      if (threadIdx.x == 0) send = start(min((size_t)r0 + FILL_ROWS, (size_t)n));
+      __syncthreads();
+      e = min(send, e_rows);
+      search = e == a;  // nothing but empty rows: there may be many more
     }
+    const UIN i0 = TILES ? a / ths * ths : a, i1 = TILES ? (e + ths - 1) / ths * ths : e;  // below 2^31
+    for (UIN i = i0 + threadIdx.x; i < i1; i += 256 * U) {
+      UIN s[U], p[U];
+      bool on[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) on[u] = place(i + 256 * u, i1, s[u], p[u]);
+      if (pad_now) {
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (on[u]) pad(s[u], p[u]);
+      } else {
+        slots_of(s, p, on);
+      }
+    }
+    r0 += FILL_ROWS;
   }
 }
 
@@ -364,6 +417,7 @@ ISPMV_API int ispmv_dev_build_axt(UIN bs, UIN thw, UIN th, const char *mode, UIN
   const size_t len = (size_t)n + 1, nb = (len + SB - 1) / SB;
   const UIN grp = th == 1 ? thw : th;
   uint64_t slots = 0;
+  Chunks ch{0, 0, nullptr};
 #define DB_TRY(expr)                              \
   do {                                            \
     cudaError_t e__ = (expr);                     \
@@ -378,12 +432,26 @@ ISPMV_API int ispmv_dev_build_axt(UIN bs, UIN thw, UIN th, const char *mode, UIN
   } while (0)
   DB_TRY(cudaEventCreate(&e0));
   DB_TRY(cudaEventCreate(&e1));
+  {
+    // whole tiles of slots per CTA, one round of its threads where that is one
+    // load of CTAs (30,000 rows of 15: 26 us, 28.5 with two rounds), else two
+    // (power-law n = 1M: 120 us, 131 with one); as many chunks as the rows'
+    // slots can make
+    const uint64_t tile = th > 1 && th <= TILES_MAX_TH ? (uint64_t)8 * th : 8;
+    const uint64_t most = std::min<uint64_t>((uint64_t)nnz + (com ? 0 : (uint64_t)n * (grp - 1)), 1ull << 31);
+    const uint64_t per = most <= FILL_SMALL * 5 * (uint64_t)sm_count() ? FILL_SMALL : FILL_SLOTS;
+    ch.chunk = (UIN)((per + tile - 1) / tile * tile);
+    ch.cap = (UIN)((most + ch.chunk - 1) / ch.chunk);
+  }
+  DB_ALLOC(m->con, (size_t)n * sizeof(UIN));
+  DB_ALLOC(ch.row_of, std::max<size_t>(1, ch.cap) * sizeof(UIN));
   if (com) {
     UIN found[3] = {0, 0, 0};
     DB_ALLOC(bsum, sizeof found);
     DB_TRY(cudaEventRecord(e0, s));
     DB_TRY(cudaMemsetAsync(bsum, 0, sizeof found, s));
-    check_rows<<<(unsigned)(((size_t)n + 255) / 256), 256, 0, s>>>(n, d_row, reinterpret_cast<UIN *>(bsum));
+    check_rows<<<(unsigned)(((size_t)n + 255) / 256), 256, 0, s>>>(n, d_row, reinterpret_cast<UIN *>(bsum),
+                                                             m->con, ch);
     if ((st = check_launch("check_rows"))) goto done;
     DB_TRY(cudaMemcpyAsync(found, bsum, sizeof found, cudaMemcpyDeviceToHost, s));
     DB_TRY(cudaStreamSynchronize(s));
@@ -403,8 +471,8 @@ ISPMV_API int ispmv_dev_build_axt(UIN bs, UIN thw, UIN th, const char *mode, UIN
     if ((st = check_launch("scan_block"))) goto done;
     scan_totals<<<1, ST, 0, s>>>(nb, bsum);
     if ((st = check_launch("scan_totals"))) goto done;
-    add_block_offsets<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(len, off, bsum);
-    if ((st = check_launch("add_block_offsets"))) goto done;
+    axt_rows<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(n, cnt, off, bsum, th, m->con, ch);
+    if ((st = check_launch("axt_rows"))) goto done;
     DB_TRY(cudaMemcpyAsync(&slots, off + n, sizeof slots, cudaMemcpyDeviceToHost, s));
     DB_TRY(cudaStreamSynchronize(s));
   }
@@ -428,13 +496,13 @@ ISPMV_API int ispmv_dev_build_axt(UIN bs, UIN thw, UIN th, const char *mode, UIN
     m->tileN = (UIN)tiles;
     m->lenAX = (UIN)lenAX;
     m->lenSEC = (UIN)lenSEC;
-    DB_ALLOC(m->con, std::max<size_t>(1, n) * sizeof(UIN));
     DB_ALLOC(m->ax, std::max<uint64_t>(1, lenAX) * sizeof(FPT));
     DB_ALLOC(m->sec, std::max<uint64_t>(1, lenSEC) * sizeof(UIN));
-    const unsigned g = (unsigned)(((size_t)n + FILL_ROWS - 1) / FILL_ROWS + 1);
+    const size_t slots_all = lenAX / 2;
+    const unsigned g = (unsigned)((slots_all + ch.chunk - 1) / ch.chunk);
     auto *k = com ? fill_axt<true, false>
                   : th > 1 && th <= TILES_MAX_TH ? fill_axt<false, true> : fill_axt<false, false>;
-    k<<<g, 256, 0, s>>>(n, d_row, d_col, d_val, d_x, off, (UIN)(lenAX / 2), th, bs, lg, m->con, m->ax, m->sec);
+    if (g) k<<<g, 256, 0, s>>>(n, d_row, d_col, d_val, d_x, off, (UIN)slots_all, ch, th, bs, lg, m->ax, m->sec);
     if ((st = check_launch("fill_axt"))) goto done;
     DB_TRY(cudaEventRecord(e1, s));
     DB_TRY(cudaEventSynchronize(e1));
@@ -453,7 +521,7 @@ ISPMV_API int ispmv_dev_build_axt(UIN bs, UIN thw, UIN th, const char *mode, UIN
 #undef DB_TRY
 #undef DB_ALLOC
 done:
-  free_scratch({cnt, off, bsum}, s);
+  free_scratch({cnt, off, bsum, ch.row_of}, s);
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   if (st != ISPMV_OK) ispmv_dev_axt_free(m);

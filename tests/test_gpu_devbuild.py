@@ -90,6 +90,74 @@ def test_device_axt_many_rows():
         check_build(row, col, val, x, mode, th, bs, run_kernel=False)
 
 
+@pytest.mark.parametrize("mode,th,bs", SHAPES + [("NOC", 3, 128), ("NOC", 64, 128), ("NOC", 65, 128), ("NOC", 200, 128)])
+@pytest.mark.parametrize("kind", ["long", "edges", "gaps", "none", "many"])
+def test_device_axt_rows_and_chunks(mode, th, bs, kind):
+    """Rows over many CTAs' slots, rows that end just before, at and after the
+    end of a CTA's slots, long runs of empty rows inside them, no slots at all,
+    and enough slots for the longer chunks."""
+    rng = np.random.default_rng(len(kind))
+    if kind == "long":
+        rl = np.r_[[0, 9001, 5, 20000, 0, 0, 1], np.full(70, 300)]
+    elif kind == "edges":
+        rl = np.r_[[1024, 1023, 1, 1025, 2047, 1, 2048, 0, 2049, 1, 511, 512, 513], np.full(600, 5), [2048, 0]]
+    elif kind == "gaps":
+        rl = np.zeros(300_000, int)
+        rl[[3, 4, 260, 70_000, 70_300, 299_999]] = [7, 600, 3, 40, 1, 12]
+    elif kind == "none":
+        rl = np.zeros(1000, int)
+    else:
+        rl = rng.integers(0, 24, 150_000)
+        rl[1000] = 30_000
+    n = len(rl) if len(rl) > 30_000 else 30_000
+    rl = np.r_[rl, np.zeros(n - len(rl), int)]
+    row = np.concatenate([[0], np.cumsum(rl)]).astype(np.uint32)
+    j = np.arange(int(row[-1])) - np.repeat(row[:-1], rl)
+    col = ((np.repeat(np.arange(n) * 13 % (n - rl.max()) if rl.max() < n else np.zeros(n, int), rl)) + j).astype(np.uint32)
+    check_build(row, col, rng.standard_normal(len(col)), rng.uniform(-1, 1, n), mode, th, bs, run_kernel=False)
+
+
+@pytest.mark.parametrize("mode,th", [("COM", 1), ("NOC", 1), ("NOC", 4)])
+def test_device_axt_counts_from_the_row_pointer(mode, th):
+    """The slots come from the row pointer: a smaller nnz argument (it only
+    names itself in the result) changes no array."""
+    import ctypes as C
+
+    import torch
+
+    from int_spmv_b200 import device as D
+    from int_spmv_b200 import matrices as M
+    row, col, val = M.random_csr(20_011, 3, rl_max=60, empty_frac=0.1)
+    t = [_dev(a) for a in (row, col, val, M.uniform_x(20_011, 3))]
+    a = D.DeviceAXT(*t, th=th, mode=mode)
+    b = D.DeviceAXT.__new__(D.DeviceAXT)
+    b.c, b.fd = D.abi.StrMatAXT(), D.abi.StrFormatData()
+    p = [x.data_ptr() for x in t]
+    assert D.load().ispmv_dev_build_axt(128, 8, th, mode.encode(), 20_011, 1, *p, C.byref(b.c), C.byref(b.fd), 0) == 0
+    torch.cuda.synchronize()
+    ha, hb = a.to_host(), b.to_host()
+    assert all(np.array_equal(ha[k].view(np.uint32), hb[k].view(np.uint32)) for k in ha)
+
+
+def test_device_axt_time_of_long_rows():
+    """Ten million nonzeros in 2000 rows convert in about the time they take
+    in a million rows."""
+    import torch
+
+    from int_spmv_b200 import device as D
+
+    def us(n, k):
+        row = torch.arange(0, n * k + 1, k, dtype=torch.int32, device="cuda")
+        col = torch.randint(0, n, (n * k,), dtype=torch.int32, device="cuda")
+        val = torch.rand(n * k, dtype=torch.float64, device="cuda")
+        x = torch.rand(n, dtype=torch.float64, device="cuda")
+        return [min(D.DeviceAXT(row, col, val, x, th=th, mode=m).conversion_s for _ in range(6))
+                for m, th in (("COM", 1), ("NOC", 1), ("NOC", 8))]
+
+    for long, short in zip(us(2_000, 5_000), us(1_000_000, 10)):
+        assert long < 2 * short, (long, short)
+
+
 def check_build_k1(row, col, val, x):
     import torch
 
