@@ -24,7 +24,9 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include <cub/device/device_scan.cuh>
@@ -80,7 +82,6 @@ struct ispmv_plan_s {
   size_t xtex_bytes = 0;
   uint32_t *tblocks = nullptr;       // the stream in TMEM-staged blocks (stream_tmem variants)
   unsigned long long *queue = nullptr;  // work-queue counter (variant ISPMV_VARIANT_QUEUE)
-  cudaStream_t cap_stream = nullptr;    // private stream for graph capture
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   const FPT *g_x = nullptr;
@@ -765,7 +766,6 @@ ISPMV_API int ispmv_plan_destroy(ispmv_plan p) {
   if (p->xtex) cudaDestroyTextureObject(p->xtex);
   if (p->graph_exec) cudaGraphExecDestroy(p->graph_exec);
   if (p->graph) cudaGraphDestroy(p->graph);
-  if (p->cap_stream) cudaStreamDestroy(p->cap_stream);
   pool_free(p->owned.data(), p->owned.size(), false);
   delete p;
   return ISPMV_OK;
@@ -1801,6 +1801,53 @@ ISPMV_API int ispmv_plan_spmv(ispmv_plan p, const FPT *x, FPT *y, int beta, void
   return run<float>(p, x, y, beta, s);
 }
 
+// Streams to capture graph products on, kept between captures: a stream made
+// for a plan and destroyed with it took 65-100 us of the plan's first graph
+// product, and the driver then keeps less for the graphs (50,000 FEM rows, a
+// new plan's first graph product 330 -> 113 us, a new x on the same plan 148 ->
+// 36).  A capture has its stream for itself; those of other contexts are left
+// alone.
+namespace {
+struct CaptureStream {
+  static constexpr size_t MOST = 4;  // kept
+  struct Idle {
+    std::mutex mu;
+    std::vector<std::pair<unsigned long long, cudaStream_t>> v;  // context, stream
+  };
+  static Idle &idle() {
+    static Idle *i = new Idle();  // never destroyed: plans may outlive static objects
+    return *i;
+  }
+  cudaStream_t s = nullptr;
+  int open() {
+    const unsigned long long ctx = current_ctx_id();
+    {
+      std::lock_guard<std::mutex> g(idle().mu);
+      auto &v = idle().v;
+      for (size_t i = 0; i < v.size() && !s; i++)
+        if (ctx && v[i].first == ctx) {
+          s = v[i].second;
+          v.erase(v.begin() + i);
+        }
+    }
+    if (!s) ISPMV_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    return ISPMV_OK;
+  }
+  ~CaptureStream() {
+    if (!s) return;
+    const unsigned long long ctx = current_ctx_id();
+    {
+      std::lock_guard<std::mutex> g(idle().mu);
+      if (ctx && idle().v.size() < MOST) {
+        idle().v.emplace_back(ctx, s);
+        return;
+      }
+    }
+    cudaStreamDestroy(s);
+  }
+};
+}  // namespace
+
 ISPMV_API int ispmv_plan_spmv_graph(ispmv_plan p, const FPT *x, FPT *y, int beta, void *stream) {
   if (!p || !x || !y || (beta != 0 && beta != 1)) return ISPMV_ERR_ARG;
   if (!p->graph_exec || p->g_x != x || p->g_y != y || p->g_beta != beta) {
@@ -1808,19 +1855,20 @@ ISPMV_API int ispmv_plan_spmv_graph(ispmv_plan p, const FPT *x, FPT *y, int beta
     if (p->graph) cudaGraphDestroy(p->graph);
     p->graph_exec = nullptr;
     p->graph = nullptr;
-    if (!p->cap_stream) ISPMV_TRY(cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking));
+    CaptureStream cap;
+    TRY(cap.open());
     // work areas a product allocates on first use, allocated before the
     // capture (no allocation may happen inside it): the FP32 copy of x of
     // FP32-value plans on the lane-interleaved kernel
     if (p->opts.val_kind != ISPMV_VAL_F64 && p->opts.kernel == ISPMV_KERNEL_WIDE && p->path == P_STREAM && !p->x32)
       TRY(dev_alloc(p, p->n, &p->x32));
-    ISPMV_TRY(cudaStreamBeginCapture(p->cap_stream, cudaStreamCaptureModeThreadLocal));
+    ISPMV_TRY(cudaStreamBeginCapture(cap.s, cudaStreamCaptureModeThreadLocal));
     p->capturing = true;
-    const int st = p->opts.val_kind == ISPMV_VAL_F64 ? run<double>(p, x, y, beta, p->cap_stream)
-                                                     : run<float>(p, x, y, beta, p->cap_stream);
+    const int st = p->opts.val_kind == ISPMV_VAL_F64 ? run<double>(p, x, y, beta, cap.s)
+                                                     : run<float>(p, x, y, beta, cap.s);
     p->capturing = false;
     cudaGraph_t g = nullptr;
-    const cudaError_t e = cudaStreamEndCapture(p->cap_stream, &g);
+    const cudaError_t e = cudaStreamEndCapture(cap.s, &g);
     if (st || e != cudaSuccess) {
       if (g) cudaGraphDestroy(g);
       // a failed capture leaves its error as the runtime's last error: clear

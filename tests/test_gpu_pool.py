@@ -195,3 +195,31 @@ def test_large_plan_takes_its_bytes(env):
     D.trim_pool(0)
     used = before - torch.cuda.mem_get_info()[0]
     assert used <= 1.01 * plan.info["device_bytes"] + (64 << 20), (used, plan.info["device_bytes"])
+
+
+def test_graph_products_in_threads(env):
+    """Graph products of new plans captured by four threads at once, the plans
+    dropped and others captured on the streams they left."""
+    torch, D, _, _ = env
+    mats = [make(env, 8_000 + 13 * t, 20 + t) for t in range(4)]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(t):
+        (row, col, val, x), ref, absax = mats[t]
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            for i in range(25):
+                plan, y = D.Plan.from_device_csr(row, col, val, val_kind="f32" if i % 3 == 1 else "f64"), torch.empty_like(x)
+                for _ in range(2):
+                    plan.spmv_graph(x, y)
+                s.synchronize()
+                if np.any(np.abs(y.cpu().numpy() - ref) > (1e-6 if i % 3 == 1 else 1e-12) * absax):
+                    wrong.append((t, i))
+
+    ts = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not wrong
