@@ -253,8 +253,11 @@ __global__ void k1_order(UIN n, const UIN *__restrict__ permi, const FPT *res_, 
 // step the warp loads 4 consecutive sub-rows of a tile (32 consecutive
 // slots), adds them per column, and after th/4 steps reduces the 4 partials
 // of each column with 2 shuffles; 4 tiles make a batch of 32 columns.
+// Bound by its gathers' latency: 6 CTAs per SM (40 registers); at the 48 the
+// compiler takes otherwise 5 fit, and power-law n = 4M takes 413.6 us for 360.1
+// (tileH 4; tileH 8 394.3 for 347.5; n = 1M 129 for 133).
 template <typename VT>
-__global__ void __launch_bounds__(TPB) noc_hn(size_t nunits, size_t nseg, UIN th, UIN useg, const UIN *__restrict__ urow,
+__global__ void __launch_bounds__(TPB, 6) noc_hn(size_t nunits, size_t nseg, UIN th, UIN useg, const UIN *__restrict__ urow,
                                               const UIN *__restrict__ col, const VT *__restrict__ val,
                                               const FPT *__restrict__ x, seg::Out o) {
   pdl_trigger();
