@@ -513,7 +513,8 @@ int ispmv_plan_kernel_ms(ispmv_plan p, double *total_ms, int *launches);
  * event pair, without the row fix-up or K1's reorder; *ms = the mean per
  * launch.  Synchronises `stream`.  y is left without the fix-up's rows: an
  * ispmv_plan_spmv gives the product.  Unlike an event pair around each
- * launch, the timing holds no event record between consecutive launches. */
+ * launch, the timing holds no event record between consecutive launches; each
+ * starts when the one before it has ended (products themselves may overlap). */
 int ispmv_plan_time_main(ispmv_plan p, const FPT *x, FPT *y, int reps, void *stream, double *ms);
 /* Name of the main kernel the plan's latest product launched (a static
  * string, "" before the first product), e.g. "stream_ldg<4,0,5>". */

@@ -49,6 +49,7 @@ struct ispmv_plan_s {
   ispmv_plan_opts opts{};
   UIN n = 0, nnz = 0, th = 1, bs = 0, lanes = 8;
   size_t slots = 0, slots_pad = 0, nunits = 0;
+  bool alone = false;   // ispmv_plan_time_main: launches wait for one another
   bool no_win = false;  // staged variants: empty x windows
   bool chosen = false;  // kernel and variant by AUTO
   bool long_rows = false;  // stream and unit plans: a row of more than seg::FIX_LONG segments (seg::fixup's form)
@@ -1433,12 +1434,17 @@ int launch_staged_w(K kernel, size_t smem, size_t nseg, int ctas_per_sm, cudaStr
   return check_launch(what);
 }
 
+// Whether a product's first kernel may start while the launch before the
+// product finishes: not where a timing event sits between them, nor where the
+// kernel is timed by itself.
+bool overlaps(const ispmv_plan_s *p) { return !p->alone && (!p->tcap || p->capturing); }
+
 // A launch; `early`: it may start while the launches before it in the stream
 // finish (its kernel waits for them before it touches anything but the plan's
-// constant arrays), unless a timing event sits between.
+// constant arrays).
 template <typename... KA, typename... A>
-int launch_dependent(const ispmv_plan_s *p, const char *name, void (*k)(KA...), size_t grid, unsigned block,
-                     size_t smem, cudaStream_t s, bool early, A... a) {
+int launch_dependent(const char *name, void (*k)(KA...), size_t grid, unsigned block, size_t smem, cudaStream_t s,
+                     bool early, A... a) {
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -1448,7 +1454,7 @@ int launch_dependent(const ispmv_plan_s *p, const char *name, void (*k)(KA...), 
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = at;
-  cfg.numAttrs = early && (!p->tcap || p->capturing) ? 1 : 0;
+  cfg.numAttrs = early ? 1 : 0;
   ISPMV_TRY(cudaLaunchKernelEx(&cfg, k, static_cast<KA>(a)...));
   return check_launch(name);
 }
@@ -1500,14 +1506,13 @@ int launch_wide(ispmv_plan_s *p, const FPT *x, seg::Out &o, cudaStream_t s, cons
     if (!p->x32) TRY(dev_alloc(p, p->n, &p->x32));
     const unsigned gc = (unsigned)std::min<size_t>(((size_t)p->n / 2 + 255) / 256, (size_t)sm_count() * 8) + 1;
     auto *kx = (reinterpret_cast<uintptr_t>(x) & 15u) == 0 ? wide::x_to_f32<true> : wide::x_to_f32<false>;
-    TRY(launch_dependent(p, "x_to_f32", kx, gc, 256, 0, s, true, p->n, x, p->x32));
+    TRY(launch_dependent("x_to_f32", kx, gc, 256, 0, s, overlaps(p), p->n, x, p->x32));
     const cudaTextureObject_t tx = TEX ? x_texture(p, p->x32, (size_t)p->n * 4, true) : 0;
     if (TEX && !tx) return launch_wide<VT, SPL, MINB, D16, false>(p, x, o, s, "stream_wide<tex: x gathered with loads>");
     auto *k = early ? wide::stream_wide<VT, float, SPL, 0, WIDE_WARPS, MINB, D16, TEX, false, false, PFC, !TEX>
                     : wide::stream_wide<VT, float, SPL, 0, WIDE_WARPS, MINB, D16, TEX, false, false, PFC, false>;
-    return launch_dependent(p, name, k, ctas, WIDE_WARPS * 32, 0, s, early, p->slots, p->slots_pad, p->seg_slots,
-                            p->nseg, static_cast<const VT *>(p->val), p->col, p->heads, p->segh, p->xw, p->x32, o,
-                            p->narrow, tx);
+    return launch_dependent(name, k, ctas, WIDE_WARPS * 32, 0, s, early, p->slots, p->slots_pad, p->seg_slots, p->nseg,
+                            static_cast<const VT *>(p->val), p->col, p->heads, p->segh, p->xw, p->x32, o, p->narrow, tx);
   } else {
     const cudaTextureObject_t tx = TEX ? x_texture(p, x, (size_t)p->n * 8, false) : 0;
     if (TEX && !tx) return launch_wide<VT, SPL, MINB, D16, false>(p, x, o, s, "stream_wide<tex: x gathered with loads>");
@@ -1515,8 +1520,9 @@ int launch_wide(ispmv_plan_s *p, const FPT *x, seg::Out &o, cudaStream_t s, cons
                     : wide::stream_wide<VT, double, SPL, NW, WIDE_WARPS, MINB, D16, TEX, STG, LO, PFC, STG>;
     const size_t smem = STG ? (size_t)p->xw.cap * sizeof(double) : 0;
     if (smem) ISPMV_TRY(cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return launch_dependent(p, name, k, ctas, WIDE_WARPS * 32, smem, s, early, p->slots, p->slots_pad, p->seg_slots, p->nseg, static_cast<const VT *>(p->val), p->col, p->heads,
-                            p->segh, p->xw, x, o, p->narrow, tx);
+    return launch_dependent(name, k, ctas, WIDE_WARPS * 32, smem, s, early && overlaps(p), p->slots, p->slots_pad,
+                            p->seg_slots, p->nseg, static_cast<const VT *>(p->val), p->col, p->heads, p->segh, p->xw, x,
+                            o, p->narrow, tx);
   }
 }
 
@@ -1705,9 +1711,9 @@ int run(ispmv_plan_s *p, const FPT *x, FPT *y, int beta, cudaStream_t s) {
   const int st = run_main<VT>(p, x, y, beta, s);
   if (st) return st;
   p->kname = last_launch();
-  // the kernels after the main one (the row fix-up, K1's reorder)
-  // the kernel after the main one is a programmatic dependent launch when
-  // nothing (a timing event) sits between the two in the stream
+  // the kernel after the main one (the row fix-up, K1's reorder) is a
+  // programmatic dependent launch when nothing (a timing event) sits between
+  // the two in the stream
   const bool pdl = !p->tcap || p->capturing;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1770,16 +1776,16 @@ int run_main(ispmv_plan_s *p, const FPT *x, FPT *y, int beta, cudaStream_t s) {
     case P_SLICES: {
       const UIN ns = (p->n + 31) / 32;
       auto *k = p->slice_w <= 5 ? sl::slice_rows<VT, 5> : sl::slice_rows<VT, 9>;
-      return launch_dependent(p, "stream_wide<rows32,d16>", k, (ns + pk::TPB / 32 - 1) / (pk::TPB / 32), pk::TPB, 0, s,
-                              true, p->n, ns, p->slices, p->slen, p->narrow.col16, val, x, y, beta);
+      return launch_dependent("stream_wide<rows32,d16>", k, (ns + pk::TPB / 32 - 1) / (pk::TPB / 32), pk::TPB, 0, s,
+                              overlaps(p), p->n, ns, p->slices, p->slen, p->narrow.col16, val, x, y, beta);
     }
     case P_K1: {
       const unsigned g = (unsigned)pk::k1_ctas(p->chunkNum, p->k1_cta, p->k1_long);
       if (p->fmt == F_K1P)
-        return launch_dependent(p, "k1_chunks<scatter>", pk::k1_chunks<VT, true>, g, pk::TPB, 0, s, true, p->n, p->chunkNum,
-                                p->k1_cta, p->k1_long, p->chp, p->nmc, p->permi, p->col, val, x, y, beta);
-      return launch_dependent(p, "k1_chunks", pk::k1_chunks<VT, false>, g, pk::TPB, 0, s, true, p->n, p->chunkNum, p->k1_cta,
-                              p->k1_long, p->chp, p->nmc, p->permi, p->col, val, x, p->res, beta);
+        return launch_dependent("k1_chunks<scatter>", pk::k1_chunks<VT, true>, g, pk::TPB, 0, s, overlaps(p), p->n,
+                                p->chunkNum, p->k1_cta, p->k1_long, p->chp, p->nmc, p->permi, p->col, val, x, y, beta);
+      return launch_dependent("k1_chunks", pk::k1_chunks<VT, false>, g, pk::TPB, 0, s, overlaps(p), p->n, p->chunkNum,
+                              p->k1_cta, p->k1_long, p->chp, p->nmc, p->permi, p->col, val, x, p->res, beta);
     }
     case P_STREAM:
     case P_UNITS: {
@@ -1926,8 +1932,10 @@ ISPMV_API int ispmv_plan_time_main(ispmv_plan p, const FPT *x, FPT *y, int reps,
   ISPMV_TRY(cudaEventCreate(&e[0]));
   int st = ck(cudaEventCreate(&e[1]), "cudaEventCreate");
   if (!st) st = ck(cudaEventRecord(e[0], s), "cudaEventRecord");
+  p->alone = true;
   for (int i = 0; i < reps && !st; i++)
     st = p->opts.val_kind == ISPMV_VAL_F64 ? run_main<double>(p, x, y, 0, s) : run_main<float>(p, x, y, 0, s);
+  p->alone = false;
   if (!st) st = ck(cudaEventRecord(e[1], s), "cudaEventRecord");
   if (!st) st = ck(cudaEventSynchronize(e[1]), "cudaEventSynchronize");
   float t = 0.f;
@@ -2004,7 +2012,7 @@ int spmm_blocks(ispmv_plan_s *p, UIN k, const FPT *X, FPT *Y, cudaStream_t s, co
     mm::stream_spmm<G, W, T, MINB, VEC, VT><<<(unsigned)ctas, 256, 0, s>>>(st, part, nparts, X, o);
     TRY(check_launch(name));
     p->kname = last_launch();
-    TRY(launch_dependent(p, "spmm_fixup", mm::spmm_fixup<CB>, (std::max(nrec, p->nempty) * CB + 255) / 256, 256, 0, s,
+    TRY(launch_dependent("spmm_fixup", mm::spmm_fixup<CB>, (std::max(nrec, p->nempty) * CB + 255) / 256, 256, 0, s,
                          true, nrec, p->empty, p->nempty, o));
   }
   return ISPMV_OK;
