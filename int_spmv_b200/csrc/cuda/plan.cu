@@ -467,20 +467,35 @@ int stage_windows(ispmv_plan_s *p, const std::vector<UIN> &c) {
 // Drops the formats' row padding (AXC bricks, AXT tiles: rows padded to 8
 // slots, or to tileH) from the slot streams: the kernels find rows by their
 // start bits and need none, and every slot costs its 12 bytes and a gather of
-// x[0].  On power-law rows (14.9 nonzeros) tileH = 8 pads 24%: 61.1 -> 53.2
-// us at n = 1M (beta = 1); on 5-point rows 8 slots hold 5.
+// x[0].  On power-law rows (14.9 nonzeros) tileH = 8 pads 24%, on 5-point rows
+// 8 slots hold 5.  Leaves the stream as it is where the format is not the CSR's
+// (row pointer decreasing, rows past the format's slots, or values outside the
+// CSR's rows): the format's own slots are multiplied then.
 void pack_rows(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v, std::vector<UIN> &c,
                std::vector<size_t> &start) {
+  const long long n = csr->nrows;
+  bool fits = true;
+  long long values = 0;
+#pragma omp parallel for schedule(static) reduction(&& : fits)
+  for (long long r = 0; r < n; r++)
+    fits = fits && csr->row[r + 1] >= csr->row[r] &&
+           (csr->row[r + 1] == csr->row[r] || start[r] + (csr->row[r + 1] - csr->row[r]) <= v.size());
+  if (!fits) return;
   std::vector<double> pv(csr->nnz);
   std::vector<UIN> pc(csr->nnz);
-#pragma omp parallel for schedule(static)
-  for (long long r = 0; r < (long long)csr->nrows; r++) {
+#pragma omp parallel for schedule(static) reduction(- : values)
+  for (long long r = 0; r < n; r++) {
     const UIN a = csr->row[r], l = csr->row[r + 1] - a;
     if (!l) continue;  // a row without slots: start[r] names no slot of its own
     std::copy_n(v.begin() + start[r], l, pv.begin() + a);
     std::copy_n(c.begin() + start[r], l, pc.begin() + a);
-    start[r] = a;
+    for (UIN k = 0; k < l; k++) values -= pv[a + k] != 0.0;
   }
+#pragma omp parallel for schedule(static) reduction(+ : values)
+  for (long long q = 0; q < (long long)v.size(); q++) values += v[q] != 0.0;
+  if (values) return;
+  for (long long r = 0; r < n; r++)
+    if (csr->row[r + 1] > csr->row[r]) start[r] = csr->row[r];
   v.swap(pv);
   c.swap(pc);
   p->slots = csr->nnz;
@@ -490,8 +505,12 @@ void pack_rows(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v, s
 // rows of a slice are nearly equally long (at most 8% padding: the bytes it
 // adds are then less than the kernel saves) and short (a row is one lane's
 // work: at most 48 elements), and every slice's columns span less than 65536.
-// v, c: the rows back to back.  Returns false where a slice does not fit.
-bool slice_fit(const ispmv_plan_s *p, const str_matCSR *csr, const std::vector<UIN> &c, std::vector<uint2> &meta) {
+// v, c: the slot stream; it fits only with the CSR's rows back to back.
+// Returns false where a slice does not fit.
+bool slice_fit(const ispmv_plan_s *p, const str_matCSR *csr, const std::vector<UIN> &c,
+               const std::vector<size_t> &start, std::vector<uint2> &meta) {
+  for (UIN r = 0; r < p->n; r++)
+    if (csr->row[r + 1] < csr->row[r] || (csr->row[r + 1] > csr->row[r] && start[r] != csr->row[r])) return false;
   const UIN ns = (p->n + 31) / 32;
   meta.assign((size_t)ns + 1, uint2{0, 0});
   uint64_t cols = 0;
@@ -550,9 +569,9 @@ int setup_stream(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v,
   p->fslots = p->slots;
   if (p->slots != csr->nnz) pack_rows(p, csr, v, c, start);
   if (p->chosen && p->opts.col_kind == ISPMV_COL_D16 && p->opts.val_kind != ISPMV_VAL_F32_LO16 &&
-      p->opts.units_per_warp <= 0 && p->slots) {
+      p->opts.units_per_warp <= 0 && p->slots && p->slots == csr->nnz) {
     std::vector<uint2> meta;
-    if (slice_fit(p, csr, c, meta)) return setup_slices(p, csr, v, c, meta);
+    if (slice_fit(p, csr, c, start, meta)) return setup_slices(p, csr, v, c, meta);
   }
   p->slots_pad = std::max(SS, (p->slots + SS - 1) / SS * SS);
   if (p->opts.kernel == ISPMV_KERNEL_WIDE && wide_variant(p->opts.variant).tmem) {

@@ -264,3 +264,23 @@ def test_one_very_long_row(env):
     short = us(np.full(70_000, 15))
     one = us(np.concatenate([np.full(5_000, 5), [1_000_000], np.full(5_000, 5)]))
     assert one < 6 * short, (one, short)
+
+
+@pytest.mark.parametrize("fmt", ["AXC", "NOC1", "NOC4"])
+@pytest.mark.parametrize("last", [1, 2, 3, 4, 300])
+def test_format_of_another_matrix(env, fmt, last):
+    """A plan multiplies what its format holds, also where the CSR beside it
+    has rows of other lengths (its last row shorter or longer here)."""
+    torch, D, F, orc = env
+    n = 300
+    row, col, val = rows_of(np.full(n, 3), n, 1)
+    made = F.CSR(row, col, val)
+    lengths = np.full(n, 3)
+    lengths[-1] = last
+    given = F.CSR(*rows_of(lengths, n, 2))
+    f = F.getFormatDataAXC(0, made, np.zeros(n))[1] if fmt == "AXC" else \
+        F.getFormatDataAXT(0, 128, 8, int(fmt[3:]), "NOC", made, np.zeros(n))[1]
+    x = np.random.default_rng(3).uniform(-1, 1, n)
+    for kw in (dict(kernel="wide", variant=4), dict(kernel="wide", variant=4, col="d16"), dict(col="d16"), {}):
+        y = D.Plan(given, f, **kw).spmv(torch.from_numpy(x).cuda()).cpu().numpy()
+        assert_parity(y, orc.cf_csr(row, col, val, x), orc.abs_csr(row, col, val, x), TOL_F64, what=str(kw))

@@ -164,3 +164,43 @@ def test_time_main_rejects_bad_arguments_before_any_device_call():
     assert lib.ispmv_plan_time_main(p, p, nul, 1, None, C.byref(ms)) == 1
     assert lib.ispmv_plan_time_main(p, p, p, 0, None, C.byref(ms)) == 1
     assert lib.ispmv_plan_time_main(p, p, p, 1, None, None) == 1
+
+
+MISMATCHED = """
+import ctypes as C, sys
+import numpy as np
+from int_spmv_b200 import device as D, formats as F
+from int_spmv_b200._lib import load
+from int_spmv_b200 import abi
+n = 64
+def csr(lengths):
+    row = np.zeros(n + 1, np.uint32); row[1:] = np.cumsum(lengths)
+    return F.CSR(row, np.arange(int(row[-1]), dtype=np.uint32) % n, np.ones(int(row[-1])))
+made = csr([3] * n)
+kind = sys.argv[1]
+if kind == "decreasing":
+    given = csr([3] * n)
+    given.row[10], given.row[11] = given.row[11], given.row[10]
+else:  # another matrix of as many rows
+    given = csr([3] * (n - 1) + [4000])
+f = F.getFormatDataAXC(0, made, np.zeros(n))[1] if sys.argv[2] == "AXC" else \
+    F.getFormatDataAXT(0, 128, 8, int(sys.argv[2]), "NOC", made, np.zeros(n))[1]
+try:
+    D.Plan(given, f, kernel="wide", variant=4, col=sys.argv[3])
+except Exception as e:
+    print(type(e).__name__)
+"""
+
+
+@pytest.mark.parametrize("col", ["u32", "d16"])
+@pytest.mark.parametrize("fmt", ["AXC", "1", "4"])
+@pytest.mark.parametrize("kind", ["decreasing", "other"])
+def test_plan_of_a_format_that_is_not_the_csrs(kind, fmt, col):
+    """A CSR whose row pointer decreases, or whose rows are longer than the
+    format's, never makes a plan read past the format's arrays on the host
+    (run as a process of its own)."""
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable, "-c", MISMATCHED, kind, fmt, col], capture_output=True, text=True,
+                       env=dict(__import__("os").environ, PYTHONPATH=str(ROOT)), timeout=300)
+    assert r.returncode == 0, (r.returncode, r.stderr[-500:])
