@@ -2024,6 +2024,8 @@ int spmm_blocks(ispmv_plan_s *p, UIN k, const FPT *X, FPT *Y, cudaStream_t s, co
     p->mm_cap = (nparts + nrec) * CB;
   }
   const unsigned spl = il_spl(p);
+  if (spl != 0 && spl != 8 && spl != 16)
+    return fail(ISPMV_ERR_UNSUPPORTED, "ispmv_plan_spmm: lane-interleaved plans of 8 or 16 slots per lane");
   const mm::Stream st{p->slots, p->slots_pad, p->seg_slots, p->val, p->col, p->heads, p->segh,
                       spl == 16 ? 4u : spl == 8 ? 3u : 0u};
   for (UIN j0 = 0; j0 < k; j0 += CB) {
