@@ -39,7 +39,8 @@ constexpr int ST = 1024;        // threads per scan block
 constexpr int SI = 4;           // items per thread
 constexpr int SB = ST * SI;     // items per scan block
 
-__global__ void row_slots(UIN n, const UIN *__restrict__ row, UIN grp, int noc, uint64_t *__restrict__ cnt) {
+// NOC mode: a row's slots, padded to whole groups.
+__global__ void row_slots(UIN n, const UIN *__restrict__ row, UIN grp, uint64_t *__restrict__ cnt) {
   const size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r > n) return;
   if (r == n) {
@@ -47,7 +48,7 @@ __global__ void row_slots(UIN n, const UIN *__restrict__ row, UIN grp, int noc, 
     return;
   }
   const uint64_t l = row[r + 1] - row[r];
-  cnt[r] = noc ? (l + grp - 1) / grp * grp : l;
+  cnt[r] = (l + grp - 1) / grp * grp;
 }
 
 // Slot s's value position in ax.  lenAX < 2^32 (checked before the fill),
@@ -465,7 +466,7 @@ ISPMV_API int ispmv_dev_build_axt(UIN bs, UIN thw, UIN th, const char *mode, UIN
     DB_ALLOC(off, len * sizeof(uint64_t));
     DB_ALLOC(bsum, nb * sizeof(uint64_t));
     DB_TRY(cudaEventRecord(e0, s));
-    row_slots<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(n, d_row, grp, noc, cnt);
+    row_slots<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(n, d_row, grp, cnt);
     if ((st = check_launch("row_slots"))) goto done;
     scan_block<<<(unsigned)nb, ST, 0, s>>>(len, cnt, off, bsum);
     if ((st = check_launch("scan_block"))) goto done;

@@ -159,29 +159,26 @@ struct Bands {
 // others.
 template <int NW>
 __device__ __forceinline__ double gather(const Bands<NW> &w, uint32_t sx_addr, const FPT *x, UIN c) {
-  if constexpr (NW == 0) {
-    return x[c];
-  } else {
-    uint32_t in = 0, off = 0;
+  static_assert(NW > 0, "without a window x is loaded in place");
+  uint32_t in = 0, off = 0;
 #pragma unroll
-    for (int k = 0; k < NW; k++) {
-      if (c - w.lo[k] < w.len[k]) {  // window starts lie in [0, n]: the unsigned difference is exact
-        in = 1;
-        off = c + w.delta[k];
-      }
+  for (int k = 0; k < NW; k++) {
+    if (c - w.lo[k] < w.len[k]) {  // window starts lie in [0, n]: the unsigned difference is exact
+      in = 1;
+      off = c + w.delta[k];
     }
-    double v;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.u32 p, %3, 0;\n"
-        "@p ld.shared.f64 %0, [%1];\n"
-        "@!p ld.global.f64 %0, [%2];\n"
-        "}\n"
-        : "=d"(v)
-        : "r"(sx_addr + 8u * off), "l"(x + c), "r"(in));
-    return v;
   }
+  double v;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.u32 p, %3, 0;\n"
+      "@p ld.shared.f64 %0, [%1];\n"
+      "@!p ld.global.f64 %0, [%2];\n"
+      "}\n"
+      : "=d"(v)
+      : "r"(sx_addr + 8u * off), "l"(x + c), "r"(in));
+  return v;
 }
 
 // One batch of 32*SPL slots: lane l holds the values v[k] and gathered x
@@ -287,8 +284,8 @@ __device__ __forceinline__ void batch(const VT (&v)[SPL], const XT (&xv)[SPL], u
 // Texture fetches, like read-only loads, are defined only for what was written
 // before the launch, so this form is never a dependent (DEP): the lines it
 // finds may be those of x (or of x's FP32 copy) before it was written anew.
-// STG: one window per CTA chosen by the plan (xw.tlo/xw.tlen: the densest
-// interval of the CTA's columns), copied into shared memory by one bulk copy
+// STG: one window per CTA chosen by the plan (xw.tlo/xw.tlen: columns that
+// hold many of the CTA's, by counting), copied into shared memory by one bulk copy
 // (cp.async.bulk, no multicast) on an mbarrier; x must be 16-byte aligned
 // (the host checks).  The copy leaves the L1 load pipe to the gathers and
 // costs no load loop.  Each warp waits for it (bounded) only before its
