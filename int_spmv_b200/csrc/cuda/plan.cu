@@ -1795,7 +1795,7 @@ int run_main(ispmv_plan_s *p, const FPT *x, FPT *y, int beta, cudaStream_t s) {
     case P_SLICES: {
       const UIN ns = (p->n + 31) / 32;
       auto *k = p->slice_w <= 5 ? sl::slice_rows<VT, 5> : sl::slice_rows<VT, 9>;
-      return launch_dependent("stream_wide<rows32,d16>", k, (ns + pk::TPB / 32 - 1) / (pk::TPB / 32), pk::TPB, 0, s,
+      return launch_dependent("slice_rows<rows32,d16>", k, (ns + pk::TPB / 32 - 1) / (pk::TPB / 32), pk::TPB, 0, s,
                               overlaps(p), p->n, ns, p->slices, p->slen, p->narrow.col16, val, x, y, beta);
     }
     case P_K1: {

@@ -227,7 +227,7 @@ def test_product_on_another_stream_right_after_the_plan(kind):
     orc = Oracle()
     mats = []
     for seed in (1, 2):  # two matrices of the same size
-        row, col, val = M.stencil27(12)
+        row, col, val = M.stencil27(30 if kind.startswith("slices") else 12)
         val = np.random.default_rng(seed).standard_normal(len(val))
         x = M.uniform_x(len(row) - 1, seed)
         csr = F.CSR(row, col, val)
@@ -248,4 +248,5 @@ def test_product_on_another_stream_right_after_the_plan(kind):
         plan.spmv(x, y, stream=side)
         side.synchronize()
         assert_parity(y.cpu().numpy(), ref, absax, 1e-6 if "f32" in kind else 1e-12, what=f"{kind} {i}")
+        assert ("rows32" in plan.kernel_name()) == kind.startswith("slices")
         del plan

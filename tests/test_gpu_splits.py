@@ -284,3 +284,13 @@ def test_format_of_another_matrix(env, fmt, last):
     for kw in (dict(kernel="wide", variant=4), dict(kernel="wide", variant=4, col="d16"), dict(col="d16"), {}):
         y = D.Plan(given, f, **kw).spmv(torch.from_numpy(x).cuda()).cpu().numpy()
         assert_parity(y, orc.cf_csr(row, col, val, x), orc.abs_csr(row, col, val, x), TOL_F64, what=str(kw))
+
+
+def test_slices_name_their_kernel(env):
+    """kernel_name() is the kernel that a profiler shows."""
+    torch, D, F, _ = env
+    from int_spmv_b200 import matrices as M
+    row, col, val = M.stencil27(30)
+    plan = D.Plan(F.CSR(row, col, val), None, col="d16")
+    plan.spmv(torch.rand(len(row) - 1, dtype=torch.float64, device="cuda"))
+    assert plan.kernel_name().startswith("slice_rows<"), plan.kernel_name()
