@@ -167,7 +167,8 @@ __global__ void __launch_bounds__(TPB) k_axt_h1(size_t slots, UIN bs, UIN lg, co
     } else {
       const size_t t = p >> 3;
       d[0] = ldg(rwp + t);
-      d[1] = p > p0 ? ldg(rwp + t - 1) : NO_ROW;
+      // of the tile's first lane alone, not of the warp's first tile: that one opens a row anyway
+      d[1] = (p & 7u) == 0 && p > p0 ? ldg(rwp + t - 1) : NO_ROW;
     }
   };
   load(p0 + 4 * lane);

@@ -194,3 +194,45 @@ def test_device_k1_random_and_ties():
     for n, seed, rl_max in ((30011, 41, 300), (20000, 7, 3), (4099, 3, 64)):  # many equal lengths
         row, col, val = M.random_csr(n, seed, rl_max=rl_max, empty_frac=0.1)
         check_build_k1(row, col, val, M.uniform_x(n, seed))
+
+
+@pytest.mark.parametrize("mode", ["NOC", "COM"])
+@pytest.mark.parametrize("k", [1, 3, 65])
+def test_axt_h1_arrays_with_nothing_around_them(mode, k):
+    """The tileH = 1 kernels on arrays that are each an allocation of their own
+    (multiples of 2 MiB, whole): they read nothing before an array or past it."""
+    import ctypes as C
+
+    import torch
+
+    from int_spmv_b200 import device as D
+    rt = C.CDLL("libcudart.so.12")
+    size = 2 << 20  # bytes of sec: k * 2 MiB (NOC: a word per tile of 8 slots; COM: per slot)
+    words = k * size // 4
+    tiles = words if mode == "NOC" else words // 8
+    n = 1000
+    rng = np.random.default_rng(k)
+    ax = rng.uniform(-1, 1, (tiles, 16))
+    rows = np.sort(rng.integers(0, n, tiles)).astype(np.uint32)
+    sec = rows if mode == "NOC" else np.zeros(words, np.uint32)
+    if mode == "COM":  # one row per tile, and one per block start: (row << 7) | length - 1
+        sec[::8] = (rows << 7) | 7
+    want = np.bincount(rows, (ax[:, :8] * ax[:, 8:]).sum(1), n)
+    bound = np.bincount(rows, np.abs(ax[:, :8] * ax[:, 8:]).sum(1), n)
+    p = []
+    for a in (ax, sec):
+        q = C.c_void_p()
+        assert rt.cudaMalloc(C.byref(q), C.c_size_t(a.nbytes)) == 0
+        assert rt.cudaMemcpy(q, a.ctypes.data_as(C.c_void_p), C.c_size_t(a.nbytes), 1) == 0
+        p.append(q)
+    y = torch.zeros(n, dtype=torch.float64, device="cuda")
+    lib = D.load()
+    if mode == "NOC":
+        assert lib.ispmv_dev_int_axt_noc_h1(tiles, p[0], p[1], y.data_ptr(), None) == 0
+    else:
+        bn = (words + 127) // 128
+        assert lib.ispmv_dev_int_axt_com_h1(bn, 128, 7, 8, tiles, 16 * tiles, words, p[0], p[1], y.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    for q in p:
+        assert rt.cudaFree(q) == 0
+    assert np.all(np.abs(y.cpu().numpy() - want) <= 1e-12 * bound)
