@@ -1578,7 +1578,8 @@ int launch_tmem(ispmv_plan_s *p, const FPT *x, seg::Out &o, cudaStream_t s, cons
     xs = p->x32;
   }
   using XT = typename std::conditional<sizeof(VT) == 4, float, double>::type;
-  auto *k = tmemk::stream_tmem<VT, XT, SPL, S, H>;
+  constexpr int B0 = SPL == 8 ? 0 : (int)seg::RED, B1 = SPL == 8 ? 1 : (int)seg::RED;
+  auto *k = o.beta ? tmemk::stream_tmem<VT, XT, SPL, S, H, B1> : tmemk::stream_tmem<VT, XT, SPL, S, H, B0>;
   const size_t smem = tmemk::smem_bytes<VT, SPL, S, H>();
   ISPMV_TRY(cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const unsigned g = (unsigned)(p->nseg / (tmemk::CW * H));

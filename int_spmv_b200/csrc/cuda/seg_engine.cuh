@@ -37,10 +37,19 @@ __device__ __forceinline__ UIN real_row(const Out &o, UIN r) { return o.rowmap ?
 // in FP64, rounded once, as a load and an add give it; every row is written
 // once, so the result does not depend on any order): a load of y in the
 // middle of a batch stalls its warp.
+// FORM: 0 or 1 = beta, known to the compiler; RED or ATOMIC: o.beta decides, and
+// the reduction is inline assembly (the compiler keeps loads and row writes in
+// their order) or the intrinsic (it may move and predicate them).  RED is the
+// faster in stream_wide (power-law n = 4M, beta = 0: 180.0 us, ATOMIC 182.6),
+// ATOMIC in the kernels of 4 slots per lane (stream_ldg's variant 2, n = 1M,
+// beta = 0: 73.7 us, RED 77.8; 75.2 with a load and an add).
+enum RowWrite : int { RED = -1, ATOMIC = -2 };
+template <int FORM>
 __device__ __forceinline__ void write_row(const Out &o, UIN r, double v) {
   FPT *q = o.y + real_row(o, r);
-  if (o.beta) asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(q), "d"(v) : "memory");
-  else *q = v;
+  if (!(FORM < 0 ? o.beta : FORM)) *q = v;
+  else if constexpr (FORM == RED) asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(q), "d"(v) : "memory");
+  else atomicAdd(q, v);
 }
 
 // One batch of 32 units, one per lane: `p` the unit's partial sum, `r` its
@@ -58,7 +67,7 @@ __device__ __forceinline__ void batch(double p, UIN r, bool live, State &st, con
       if (lane == 0) { o.rec_row[2 * segid] = st.crow; o.rec_sum[2 * segid] = st.csum; }
       st.head_done = true;
     } else if (lane == 0) {
-      write_row(o, st.crow, st.csum);
+      write_row<ATOMIC>(o, st.crow, st.csum);
     }
   }
   if (lane == 0 && !head) p += st.csum;
@@ -73,7 +82,7 @@ __device__ __forceinline__ void batch(double p, UIN r, bool live, State &st, con
     ends &= ~(1u << first);
     st.head_done = true;
   }
-  if ((ends >> lane) & 1u) write_row(o, r, s);
+  if ((ends >> lane) & 1u) write_row<ATOMIC>(o, r, s);
   const unsigned lives = __ballot_sync(FULL, live);
   const int last = lives ? 31 - __clz(lives) : 0;
   const UIN lr = __shfl_sync(FULL, r, last);

@@ -32,12 +32,13 @@ struct Run {
   UIN seg;
 };
 
+template <int FORM = seg::ATOMIC>
 __device__ __forceinline__ void emit(const seg::Out &o, const Run &st, UIN row, double v) {
   if (row == st.row_a) {
     o.rec_row[2 * (size_t)st.seg] = row;
     o.rec_sum[2 * (size_t)st.seg] = v;
   } else {
-    seg::write_row(o, row, v);
+    seg::write_row<FORM>(o, row, v);
   }
 }
 

@@ -94,7 +94,11 @@ __device__ __forceinline__ void ld8(uint32_t taddr, uint32_t (&r)[8]) {
                : "r"(taddr));
 }
 
-template <typename VT, typename XT, int SPL, int S, int H>
+// FORM (seg::write_row): beta at compile time with 8 slots per lane: with both
+// forms of a row write in one kernel a product with beta = 0 takes up to 20%
+// longer (300,000 rows of 5, 4 stages: 57.2 us, 47.3 so); with 16 slots one
+// kernel is the faster (300 rows of 15,000: 49.2 us, 54.2 apart).
+template <typename VT, typename XT, int SPL, int S, int H, int FORM>
 __global__ void __launch_bounds__((CW * H + 1) * 32)
     stream_tmem(size_t nslots, size_t seg_slots, const uint32_t *__restrict__ blocks, const UIN *__restrict__ heads,
                 const UIN *__restrict__ segh, const XT *__restrict__ x, seg::Out o, int *status) {
@@ -222,7 +226,7 @@ __global__ void __launch_bounds__((CW * H + 1) * 32)
         for (int k = 0; k < SPL; k++)
           if (sl + k >= nslots) xv[k] = (XT)0;
       }
-      wide::batch<VT, XT, SPL>(v, xv, bits, st, o);
+      wide::batch<VT, XT, SPL, FORM>(v, xv, bits, st, o);
     }
     if (ok) sss::finish(st, o);
     else if (lane == 0) atomicExch(&failed, 1);

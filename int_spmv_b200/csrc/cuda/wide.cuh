@@ -192,7 +192,7 @@ __device__ __forceinline__ double gather(const Bands<NW> &w, uint32_t sx_addr, c
 // lane are written as they end.  Both paths add the same products in the
 // same order, so the result does not depend on the path.  Every row goes to
 // y (or to the segment's head record) from the lane that ends it.
-template <typename VT, typename XT, int SPL>
+template <typename VT, typename XT, int SPL, int FORM = seg::RED>
 __device__ __forceinline__ void batch(const VT (&v)[SPL], const XT (&xv)[SPL], unsigned bits, sss::Run &st,
                                       const seg::Out &o) {
   const unsigned lane = threadIdx.x & 31u;
@@ -224,7 +224,7 @@ __device__ __forceinline__ void batch(const VT (&v)[SPL], const XT (&xv)[SPL], u
     for (int k = 0; k < SPL; k++) {
       if ((bits >> k) & 1u) {
         if (k > first) {  // a row that starts and ends in this lane
-          seg::write_row(o, r, acc);  // never the segment's open row: it started in this segment
+          seg::write_row<FORM>(o, r, acc);  // never the segment's open row: it started in this segment
           r++;
         } else {
           pre = acc;
@@ -259,7 +259,7 @@ __device__ __forceinline__ void batch(const VT (&v)[SPL], const XT (&xv)[SPL], u
   double E = __shfl_up_sync(FULL, I, 1);
   if (lane == 0) E = 0.0;
   // the run open at my lane's start ends at my first row start
-  if (f && (lane > 0 || !(bits & 1u) || st.carry)) sss::emit(o, st, rb - 1u, E + pre);
+  if (f && (lane > 0 || !(bits & 1u) || st.carry)) sss::emit<FORM>(o, st, rb - 1u, E + pre);
   st.csum = __shfl_sync(FULL, I, 31);
   st.carry = true;
   st.rbase += tot;
