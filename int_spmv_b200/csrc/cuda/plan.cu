@@ -468,7 +468,11 @@ int stage_windows(ispmv_plan_s *p, const std::vector<UIN> &c) {
 // slots, or to tileH) from the slot streams: the kernels find rows by their
 // start bits and need none, and every slot costs its 12 bytes and a gather of
 // x[0].  On power-law rows (14.9 nonzeros) tileH = 8 pads 24%, on 5-point rows
-// 8 slots hold 5.  Leaves the stream as it is where the format is not the CSR's
+// 8 slots hold 5.  For the lane-interleaved kernels: the 4-slots-per-lane ones
+// find fewer row starts per batch with the padding and are not bound by the
+// slots (tileH = 1 at power-law n = 200,000, padded and packed: staged 33 and 37
+// us, plain 20.6 and 22.7).
+// Leaves the stream as it is, too, where the format is not the CSR's
 // (row pointer decreasing, rows past the format's slots, or values outside the
 // CSR's rows): the format's own slots are multiplied then.
 void pack_rows(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v, std::vector<UIN> &c,
@@ -567,7 +571,7 @@ int setup_stream(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v,
                  std::vector<size_t> &start) {
   p->path = P_STREAM;
   p->fslots = p->slots;
-  if (p->slots != csr->nnz) pack_rows(p, csr, v, c, start);
+  if (p->slots != csr->nnz && p->opts.kernel == ISPMV_KERNEL_WIDE) pack_rows(p, csr, v, c, start);
   if (p->chosen && p->opts.col_kind == ISPMV_COL_D16 && p->opts.val_kind != ISPMV_VAL_F32_LO16 &&
       p->opts.units_per_warp <= 0 && p->slots && p->slots == csr->nnz) {
     std::vector<uint2> meta;
