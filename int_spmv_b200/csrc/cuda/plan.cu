@@ -1522,8 +1522,12 @@ template <typename VT, int SPL, int MINB, bool D16 = false, bool TEX = false, bo
 int launch_wide(ispmv_plan_s *p, const FPT *x, seg::Out &o, cudaStream_t s, const char *name) {
   constexpr int NW = STG ? 1 : 0;
   const size_t ctas = (p->nseg + WIDE_WARPS - 1) / WIDE_WARPS;
-  // one load of CTAs: stream_wide's DEP form; never with texture gathers
-  const bool early = STG || (!TEX && ctas <= (size_t)sm_count() * MINB);
+  // one load of CTAs: stream_wide's DEP form; never with texture gathers.  Not
+  // with a caller's segment length either: a few long CTAs started early pile
+  // up on the SMs that are free first (power-law n = 200,000, 2048-slot
+  // segments: 22-26 us, 20.9 late; the automatic lengths 17.4 and 21.0)
+  const bool early =
+      STG || (!TEX && p->opts.units_per_warp <= 0 && ctas <= (size_t)sm_count() * MINB);
   if constexpr (sizeof(VT) == 4 && !STG && !LO) {
     // FP32 values: gather from an FP32 copy of x (the value the FP32 multiply uses)
     if (!p->x32) TRY(dev_alloc(p, p->n, &p->x32));
