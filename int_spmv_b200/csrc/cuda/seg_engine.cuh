@@ -119,7 +119,7 @@ __device__ __forceinline__ void finish(const State &st, const Out &o, size_t seg
 // 492.7 us a product with the records added one by one, 17.5 so.  Without
 // such a row the warp's part only costs: 52.0 -> 52.4 us (power-law n = 1M).
 constexpr size_t FIX_LONG = 8;
-constexpr int FIX_WALK = 16, FIX_U = 8;
+constexpr int FIX_WALK = 4, FIX_U = 8;
 template <bool LONG>
 __global__ void __launch_bounds__(256) fixup(size_t nrec, const UIN *rec_row_, const double *rec_sum_,
                                              const UIN *__restrict__ rowmap, const UIN *__restrict__ empty,
