@@ -475,33 +475,34 @@ int stage_windows(ispmv_plan_s *p, const std::vector<UIN> &c) {
 // Leaves the stream as it is, too, where the format is not the CSR's
 // (row pointer decreasing, rows past the format's slots, or values outside the
 // CSR's rows): the format's own slots are multiplied then.
+// In place, row after row: a copy of the stream takes the host as long again as
+// the rest of the plan (first touch of its pages).
 void pack_rows(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v, std::vector<UIN> &c,
                std::vector<size_t> &start) {
-  const long long n = csr->nrows;
+  const long long n = csr->nrows, slots = (long long)v.size();
   bool fits = true;
-  long long values = 0;
-#pragma omp parallel for schedule(static) reduction(&& : fits)
-  for (long long r = 0; r < n; r++)
-    fits = fits && csr->row[r + 1] >= csr->row[r] &&
-           (csr->row[r + 1] == csr->row[r] || start[r] + (csr->row[r + 1] - csr->row[r]) <= v.size());
-  if (!fits) return;
-  std::vector<double> pv(csr->nnz);
-  std::vector<UIN> pc(csr->nnz);
-#pragma omp parallel for schedule(static) reduction(- : values)
+  long long values = 0;  // outside the CSR's rows
+#pragma omp parallel for schedule(static) reduction(+ : values)
+  for (long long q = 0; q < slots; q++) values += v[q] != 0.0;
+#pragma omp parallel for schedule(static) reduction(&& : fits) reduction(- : values)
+  for (long long r = 0; r < n; r++) {
+    const UIN a = csr->row[r], e = csr->row[r + 1];
+    const size_t s = start[r], l = e - a;
+    // in order, inside the format, and no further left than in the CSR
+    const bool ok = e >= a && s >= a && s + l <= (r + 1 < n ? start[r + 1] : v.size()) && s + l <= v.size();
+    fits = fits && ok;
+    for (size_t k = 0; ok && k < l; k++) values -= v[s + k] != 0.0;
+  }
+  if (!fits || values) return;
   for (long long r = 0; r < n; r++) {
     const UIN a = csr->row[r], l = csr->row[r + 1] - a;
     if (!l) continue;  // a row without slots: start[r] names no slot of its own
-    std::copy_n(v.begin() + start[r], l, pv.begin() + a);
-    std::copy_n(c.begin() + start[r], l, pc.begin() + a);
-    for (UIN k = 0; k < l; k++) values -= pv[a + k] != 0.0;
+    std::copy_n(v.begin() + start[r], l, v.begin() + a);
+    std::copy_n(c.begin() + start[r], l, c.begin() + a);
+    start[r] = a;
   }
-#pragma omp parallel for schedule(static) reduction(+ : values)
-  for (long long q = 0; q < (long long)v.size(); q++) values += v[q] != 0.0;
-  if (values) return;
-  for (long long r = 0; r < n; r++)
-    if (csr->row[r + 1] > csr->row[r]) start[r] = csr->row[r];
-  v.swap(pv);
-  c.swap(pc);
+  v.resize(csr->nnz);
+  c.resize(csr->nnz);
   p->slots = csr->nnz;
 }
 
