@@ -13,7 +13,8 @@ Inputs are larger than L2 (~0.8 GB streamed per step), so no flush is needed.
 `--impl reference` times the reference's own CPU kernel (edoardoCB/int_spmv
 intSpmv_main.c, compiled from its own source into oracle/_ref) for the same
 format on the host cores, each step a bounded row sample of the workload.
-Prints ONE JSON line on rank 0.
+Prints ONE JSON line on rank 0 (below 4 KB; the tables of every format and form
+go to stderr as a `details:` line).
 """
 from __future__ import annotations
 
@@ -573,7 +574,8 @@ def main(argv=None):
             "batched": batched,
             "conversion": conversion,
         }
-        print(json.dumps(out), flush=True)
+        print("details: " + json.dumps(out), file=sys.stderr, flush=True)
+        print(json.dumps(headline(out)), flush=True)
     if ws > 1:
         import torch.distributed as dist
         dist.barrier()
@@ -637,6 +639,33 @@ def precision_lines(a, rank, ws, stream, dev, peak):
                      for f in ("f32/u32", "f32/d16", "f64/d16", "f32lo/u32")}
     out["target"] = "FP32 values / FP64 accumulate >= 1.4x plain FP64 at <= 1e-6 relative error"
     return out
+
+
+def headline(out: dict) -> dict:
+    """The printed line: the whole result (which goes to stderr) without its
+    per-format, per-form and per-block tables, of which each form's
+    milliseconds stay, and without the notes: a line of 23 KB was cut where it
+    was read."""
+    def digits(v):
+        if isinstance(v, float):
+            return float(f"{v:.6g}")
+        if isinstance(v, dict):
+            return {k: digits(w) for k, w in v.items() if k != "note"}
+        return [digits(w) for w in v] if isinstance(v, list) else v
+
+    def times(table):
+        return {k: float(f"{r['ms']:.4g}") for k, r in table.items() if isinstance(r, dict) and "ms" in r}
+
+    line = {k: digits(v) for k, v in out.items()
+            if k not in ("formats", "precision", "spmm", "batched", "conversion")}
+    tables = {"formats": out["formats"], "precision": out["precision"], "spmm": out["spmm"],
+              "batched": (out["batched"] or {}).get("results")}
+    line["ms"] = {k: times(t) for k, t in tables.items() if t}
+    plan = (out["conversion"] or {}).get("plan")
+    if plan:
+        line["conversion_s"] = digits({"host": out["conversion"]["host_s"], "gpu": out["conversion"]["gpu_s"],
+                                       "plan_host": plan.get("host_s"), "plan_gpu": plan.get("gpu_s")})
+    return line
 
 
 def _event_time(fn, steps: int, warmup: int) -> float:

@@ -131,3 +131,44 @@ def test_fem_batch_c_sizes_match_fem_batch():
     rng = np.random.default_rng(4)
     ns = np.exp(rng.uniform(np.log(1e3), np.log(3e3), 6)).astype(np.int64)
     assert [len(r) - 1 for r, _, _ in mats] == list(ns)
+
+
+def test_bench_line_is_short():
+    """bench.py's printed line keeps what a reader of the run needs (value,
+    config, roofline, end to end, clocks, parity, each form's time) and stays
+    below 4 KB, however many formats were timed."""
+    import json
+
+    import bench
+    wl = dict(name="powerlaw_n4M_seed1", row=np.zeros(4_000_001, np.int8), col=np.zeros(59_395_000, np.int8))
+    row = {"ms": 0.168212345678, "gflops": 700.123456789, "gbs": 4800.123456789, "frac": 0.7432123456789,
+           "kernel_ms": 0.1581234567, "kernel_frac": 0.78123456789, "kernel": "stream_wide<8,stg,b4>",
+           "max_componentwise_err": 6.123456789e-16, "normwise_err": 1.23456789e-16, "aErr": 1.0, "rErr": 2.0, "pos": 7}
+    out = {"metric": bench.METRIC, "value": 701.123456789, "unit": bench.UNIT, "n_gpus": 1, "steps": 20, "warmup": 5,
+           "ms_per_step": 0.169123456789, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
+           "dtype": "f64", "data": "synthetic: " + "x" * 200,
+           "config": bench.run_config(wl, bench.format_name("COM128"), "f64", "u32", 8.1e8),
+           "kernel": {"family": "wide", "name": "stream_wide<8,stg,b4>", "replicas": 1}, "gb_per_s": 4700.123456,
+           "roofline": {"bound": "hbm", "achieved": 5043.123456, "peak": 6463.0, "unit": "GB/s", "frac": 0.78,
+                        "traffic": {"dram_bytes": 1, "source": "x" * 80}, "kernel": "stream_wide<8,stg,b4>",
+                        "kernel_ms": 0.158123456, "kernel_ms_chunks": [0.158123456789] * 5, "note": "n" * 700},
+           "cpu_baseline": {"value": 31.5, "unit": bench.UNIT, "cores": 64, "kind": "reference", "sample": "s" * 160},
+           "e2e": {"value": 93.1, "unit": bench.UNIT, "h2d_bytes_per_step": 32_000_000, "d2h_bytes_per_step": 32_000_000},
+           "gpu_launches": 40, "clocks": {"sm_mhz": 1965.0, "sm_max_mhz": 1965.0, "reasons": [], "samples": 9},
+           "parity": {"max_componentwise": 6e-16, "bound": 1e-12, "pass": True, "normwise": 1e-16},
+           "formats": {f"AXT_COM_H1_HW8_BS{i}/f32lo/d16/wide": dict(row) for i in range(40)},
+           "precision": {"workload": "w", "n": 1, **{f"f{i}/u32/plain-loads": dict(row) for i in range(6)}},
+           "spmm": {"workload": "w", **{f"f64/k{i}": dict(row) for i in range(6)}},
+           "batched": {"results": {"graph_wide": dict(row), "graph_queue": dict(row), "separate": dict(row)}},
+           "conversion": {"host_s": 0.1, "gpu_s": 0.001, "note": "n" * 90, "plan": {"host_s": 1.0, "gpu_s": 0.01, "note": "n"}}}
+    line = bench.headline(out)
+    assert len(json.dumps(line)) < 4096
+    for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+              "vs_baseline", "dtype", "data", "config", "roofline", "e2e", "gpu_launches", "clocks", "parity"):
+        assert k in line, k
+    assert line["config"] == out["config"] and line["e2e"]["h2d_bytes_per_step"] == 32_000_000
+    assert abs(line["value"] / out["value"] - 1) < 1e-5 and len(line["ms"]["formats"]) == 40
+    # without the extra tables (another workload, several GPUs)
+    assert "ms" in bench.headline(dict(out, formats={}, precision=None, spmm=None, batched=None, conversion=None))
+    assert bench.headline(dict(out, precision={"unavailable": "x"}, batched={"unavailable": "x"},
+                               conversion={"unavailable": "x"}))["value"]
