@@ -431,8 +431,9 @@ void ispmv_plan_opts_default(ispmv_plan_opts *o);
 
 /* Plans from host-built formats.  The host arrays are only read during the
  * call; the plan owns its device copies.  `csr` must have rl filled.  The
- * lane-interleaved kernels' plans hold the rows back to back, without the
- * padding of AXC bricks and AXT tiles (info.slots counts the format's slots). */
+ * lane-interleaved kernels' plans, and large ones of ISPMV_KERNEL_LDG, hold the
+ * rows back to back, without the padding of AXC bricks and AXT tiles
+ * (info.slots counts the format's slots). */
 int ispmv_plan_csr(const str_matCSR *csr, const ispmv_plan_opts *o, ispmv_plan *out);
 int ispmv_plan_axc(const str_matCSR *csr, const str_matAXC *axc, const UIN *axi,
                    const ispmv_plan_opts *o, ispmv_plan *out);

@@ -390,7 +390,7 @@ void auto_wide(ispmv_plan_s *p, const str_matCSR *csr) {
 // column inside x[0, n rounded down to even), so the bulk copy starts on a
 // 16-byte boundary and moves a multiple of 16 bytes.  Columns outside a CTA's
 // window are gathered from x, so the choice costs time only; it is made from
-// every fourth group of 8 slots, by counting twice:
+// every eighth group of 8 slots, by counting twice:
 //   1. columns per bin of 2^s1 (at most 8192 bins): the l1 neighbouring bins
 //      with the most columns, l1 bins being wide enough for any W columns;
 //   2. columns per bin of 2^s2 inside those (at most 2048 bins): the W >> s2
@@ -468,15 +468,17 @@ int stage_windows(ispmv_plan_s *p, const std::vector<UIN> &c) {
 // slots, or to tileH) from the slot streams: the kernels find rows by their
 // start bits and need none, and every slot costs its 12 bytes and a gather of
 // x[0].  On power-law rows (14.9 nonzeros) tileH = 8 pads 24%, on 5-point rows
-// 8 slots hold 5.  For the lane-interleaved kernels: the 4-slots-per-lane ones
-// find fewer row starts per batch with the padding and are not bound by the
-// slots (tileH = 1 at power-law n = 200,000, padded and packed: staged 33 and 37
-// us, plain 20.6 and 22.7).
+// 8 slots hold 5.  The 4-slots-per-lane kernels find fewer row starts per batch
+// with the padding, and only the plain one is bound by the slots, on large
+// matrices (AXT tileH = 1, padded and packed: staged at power-law n = 200,000 33
+// and 37 us, n = 1M 107 and 112; plain at n = 200,000, 3.7M slots, 20.6 and 22.7,
+// n = 1M 69.9 and 66.8, n = 4M 230 and 207).
 // Leaves the stream as it is, too, where the format is not the CSR's
 // (row pointer decreasing, rows past the format's slots, or values outside the
 // CSR's rows): the format's own slots are multiplied then.
 // In place, row after row: a copy of the stream takes the host as long again as
 // the rest of the plan (first touch of its pages).
+constexpr size_t PACK_LDG = (size_t)1 << 22;  // slots
 void pack_rows(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v, std::vector<UIN> &c,
                std::vector<size_t> &start) {
   const long long n = csr->nrows, slots = (long long)v.size();
@@ -572,7 +574,9 @@ int setup_stream(ispmv_plan_s *p, const str_matCSR *csr, std::vector<double> &v,
                  std::vector<size_t> &start) {
   p->path = P_STREAM;
   p->fslots = p->slots;
-  if (p->slots != csr->nnz && p->opts.kernel == ISPMV_KERNEL_WIDE) pack_rows(p, csr, v, c, start);
+  if (p->slots != csr->nnz && (p->opts.kernel == ISPMV_KERNEL_WIDE ||
+                               (p->opts.kernel == ISPMV_KERNEL_LDG && p->slots >= PACK_LDG)))
+    pack_rows(p, csr, v, c, start);
   if (p->chosen && p->opts.col_kind == ISPMV_COL_D16 && p->opts.val_kind != ISPMV_VAL_F32_LO16 &&
       p->opts.units_per_warp <= 0 && p->slots && p->slots == csr->nnz) {
     std::vector<uint2> meta;
@@ -2012,7 +2016,8 @@ bool tmem_plan(const ispmv_plan_s *p) {
 // share of as many loads of the GPU's `held` groups as keep it at 192 or less.
 // Longer parts spread the resident groups over more of the matrix (less of X
 // found in L2), shorter ones pay their start more often: k = 8 / 32 on
-// power-law rows 144 / 323 us at 128 slots, 138 / 330 at 192, 149 / 339 at 256.
+// power-law rows 144 / 323 us at 128 slots, 138 / 330 at 192, 149 / 339 at 256
+// (the same X each time).
 size_t spmm_part(size_t slots, size_t held) {
   const size_t loads = std::max<size_t>(1, (slots + held * 192 - 1) / (held * 192));
   return std::max<size_t>(64, ((slots + loads * held - 1) / (loads * held) + 63) / 64 * 64);

@@ -22,13 +22,14 @@
 //     per lane in flight: four slots of a step are consumed, then the pieces of
 //     the same four slots of the next step are loaded into the registers freed
 //     (slot by slot, the loads outnumber the barriers a warp waits on, and the
-//     two-column form took 175 us where it takes 138 so);
+//     two-column form took 175 us where it takes 138 so, the same X each time);
 //   - parts are short (spmm_part): the warps resident at a time then work on
 //     neighbouring rows, whose columns' X rows stay in L2 (k = 32, 256 MB of
 //     X: 323 us at 128 slots, 413 at 512), and the joins inside the CTA keep
 //     the records few (records per part cost 12-44 us of fix-up).
 // Power-law n = 1M, 14.9M nonzeros, FP64, against one slot's value and column
-// per lane and step: k = 8 237 us -> 149, k = 32 434 -> 364 (fresh X each time).
+// per lane and step, three matrices and X in turn (neither in L2 when a product
+// starts): k = 8 236 us -> 151, k = 32 450 -> 372.
 #pragma once
 #include <type_traits>
 

@@ -24,8 +24,8 @@
 // slots, row starts are bits of `heads` (slot order), a warp owns a segment
 // of slots and leaves two (row, partial) records per segment for
 // seg::fixup.  A row is written by the lane that ends it.  Every row is
-// written exactly once, without atomics, and the summation order is fixed,
-// so results are bitwise repeatable.
+// written exactly once (beta = 1: by one reduction), and the summation order is
+// fixed, so results are bitwise repeatable.
 //
 // stream_wide_tma is the same reduction fed by 1D bulk copies
 // (cp.async.bulk, no multicast) into a per-warp ring of stages in shared
@@ -285,8 +285,8 @@ __device__ __forceinline__ void batch(const VT (&v)[SPL], const XT (&xv)[SPL], u
 // before the launch, so this form is never a dependent (DEP): the lines it
 // finds may be those of x (or of x's FP32 copy) before it was written anew.
 // STG: one window per CTA chosen by the plan (xw.tlo/xw.tlen: columns that
-// hold many of the CTA's, by counting), copied into shared memory by one bulk copy
-// (cp.async.bulk, no multicast) on an mbarrier; x must be 16-byte aligned
+// hold many of the CTA's, by counting), copied into shared memory by one bulk
+// copy (cp.async.bulk, no multicast) on an mbarrier; x must be 16-byte aligned
 // (the host checks).  The copy leaves the L1 load pipe to the gathers and
 // costs no load loop.  Each warp waits for it (bounded) only before its
 // first gathers, after its first batch's values and columns are on their

@@ -294,3 +294,27 @@ def test_slices_name_their_kernel(env):
     plan = D.Plan(F.CSR(row, col, val), None, col="d16")
     plan.spmv(torch.rand(len(row) - 1, dtype=torch.float64, device="cuda"))
     assert plan.kernel_name().startswith("slice_rows<"), plan.kernel_name()
+
+
+@pytest.mark.parametrize("empty", ["none", "first", "last", "some", "all but one"])
+def test_padding_is_dropped(env, empty):
+    """The lane-interleaved plans of padded formats hold the nonzeros alone,
+    wherever the empty rows are; the 4-slots-per-lane ones of small matrices
+    hold the format's slots."""
+    _, D, F, _ = env
+    n = 700
+    lengths = np.random.default_rng(3).integers(1, 30, n)
+    lengths[{"none": [], "first": [0, 1, 2], "last": [n - 1, n - 2], "some": [5, 6, 100, 690],
+             "all but one": [r for r in range(n) if r != 400]}[empty]] = 0
+    row, col, val = rows_of(lengths, n, 4)
+    csr = F.CSR(row, col, val)
+    z = np.zeros(n)
+    for f in [F.getFormatDataAXC(0, csr, z)[1]] + [F.getFormatDataAXT(0, 128, 8, th, "NOC", csr, z)[1] for th in (1, 3, 4, 8, 16)]:
+        p = D.Plan(csr, f)
+        assert p.export_stream()["layout"]["slots"] == len(col)
+        check(env, row, col, val, p, "f64")
+    axc = F.getFormatDataAXC(0, csr, z)[1]
+    for kernel in ("ldg", "tma"):
+        p = D.Plan(csr, axc, kernel=kernel)
+        assert p.export_stream()["layout"]["slots"] == p.info["slots"]
+        check(env, row, col, val, p, "f64")
