@@ -42,7 +42,8 @@ __device__ __forceinline__ UIN real_row(const Out &o, UIN r) { return o.rowmap ?
 // their order) or the intrinsic (it may move and predicate them).  RED is the
 // faster in stream_wide (power-law n = 4M, beta = 0: 180.0 us, ATOMIC 182.6),
 // ATOMIC in the kernels of 4 slots per lane (stream_ldg's variant 2, n = 1M,
-// beta = 0: 73.7 us, RED 77.8; 75.2 with a load and an add).
+// beta = 0: 73.7 us, RED 77.8; 75.2 with a load and an add) but the work-queue
+// one (64 FEM blocks, 147M nonzeros: RED 373 us, ATOMIC 400).
 enum RowWrite : int { RED = -1, ATOMIC = -2 };
 template <int FORM>
 __device__ __forceinline__ void write_row(const Out &o, UIN r, double v) {

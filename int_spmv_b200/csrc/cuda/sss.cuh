@@ -75,10 +75,75 @@ struct Words<4> {
   __device__ __forceinline__ UIN get(int i) const { return i == 0 ? w.x : i == 1 ? w.y : i == 2 ? w.z : w.w; }
 };
 
+__device__ __forceinline__ unsigned lanemask_le() {
+  unsigned m;
+  asm("mov.u32 %0, %%lanemask_le;" : "=r"(m));
+  return m;
+}
+
+// The 4-slot batch without per-slot branches: a lane's leading piece (slots
+// before its first row start) and trailing piece (from its last row start)
+// are masked sums; only lanes holding two or more row starts (rows shorter
+// than 4 slots) take the loop that writes the runs between them.
+template <int FORM>
+__device__ __forceinline__ void batch4(const double (&p)[4], const Words<4> &hw, Run &st, const seg::Out &o) {
+  const unsigned lane = threadIdx.x & 31u;
+  const unsigned q = lane >> 3, sh = 4u * (lane & 7u);
+  const UIN w0 = hw.w.x, w1 = hw.w.y, w2 = hw.w.z, w3 = hw.w.w;
+  const unsigned c0 = __popc(w0), c1 = c0 + __popc(w1), c2 = c1 + __popc(w2), tot = c2 + __popc(w3);
+  const UIN myw = q == 0 ? w0 : q == 1 ? w1 : q == 2 ? w2 : w3;
+  const unsigned before = q == 0 ? 0u : q == 1 ? c0 : q == 2 ? c1 : c2;
+  const unsigned bits = (myw >> sh) & 0xFu;
+  const UIN rb = st.rbase + before + __popc(myw & ((1u << sh) - 1u));  // row of my first start
+  const int first = bits ? __ffs(bits) - 1 : 4;
+  const int last = bits ? 31 - __clz(bits) : 4;
+  double pre = 0.0, run = 0.0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    pre += (k < first) ? p[k] : 0.0;
+    run += (k >= last) ? p[k] : 0.0;
+  }
+  if (__popc(bits) >= 2) {
+    UIN r = rb;
+    double acc = 0.0;
+    bool open = false;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if ((bits >> k) & 1u) {
+        if (open) emit<FORM>(o, st, r++, acc);
+        acc = 0.0;
+        open = true;
+      }
+      acc += open ? p[k] : 0.0;
+    }
+  }
+  if (lane == 0 && st.carry) pre += st.csum;
+  const bool f = bits != 0;
+  const unsigned F = __ballot_sync(FULL, f) & lanemask_le();
+  const int start = F ? 31 - __clz(F) : 0;  // my segment's first lane
+  const int reach = (int)lane - start;      // lanes below me in my segment
+  double I = f ? run : pre;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const double u = __shfl_up_sync(FULL, I, d);
+    if (reach >= d) I += u;
+  }
+  double E = __shfl_up_sync(FULL, I, 1);
+  if (lane == 0) E = 0.0;
+  if (f && (lane > 0 || !(bits & 1u) || st.carry)) emit<FORM>(o, st, rb - 1u, E + pre);
+  st.csum = __shfl_sync(FULL, I, 31);
+  st.carry = true;
+  st.rbase += tot;
+}
+
 // One batch of 32*SPL slots; lane l holds slots SPL*l .. SPL*l+SPL-1 with
 // products p, the batch's bitmap words hw.
-template <int SPL>
+template <int SPL, int FORM = seg::ATOMIC>
 __device__ __forceinline__ void batch(const double (&p)[SPL], const Words<SPL> &hw, Run &st, const seg::Out &o) {
+  if constexpr (SPL == 4) {
+    batch4<FORM>(p, hw, st, o);
+    return;
+  }
   constexpr unsigned LPW = 32 / SPL;  // lanes per bitmap word
   const unsigned lane = threadIdx.x & 31u;
   const unsigned q = lane / LPW, sh = SPL * (lane % LPW);
@@ -106,7 +171,7 @@ __device__ __forceinline__ void batch(const double (&p)[SPL], const Words<SPL> &
 #pragma unroll
     for (int k = 0; k < SPL; k++) {
       if ((bits >> k) & 1u) {
-        if (nh) emit(o, st, rb + nh - 1u, run);
+        if (nh) emit<FORM>(o, st, rb + nh - 1u, run);
         run = 0.0;
         nh++;
       }
@@ -128,68 +193,7 @@ __device__ __forceinline__ void batch(const double (&p)[SPL], const Words<SPL> &
   double E = __shfl_up_sync(FULL, I, 1);
   if (lane == 0) E = 0.0;
   // the run open at my lane start ends at my first start
-  if (f && (lane > 0 || !(bits & 1u) || st.carry)) emit(o, st, rb - 1u, E + pre);
-  st.csum = __shfl_sync(FULL, I, 31);
-  st.carry = true;
-  st.rbase += tot;
-}
-
-__device__ __forceinline__ unsigned lanemask_le() {
-  unsigned m;
-  asm("mov.u32 %0, %%lanemask_le;" : "=r"(m));
-  return m;
-}
-
-// The 4-slot batch without per-slot branches: a lane's leading piece (slots
-// before its first row start) and trailing piece (from its last row start)
-// are masked sums; only lanes holding two or more row starts (rows shorter
-// than 4 slots) take the loop that writes the runs between them.
-template <>
-__device__ __forceinline__ void batch<4>(const double (&p)[4], const Words<4> &hw, Run &st, const seg::Out &o) {
-  const unsigned lane = threadIdx.x & 31u;
-  const unsigned q = lane >> 3, sh = 4u * (lane & 7u);
-  const UIN w0 = hw.w.x, w1 = hw.w.y, w2 = hw.w.z, w3 = hw.w.w;
-  const unsigned c0 = __popc(w0), c1 = c0 + __popc(w1), c2 = c1 + __popc(w2), tot = c2 + __popc(w3);
-  const UIN myw = q == 0 ? w0 : q == 1 ? w1 : q == 2 ? w2 : w3;
-  const unsigned before = q == 0 ? 0u : q == 1 ? c0 : q == 2 ? c1 : c2;
-  const unsigned bits = (myw >> sh) & 0xFu;
-  const UIN rb = st.rbase + before + __popc(myw & ((1u << sh) - 1u));  // row of my first start
-  const int first = bits ? __ffs(bits) - 1 : 4;
-  const int last = bits ? 31 - __clz(bits) : 4;
-  double pre = 0.0, run = 0.0;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    pre += (k < first) ? p[k] : 0.0;
-    run += (k >= last) ? p[k] : 0.0;
-  }
-  if (__popc(bits) >= 2) {
-    UIN r = rb;
-    double acc = 0.0;
-    bool open = false;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      if ((bits >> k) & 1u) {
-        if (open) emit(o, st, r++, acc);
-        acc = 0.0;
-        open = true;
-      }
-      acc += open ? p[k] : 0.0;
-    }
-  }
-  if (lane == 0 && st.carry) pre += st.csum;
-  const bool f = bits != 0;
-  const unsigned F = __ballot_sync(FULL, f) & lanemask_le();
-  const int start = F ? 31 - __clz(F) : 0;  // my segment's first lane
-  const int reach = (int)lane - start;      // lanes below me in my segment
-  double I = f ? run : pre;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const double u = __shfl_up_sync(FULL, I, d);
-    if (reach >= d) I += u;
-  }
-  double E = __shfl_up_sync(FULL, I, 1);
-  if (lane == 0) E = 0.0;
-  if (f && (lane > 0 || !(bits & 1u) || st.carry)) emit(o, st, rb - 1u, E + pre);
+  if (f && (lane > 0 || !(bits & 1u) || st.carry)) emit<FORM>(o, st, rb - 1u, E + pre);
   st.csum = __shfl_sync(FULL, I, 31);
   st.carry = true;
   st.rbase += tot;
@@ -374,7 +378,7 @@ __global__ void __launch_bounds__(256, 6) stream_queue(size_t nslots, size_t nsl
         for (int k = 0; k < SPL; k++)
           if (sl + k >= nslots) p[k] = 0.0;
       }
-      batch<SPL>(p, cur.h, st, o);
+      batch<SPL, seg::RED>(p, cur.h, st, o);
     }
     finish(st, o);
   }
